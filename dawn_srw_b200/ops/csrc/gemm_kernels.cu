@@ -1473,6 +1473,10 @@ extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void*
         const double fill = static_cast<double>(items) / ((items + units - 1) / units * units);
         if (fill > best + 0.05) { best = fill; want = s; }
       }
+      // Every split has to have K tiles of its own: one without would add whatever its CTA's
+      // accumulator still holds (163 tiles in 20 splits of 9 leave the last one empty).
+      const int per_split = (k_tiles + want - 1) / want;
+      want = (k_tiles + per_split - 1) / per_split;
       if (want > 1) gp.k_splits = want;
     }
   }

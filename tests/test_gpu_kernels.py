@@ -58,6 +58,29 @@ def test_gemm_epilogue_options(cb):
     cb.check_status()
 
 
+@pytest.mark.parametrize("M,N,K,a_mn", [(8, 384, 25200, False), (6, 1280, 10400, False),
+                                        (231, 384, 25200, False), (256, 256, 10400, True),
+                                        (128, 128, 25200, True)])
+def test_accumulating_gemm_whose_k_tiles_do_not_divide_into_splits(cb, M, N, K, a_mn):
+    """K tiles that leave the last of the wanted splits empty (163 = 18 * 9 + 1, not 20 * 9): a
+    split without K tiles would add the previous launch's accumulators.  fp32 accumulation of
+    exact bf16 products in any order is within K * 2^-24 of the row norms' product, i.e. far
+    below 1e-5 of a random result's norm; a stale accumulator is of the order of one."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(K + M)
+    A = torch.randn(M, K, device=dev, generator=g).bfloat16()
+    B = torch.randn(K, N, device=dev, generator=g).bfloat16()
+    ref = A.double() @ B.double()
+    As = A.t().contiguous() if a_mn else A
+    big = torch.randn(512, 1024, device=dev, generator=g).bfloat16()
+    for _ in range(2):
+        cb.gemm(big, False, big, False)                      # leaves values in the accumulators
+        out = torch.zeros(M, N, device=dev)
+        cb.gemm(As, a_mn, B, True, out=out, accumulate=True)
+        assert _rel(out, ref) < 1e-5
+    cb.check_status()
+
+
 @pytest.mark.parametrize("M", [1, 32, 128])
 def test_engine_gemm_with_few_rows(cb, M):
     """Up to 128 rows: single-CTA tiles, and the long K of a decode-step write GEMM is cut
