@@ -18,6 +18,7 @@
 #include <stdint.h>
 
 #include "common/gate_math.cuh"
+#include "common/ptx.cuh"
 #include "dsb_api.h"
 #include "dsb_api_ops.h"
 
@@ -254,10 +255,176 @@ __global__ void __launch_bounds__(256) srw_rows_finish_kernel(
   }
 }
 
+// ------------------------------------------------- attention over the KV cache
 // One decoded token of one (batch, head): append k, v to the cache at position
 // pos[0], then softmax(q . K[0..pos]^T / sqrt(dh)) . V[0..pos].  q, k, v, out are
 // token-major fp32 [B, H * dh]; the caches are fp32 [B, H, S_max, dh].  The position
 // is a device scalar so that the launch can sit in a captured graph.
+//
+// The op reads n * dh * 8 bytes per (batch, head) and is bound by how many of them are in
+// flight, so the positions are split over the CTAs of a cluster, over warps and over
+// eight groups of four lanes: a group takes a position, a lane every fourth 16-byte
+// chunk of its K and V rows (64 contiguous bytes per group and load), all of them
+// in flight together.  Every group keeps a running (max, sum, output), merged by shuffles,
+// then in shared memory, then through the cluster's shared memory by its first CTA.
+struct KvParams {
+  const float *q, *k, *v;
+  float *cache_k, *cache_v;
+  const long long* pos;
+  float* out;
+  int H, dh, s_max;
+  float scale;
+};
+constexpr int kKvThreads = 128, kKvGroups = kKvThreads / 4;
+constexpr int kKvMaxDh = 128;
+
+__device__ __forceinline__ float merge_weight(float m, float m_all) {
+  return m > -INFINITY ? __expf(m - m_all) : 0.f;
+}
+
+// NV: 16-byte chunks of a head row per lane (dh <= 16 * NV, dh % 4 == 0).
+template <int NV>
+__global__ void __launch_bounds__(kKvThreads) kv_decode_split_kernel(const KvParams p) {
+  __shared__ float s_m[kKvThreads / 32], s_l[kKvThreads / 32];
+  __shared__ __align__(16) float s_o[kKvThreads / 32][kKvMaxDh];
+  __shared__ float c_ml[2];
+  __shared__ float c_o[kKvMaxDh];
+  const int splits = gridDim.x, rank = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane & 3, grp = tid >> 2;
+  const int nv4 = p.dh >> 2;
+  long long pos = p.pos[0];
+  pos = pos < 0 ? 0 : (pos >= p.s_max ? p.s_max - 1 : pos);
+  const int n_old = static_cast<int>(pos);
+  const size_t row = (static_cast<size_t>(b) * p.H + h) * p.dh;
+  float* ck = p.cache_k + row * p.s_max;
+  float* cv = p.cache_v + row * p.s_max;
+  const float4* q4 = reinterpret_cast<const float4*>(p.q + row);
+  float4 qv[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = sub + 4 * i;
+    qv[i] = c < nv4 ? q4[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    qv[i].x *= p.scale; qv[i].y *= p.scale; qv[i].z *= p.scale; qv[i].w *= p.scale;
+  }
+  float m = -INFINITY, l = 0.f;
+  float4 o[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto take = [&](const float* kr, const float* vr, bool valid) {
+    float4 kq[NV], vq[NV];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = sub + 4 * i;
+      const bool ok = valid && c < nv4;
+      kq[i] = ok ? __ldcs(reinterpret_cast<const float4*>(kr) + c) : zero;
+      vq[i] = ok ? __ldcs(reinterpret_cast<const float4*>(vr) + c) : zero;
+    }
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      s = fmaf(qv[i].x, kq[i].x, s);
+      s = fmaf(qv[i].y, kq[i].y, s);
+      s = fmaf(qv[i].z, kq[i].z, s);
+      s = fmaf(qv[i].w, kq[i].w, s);
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if (!valid) return;
+    const float mn = fmaxf(m, s);
+    const float f = __expf(m - mn), e = __expf(s - mn);
+    l = fmaf(l, f, e);
+    m = mn;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      o[i].x = fmaf(o[i].x, f, e * vq[i].x);
+      o[i].y = fmaf(o[i].y, f, e * vq[i].y);
+      o[i].z = fmaf(o[i].z, f, e * vq[i].z);
+      o[i].w = fmaf(o[i].w, f, e * vq[i].w);
+    }
+  };
+  // cached positions 0..pos-1 of this CTA
+  const int per = (n_old + splits - 1) / splits;
+  const int j1 = min(n_old, (rank + 1) * per);
+  for (int j0 = rank * per; j0 < j1; j0 += kKvGroups) {       // block-uniform trip count
+    const int j = j0 + grp;
+    take(ck + static_cast<size_t>(j) * p.dh, cv + static_cast<size_t>(j) * p.dh, j < j1);
+  }
+  // the new position comes from the inputs; the first warp of the first CTA appends it
+  if (rank == 0 && warp == 0) {
+    take(p.k + row, p.v + row, grp == 0);
+    for (int c = lane; c < nv4; c += 32) {
+      reinterpret_cast<float4*>(ck + pos * p.dh)[c] = reinterpret_cast<const float4*>(p.k + row)[c];
+      reinterpret_cast<float4*>(cv + pos * p.dh)[c] = reinterpret_cast<const float4*>(p.v + row)[c];
+    }
+  }
+  // ---- groups of a warp
+  float mw = m;
+#pragma unroll
+  for (int x = 4; x < 32; x <<= 1) mw = fmaxf(mw, __shfl_xor_sync(0xffffffffu, mw, x));
+  const float fg = merge_weight(m, mw);
+  l *= fg;
+#pragma unroll
+  for (int x = 4; x < 32; x <<= 1) l += __shfl_xor_sync(0xffffffffu, l, x);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    float* e = reinterpret_cast<float*>(&o[i]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float t = e[k] * fg;
+#pragma unroll
+      for (int x = 4; x < 32; x <<= 1) t += __shfl_xor_sync(0xffffffffu, t, x);
+      e[k] = t;
+    }
+    const int c = sub + 4 * i;
+    if (lane < 4 && c < nv4) *reinterpret_cast<float4*>(&s_o[warp][4 * c]) = o[i];
+  }
+  if (lane == 0) { s_m[warp] = mw; s_l[warp] = l; }
+  __syncthreads();
+  // ---- warps of the CTA: thread t owns output column t
+  float mc = s_m[0];
+#pragma unroll
+  for (int w = 1; w < kKvThreads / 32; ++w) mc = fmaxf(mc, s_m[w]);
+  float lc = 0.f, oc = 0.f;
+#pragma unroll
+  for (int w = 0; w < kKvThreads / 32; ++w) {
+    const float f = merge_weight(s_m[w], mc);
+    lc = fmaf(f, s_l[w], lc);
+    if (tid < p.dh) oc = fmaf(f, s_o[w][tid], oc);
+  }
+  if (splits == 1) {
+    if (tid < p.dh) p.out[row + tid] = oc / lc;
+    return;
+  }
+  // ---- CTAs of the cluster
+  if (tid < p.dh) c_o[tid] = oc;
+  if (tid == 0) { c_ml[0] = mc; c_ml[1] = lc; }
+  cluster_sync_all();
+  if (rank == 0) {
+    float ms[8], ls[8], ma = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (r < splits) {
+        ms[r] = ld_cluster_f32(mapa_shared(smem_u32(&c_ml[0]), r));
+        ls[r] = ld_cluster_f32(mapa_shared(smem_u32(&c_ml[1]), r));
+        ma = fmaxf(ma, ms[r]);
+      }
+    }
+    float lt = 0.f, ot = 0.f;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      if (r < splits) {
+        const float f = merge_weight(ms[r], ma);
+        lt = fmaf(f, ls[r], lt);
+        if (tid < p.dh) ot = fmaf(f, ld_cluster_f32(mapa_shared(smem_u32(&c_o[tid]), r)), ot);
+      }
+    }
+    if (tid < p.dh) p.out[row + tid] = ot / lt;
+  }
+  cluster_sync_all();      // nobody leaves while its shared memory may still be read
+}
+
+// Any head dimension up to 128 and any alignment: a block per (batch, head), a warp per position.
 __global__ void __launch_bounds__(128) kv_decode_attention_kernel(
     const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
     float* __restrict__ cache_k, float* __restrict__ cache_v, const long long* __restrict__ pos_ptr,
@@ -355,6 +522,41 @@ __global__ void __launch_bounds__(256) gemv_rows_kernel(const __nv_bfloat16* __r
   }
 }
 
+int device_sms() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n > 0 ? n : 148;
+}
+
+template <int NV>
+int launch_kv_nv(const KvParams& p, int splits, int B, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(splits, p.H, B);
+  cfg.blockDim = dim3(kKvThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kv_decode_split_kernel<NV>, p) == cudaSuccess ? 0 : 913;
+}
+
+// The position is not known here, so the split follows from what the cache can hold: up to
+// eight CTAs per (batch, head) until there are four CTAs per SM, none shorter than 32 positions.
+int launch_kv(const KvParams& p, int B, cudaStream_t stream) {
+  const int want = 4 * device_sms();
+  int splits = 1;
+  while (splits < 8 && B * p.H * splits < want && p.s_max / (2 * splits) >= kKvGroups) splits *= 2;
+  if (p.dh <= 32) return launch_kv_nv<2>(p, splits, B, stream);
+  if (p.dh <= 64) return launch_kv_nv<4>(p, splits, B, stream);
+  if (p.dh <= 80) return launch_kv_nv<5>(p, splits, B, stream);
+  return launch_kv_nv<8>(p, splits, B, stream);
+}
+
 template <int KIND, int NR, int KC>
 int launch_rows(const RowsParams& p, int blocks, cudaStream_t stream) {
   const size_t smem = static_cast<size_t>(NR) * (p.D + p.r) * 2 + static_cast<size_t>(NR) * p.D * 4 + NR * 4 + 16;
@@ -393,10 +595,7 @@ extern "C" int dsb_srw_rows_max(int D) {
 }
 
 extern "C" int dsb_srw_rows_blocks(int N, int D) {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  if (n <= 0) n = 148;
+  const int n = device_sms();
   return (N <= 1 && D <= 1280) ? 2 * n : n;   // one row needs 128 registers: two blocks per SM
 }
 
@@ -444,9 +643,17 @@ extern "C" int dsb_kv_decode_attention(const float* q, const float* k, const flo
                                        int s_max, float* out, cudaStream_t stream) {
   if (B <= 0 || H <= 0) return 0;
   if (dh <= 0 || dh > 128 || s_max <= 0 || s_max > 8192) return 911;
+  const float scale = rsqrtf(static_cast<float>(dh));
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
+                         reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(cache_k) |
+                         reinterpret_cast<uintptr_t>(cache_v);
+  if (dh % 4 == 0 && (bits & 15) == 0) {
+    const KvParams p = {q, k, v, cache_k, cache_v, pos, out, H, dh, s_max, scale};
+    return launch_kv(p, B, stream);
+  }
   const dim3 grid(H, B);
   kv_decode_attention_kernel<<<grid, 128, static_cast<size_t>(s_max) * sizeof(float), stream>>>(
-      q, k, v, cache_k, cache_v, pos, H, dh, s_max, rsqrtf(static_cast<float>(dh)), out);
+      q, k, v, cache_k, cache_v, pos, H, dh, s_max, scale, out);
   return cudaGetLastError() == cudaSuccess ? 0 : 912;
 }
 

@@ -195,6 +195,27 @@ def test_decode_attention_kernel_extends_the_cache_and_matches_torch(cb):
         assert _rel(out, ref) < 1e-5
 
 
+@pytest.mark.parametrize("B,H,dh,S", [(1, 16, 80, 512), (1, 2, 128, 1000), (6, 16, 128, 512), (5, 3, 36, 100),
+                                      (40, 16, 64, 70), (2, 2, 20, 40), (3, 1, 30, 64)])
+def test_decode_attention_over_split_positions(cb, B, H, dh, S):
+    """Clusters of one to eight CTAs, groups without a position of their own, head rows that
+    are no multiple of the lanes' chunks, and (dh = 30) the kernel for unaligned rows.  fp32
+    throughout: the two sides differ by the order of the sums."""
+    from dawn_srw_b200.ops import reference as R
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(S)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    ck, cv = rn(B, H, S, dh), rn(B, H, S, dh)
+    be = cb.CudaBackend()
+    for pos in (0, 1, 31, 33, S // 2, S - 1):
+        q, k, v = rn(B, H * dh), rn(B, H * dh), rn(B, H * dh)
+        ck[:, :, pos], cv[:, :, pos] = 7.0, float("nan")       # the call has to overwrite the slot
+        out = be.decode_attention(q, k, v, ck, cv, torch.tensor([pos], device=dev), H)
+        assert torch.equal(ck[:, :, pos].reshape(B, -1), k) and torch.equal(cv[:, :, pos].reshape(B, -1), v)
+        ref = R.cached_attention(q.view(B, H, 1, dh), ck, cv, pos + 1).reshape(B, H * dh)
+        assert _rel(out, ref) < 1e-5
+
+
 def test_score_statistics_of_a_few_rows(cb):
     """The one-launch statistics kernel of the generation path against fp32 torch."""
     from dawn_srw_b200.ops.score_stats import score_stats_rows
