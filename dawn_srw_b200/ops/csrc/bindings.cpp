@@ -790,6 +790,52 @@ std::vector<Tensor> score_stats_bwd(c10::optional<Tensor> d_tau, c10::optional<T
   return {dh, w.slice(1, 0, r), d_off, d_esum};
 }
 
+// -> lb [] , m_u [U], stat [2]
+std::vector<Tensor> load_balance_fwd(const Tensor& emb, const Tensor& hsum, double inv_n, double units) {
+  check_bf16_2d(emb, "emb");
+  const c10::cuda::CUDAGuard guard(emb.device());
+  const int U = emb.size(0), r = emb.size(1);
+  TORCH_CHECK(hsum.is_cuda() && hsum.scalar_type() == torch::kFloat32 && hsum.is_contiguous() &&
+              hsum.numel() == r);
+  auto o = hsum.options();
+  auto lb = torch::empty({}, o), m_u = torch::empty({U}, o), stat = torch::empty({2}, o),
+       part = torch::empty({2 * dsb_load_balance_blocks(U, r)}, o);
+  int rc = dsb_load_balance_fwd(emb.data_ptr(), emb.stride(0), hsum.data_ptr<float>(), inv_n, units, U, r,
+                                m_u.data_ptr<float>(), part.data_ptr<float>(), lb.data_ptr<float>(),
+                                stat.data_ptr<float>(), cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_load_balance_fwd failed with code ", rc);
+  return {lb, m_u, stat};
+}
+
+// -> dmn [U], d_hsum [r]
+std::vector<Tensor> load_balance_bwd(const Tensor& emb, const Tensor& m_u, const Tensor& stat,
+                                     const Tensor& g_lb, double inv_n, double units) {
+  check_bf16_2d(emb, "emb");
+  const c10::cuda::CUDAGuard guard(emb.device());
+  const int U = emb.size(0), r = emb.size(1);
+  TORCH_CHECK(g_lb.is_cuda() && g_lb.scalar_type() == torch::kFloat32 && g_lb.numel() == 1 &&
+              m_u.numel() == U && m_u.is_contiguous() && stat.numel() == 2);
+  auto dmn = torch::empty({U}, m_u.options()), d_hsum = torch::zeros({r}, m_u.options());
+  int rc = dsb_load_balance_bwd(emb.data_ptr(), emb.stride(0), m_u.data_ptr<float>(), stat.data_ptr<float>(),
+                                g_lb.data_ptr<float>(), inv_n, units, U, r, dmn.data_ptr<float>(),
+                                d_hsum.data_ptr<float>(), cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_load_balance_bwd failed with code ", rc);
+  return {dmn, d_hsum};
+}
+
+void rank1_add(Tensor& g, const Tensor& dm, const Tensor& hs) {
+  const int L = dm.size(0), U = dm.size(1), r = hs.size(1);
+  TORCH_CHECK(g.is_cuda() && g.dim() == 2 && g.scalar_type() == torch::kFloat32 && g.size(0) == U &&
+              g.size(1) == r && g.stride(1) == 1 && g.stride(0) % 4 == 0 &&
+              (reinterpret_cast<uintptr_t>(g.data_ptr()) & 15) == 0);
+  TORCH_CHECK(dm.scalar_type() == torch::kFloat32 && dm.is_contiguous() && hs.is_contiguous() &&
+              hs.scalar_type() == torch::kFloat32 && hs.size(0) == L);
+  const c10::cuda::CUDAGuard guard(g.device());
+  int rc = dsb_rank1_add(g.data_ptr<float>(), g.stride(0), dm.data_ptr<float>(), hs.data_ptr<float>(), L, U,
+                         r, cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_rank1_add failed with code ", rc);
+}
+
 void adamw_multi(std::vector<Tensor> params, std::vector<Tensor> grads, std::vector<Tensor> exp_avg,
                  std::vector<Tensor> exp_avg_sq, const Tensor& clip_scale, double lr, double b1,
                  double b2, double eps, double wd, double bc1, double bc2) {
@@ -863,6 +909,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("score_stats_fwd", &score_stats_fwd);
   m.def("score_stats_bwd", &score_stats_bwd);
   m.def("score_stats_rows", &score_stats_rows);
+  m.def("load_balance_fwd", &load_balance_fwd);
+  m.def("load_balance_bwd", &load_balance_bwd);
+  m.def("rank1_add", &rank1_add);
   m.def("srw_rows", &srw_rows);
   m.def("gemv_rows", &gemv_rows);
   m.def("dropout", &dropout);

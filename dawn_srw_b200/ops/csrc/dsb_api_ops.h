@@ -76,6 +76,22 @@ int dsb_score_stats_bwd(const float* d_tau, const float* d_isd, const float* d_h
                         float inv_u, int N, int r, float* dh, void* w_bf16, long long ldw,
                         float* d_off, float* d_esum, cudaStream_t stream);
 
+// Load-balance term of a pool from the column sums of h: m_u = <e_u, hsum> * inv_n [U],
+//   lb = var / (mean^2 + var + 0.01) with mean = sum m_u / units, var = sum m_u^2 / units - mean^2.
+// emb bf16 [U, lde], r and lde multiples of 8, r <= 512.  part: 2 * dsb_load_balance_blocks floats of
+// scratch; m_u and stat [2] are kept for the backward call, which writes dmn [U] (= d m_u * inv_n)
+// and accumulates d_hsum [r] (zero it first); the embedding gradient is dmn[u] * hsum.
+int dsb_load_balance_blocks(int U, int r);
+int dsb_load_balance_fwd(const void* emb_bf16, long long lde, const float* hsum, float inv_n,
+                         float units, int U, int r, float* m_u, float* part, float* lb, float* stat,
+                         cudaStream_t stream);
+int dsb_load_balance_bwd(const void* emb_bf16, long long lde, const float* m_u, const float* stat,
+                         const float* g_lb, float inv_n, float units, int U, int r, float* dmn,
+                         float* d_hsum, cudaStream_t stream);
+// g[u, :] += sum_l dm[l, u] * hs[l, :]  (g fp32 [U, ldg], dm [L, U], hs [L, r], r % 4 == 0).
+int dsb_rank1_add(float* g, long long ldg, const float* dm, const float* hs, int L, int U, int r,
+                  cudaStream_t stream);
+
 // SRW pool op for a handful of token rows (decoding): one streaming pass over the pool.
 // h [N, r], x [N, D] bf16 contiguous (row n of x belongs to row n of h), tau / isd [N];
 // emb / read / write bf16 with row strides in elements (multiples of 8); unit_mask [U] or null.

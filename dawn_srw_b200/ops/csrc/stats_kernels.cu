@@ -208,6 +208,214 @@ __global__ void score_stats_rows_kernel(const float* __restrict__ h, long long h
   }
 }
 
+// ------------------------------------------------------------ load balance
+// m_u = <e_u, hbar>, hbar = hsum * inv_n (mean score of unit u over the tokens), and from it
+//   lb = var / (mean^2 + var + 0.01),   mean = sum_u m_u / U,   var = sum_u m_u^2 / U - mean^2.
+// The op reads the pool's bf16 embedding rows once (51 MB for 100 000 units of 256) and is bound
+// by those bytes at that size, by its launches below a few MB; so it is one pass that also takes
+// the sums (per-block partials, fixed order), and one block that finishes the scalar.  As a chain
+// of tensor ops on an fp32 copy of the rows it was 14 launches forward and about 35 backward.
+// A unit belongs to `lpu` lanes (a power of two), each with every lpu-th 16-byte chunk of the row.
+constexpr int kLbThreads = 256, kLbUnroll = 4;
+constexpr float kLbEps = 1e-2f;
+
+__device__ __forceinline__ void unpack_bf16x8(const uint4& q, float (&f)[8]) {
+  const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 v = __bfloat1622float2(h2[i]);
+    f[2 * i] = v.x;
+    f[2 * i + 1] = v.y;
+  }
+}
+
+// KC: chunks per lane (r <= 8 * lpu * KC).
+template <int KC>
+__global__ void __launch_bounds__(kLbThreads) lb_fwd_kernel(const __nv_bfloat16* __restrict__ emb,
+                                                            long long lde, const float* __restrict__ hsum,
+                                                            float inv_n, int U, int r, int lpu,
+                                                            float* __restrict__ m_u,
+                                                            float* __restrict__ part) {
+  __shared__ float s_red[2][kLbThreads / 32];
+  const int lane = threadIdx.x & 31, sub = lane & (lpu - 1), chunks = r >> 3;
+  const int per_warp = 32 / lpu;
+  float hb[KC][8];
+#pragma unroll
+  for (int k = 0; k < KC; ++k) {
+    const int c = sub + lpu * k;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) hb[k][j] = c < chunks ? hsum[8 * c + j] * inv_n : 0.f;
+  }
+  const int stride = gridDim.x * (kLbThreads / 32) * per_warp;
+  const int first = (blockIdx.x * (kLbThreads / 32) + (threadIdx.x >> 5)) * per_warp;   // of the warp
+  float s1 = 0.f, s2 = 0.f;
+  for (int u0 = first; u0 < U; u0 += kLbUnroll * stride) {                // warp-uniform trip count
+    uint4 q[kLbUnroll][KC];
+#pragma unroll
+    for (int i = 0; i < kLbUnroll; ++i) {
+      const int u = u0 + i * stride + lane / lpu;
+#pragma unroll
+      for (int k = 0; k < KC; ++k) {
+        const int c = sub + lpu * k;
+        q[i][k] = u < U && c < chunks
+                      ? *reinterpret_cast<const uint4*>(emb + static_cast<size_t>(u) * lde + 8 * c)
+                      : make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kLbUnroll; ++i) {
+      const int u = u0 + i * stride + lane / lpu;
+      float a = 0.f;
+#pragma unroll
+      for (int k = 0; k < KC; ++k) {
+        float e[8];
+        unpack_bf16x8(q[i][k], e);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a = fmaf(e[j], hb[k][j], a);
+      }
+      for (int o = lpu >> 1; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (sub == 0 && u < U) {
+        m_u[u] = a;
+        s1 += a;
+        s2 = fmaf(a, a, s2);
+      }
+    }
+  }
+  s1 = warp_sum(s1);
+  s2 = warp_sum(s2);
+  if (lane == 0) { s_red[0][threadIdx.x >> 5] = s1; s_red[1][threadIdx.x >> 5] = s2; }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < kLbThreads / 32; ++w) t += s_red[threadIdx.x][w];
+    part[2 * blockIdx.x + threadIdx.x] = t;
+  }
+}
+
+// lb[0] and stat = (mean, mean^2 + var + eps) from the blocks' partial sums.
+__global__ void __launch_bounds__(256) lb_finish_kernel(const float* __restrict__ part, int blocks,
+                                                        float units, float* __restrict__ lb,
+                                                        float* __restrict__ stat) {
+  __shared__ float s_red[2][8];
+  float s1 = 0.f, s2 = 0.f;
+  for (int b = threadIdx.x; b < blocks; b += 256) { s1 += part[2 * b]; s2 += part[2 * b + 1]; }
+  s1 = warp_sum(s1);
+  s2 = warp_sum(s2);
+  if ((threadIdx.x & 31) == 0) { s_red[0][threadIdx.x >> 5] = s1; s_red[1][threadIdx.x >> 5] = s2; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s1 = s2 = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) { s1 += s_red[0][w]; s2 += s_red[1][w]; }
+    const float mean = s1 / units, var = s2 / units - mean * mean;
+    const float q = mean * mean + var + kLbEps;
+    lb[0] = var / q;
+    stat[0] = mean;
+    stat[1] = q;
+  }
+}
+
+// With q = mean^2 + var + eps:  d mean = -2 mean / q,  d (sum m^2 / U) = (mean^2 + eps) / q^2, so
+//   dm_u = g / U * (d mean + 2 m_u d(sum m^2 / U)),   dmn[u] = dm_u * inv_n,
+//   d_hsum += sum_u dmn[u] e_u.   The embedding gradient dmn[u] * hsum is left to
+// rank1_add_kernel, which takes the calls of all layers in one pass over the gradient buffer.
+template <int KC>
+__global__ void __launch_bounds__(kLbThreads) lb_bwd_kernel(const __nv_bfloat16* __restrict__ emb,
+                                                            long long lde, const float* __restrict__ m_u,
+                                                            const float* __restrict__ stat,
+                                                            const float* __restrict__ g_lb, float units,
+                                                            float inv_n, int U, int r, int lpu,
+                                                            float* __restrict__ dmn,
+                                                            float* __restrict__ d_hsum) {
+  __shared__ float s_sum[kMaxR];
+  for (int j = threadIdx.x; j < r; j += kLbThreads) s_sum[j] = 0.f;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, sub = lane & (lpu - 1), chunks = r >> 3;
+  const int per_warp = 32 / lpu;
+  const float mean = stat[0], q = stat[1], g = g_lb[0] * inv_n / units;
+  const float c0 = -2.f * mean / q * g, c1 = 2.f * (fmaf(mean, mean, kLbEps) / q) / q * g;
+  float acc[KC][8];
+#pragma unroll
+  for (int k = 0; k < KC; ++k)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[k][j] = 0.f;
+  const int stride = gridDim.x * (kLbThreads / 32) * per_warp;
+  const int first = (blockIdx.x * (kLbThreads / 32) + (threadIdx.x >> 5)) * per_warp;
+  for (int u0 = first; u0 < U; u0 += kLbUnroll * stride) {
+    uint4 e4[kLbUnroll][KC];
+    float d[kLbUnroll];
+#pragma unroll
+    for (int i = 0; i < kLbUnroll; ++i) {
+      const int u = u0 + i * stride + lane / lpu;
+      d[i] = u < U ? fmaf(c1, m_u[u], c0) : 0.f;
+#pragma unroll
+      for (int k = 0; k < KC; ++k) {
+        const int c = sub + lpu * k;
+        e4[i][k] = u < U && c < chunks
+                       ? *reinterpret_cast<const uint4*>(emb + static_cast<size_t>(u) * lde + 8 * c)
+                       : make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kLbUnroll; ++i) {
+      const int u = u0 + i * stride + lane / lpu;
+      if (sub == 0 && u < U) dmn[u] = d[i];
+#pragma unroll
+      for (int k = 0; k < KC; ++k) {
+        float e[8];
+        unpack_bf16x8(e4[i][k], e);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[k][j] = fmaf(d[i], e[j], acc[k][j]);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < KC; ++k) {
+    const int c = sub + lpu * k;
+    if (c < chunks) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) atomicAdd(&s_sum[8 * c + j], acc[k][j]);
+    }
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < r; j += kLbThreads) atomicAdd(d_hsum + j, s_sum[j]);
+}
+
+// g[u, :] += sum_l dm[l, u] * hs[l, :] (fp32 [U, r], row stride ldg): one read and write of the
+// gradient rows for up to kRank1Max layers instead of one per layer.
+constexpr int kRank1Max = 24;
+__global__ void __launch_bounds__(256) rank1_add_kernel(float* __restrict__ g, long long ldg,
+                                                        const float* __restrict__ dm,
+                                                        const float* __restrict__ hs, int L, int U,
+                                                        int r) {
+  extern __shared__ __align__(16) float s_hs[];                  // [L][r]
+  for (int i = threadIdx.x; i < L * r; i += 256) s_hs[i] = hs[i];
+  __syncthreads();
+  const int c4 = r >> 2;
+  const long long total = static_cast<long long>(U) * c4;
+  for (long long i = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x; i < total;
+       i += static_cast<long long>(gridDim.x) * 256) {
+    const int u = static_cast<int>(i / c4), c = static_cast<int>(i - static_cast<long long>(u) * c4);
+    float4* dst = reinterpret_cast<float4*>(g + static_cast<size_t>(u) * ldg) + c;
+    float4 a = *dst;
+#pragma unroll 4
+    for (int l = 0; l < L; ++l) {
+      const float d = dm[static_cast<size_t>(l) * U + u];
+      const float4 h = *reinterpret_cast<const float4*>(s_hs + l * r + 4 * c);
+      a.x = fmaf(d, h.x, a.x); a.y = fmaf(d, h.y, a.y);
+      a.z = fmaf(d, h.z, a.z); a.w = fmaf(d, h.w, a.w);
+    }
+    *dst = a;
+  }
+}
+
+int lb_lanes(int r) {
+  int lpu = 1;
+  while (lpu < 32 && 8 * lpu < r) lpu *= 2;
+  return lpu;
+}
+
 int stats_grid(int N) {
   const int blocks = (N + 7) / 8;
   return blocks < 148 * 4 ? (blocks < 1 ? 1 : blocks) : 148 * 4;
@@ -252,5 +460,50 @@ extern "C" int dsb_score_stats_rows(const float* h, long long h_st, long long h_
   score_stats_rows_kernel<<<T * R, kRowGroups * kRowThreads, 0, stream>>>(h, h_st, h_sr, off, o_st, o_sr, gram, esum, inv_u,
                                                      T, r, tau, isd,
                                                      static_cast<__nv_bfloat16*>(hb_bf16));
+  return cudaGetLastError() == cudaSuccess ? 0 : 802;
+}
+
+extern "C" int dsb_load_balance_blocks(int U, int r) {
+  const int warps_units = (kLbThreads / 32) * (32 / lb_lanes(r));      // units of a block per pass
+  const int b = (U + warps_units - 1) / warps_units;
+  return b < 148 * 4 ? (b < 1 ? 1 : b) : 148 * 4;
+}
+
+extern "C" int dsb_load_balance_fwd(const void* emb_bf16, long long lde, const float* hsum, float inv_n,
+                                    float units, int U, int r, float* m_u, float* part, float* lb,
+                                    float* stat, cudaStream_t stream) {
+  if (U <= 0 || r <= 0 || r > kMaxR || r % 8 != 0 || lde % 8 != 0) return 803;
+  const int lpu = lb_lanes(r), blocks = dsb_load_balance_blocks(U, r);
+  const __nv_bfloat16* e = static_cast<const __nv_bfloat16*>(emb_bf16);
+  if (r <= 8 * lpu) lb_fwd_kernel<1><<<blocks, kLbThreads, 0, stream>>>(e, lde, hsum, inv_n, U, r, lpu, m_u, part);
+  else lb_fwd_kernel<2><<<blocks, kLbThreads, 0, stream>>>(e, lde, hsum, inv_n, U, r, lpu, m_u, part);
+  lb_finish_kernel<<<1, 256, 0, stream>>>(part, blocks, units, lb, stat);
+  return cudaGetLastError() == cudaSuccess ? 0 : 802;
+}
+
+extern "C" int dsb_load_balance_bwd(const void* emb_bf16, long long lde, const float* m_u,
+                                    const float* stat, const float* g_lb, float inv_n, float units,
+                                    int U, int r, float* dmn, float* d_hsum, cudaStream_t stream) {
+  if (U <= 0 || r <= 0 || r > kMaxR || r % 8 != 0 || lde % 8 != 0) return 803;
+  const int lpu = lb_lanes(r), blocks = dsb_load_balance_blocks(U, r);
+  const __nv_bfloat16* e = static_cast<const __nv_bfloat16*>(emb_bf16);
+  if (r <= 8 * lpu)
+    lb_bwd_kernel<1><<<blocks, kLbThreads, 0, stream>>>(e, lde, m_u, stat, g_lb, units, inv_n, U, r, lpu, dmn, d_hsum);
+  else
+    lb_bwd_kernel<2><<<blocks, kLbThreads, 0, stream>>>(e, lde, m_u, stat, g_lb, units, inv_n, U, r, lpu, dmn, d_hsum);
+  return cudaGetLastError() == cudaSuccess ? 0 : 802;
+}
+
+extern "C" int dsb_rank1_add(float* g, long long ldg, const float* dm, const float* hs, int L, int U,
+                             int r, cudaStream_t stream) {
+  if (L <= 0 || U <= 0) return 0;
+  if (r <= 0 || r > kMaxR || r % 4 != 0 || ldg % 4 != 0) return 803;
+  const long long n = static_cast<long long>(U) * (r >> 2);
+  const int blocks = static_cast<int>(n / 256 + 1 < 148 * 8 ? n / 256 + 1 : 148 * 8);
+  for (int l0 = 0; l0 < L; l0 += kRank1Max) {
+    const int cnt = L - l0 < kRank1Max ? L - l0 : kRank1Max;      // 24 x 512 floats = 48 KB
+    rank1_add_kernel<<<blocks, 256, static_cast<size_t>(cnt) * r * sizeof(float), stream>>>(
+        g, ldg, dm + static_cast<size_t>(l0) * U, hs + static_cast<size_t>(l0) * r, cnt, U, r);
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : 802;
 }

@@ -277,12 +277,13 @@ class _LayerNormFn(torch.autograd.Function):
 # ---------------------------------------------------------------------------
 class _PoolTensors:
     """bf16 compute copies of a pool and the fp32 gradient accumulators of the current step."""
-    __slots__ = ("emb", "read", "write", "g_emb", "g_read", "g_write", "emb_f", "__weakref__")
+    __slots__ = ("emb", "read", "write", "g_emb", "g_read", "g_write", "emb_f", "rank1", "__weakref__")
 
     def __init__(self):
         self.emb = self.read = self.write = None
         self.g_emb = self.g_read = self.g_write = None
         self.emb_f = None          # fp32 copy of emb for the per-unit mat-vecs (made on first use)
+        self.rank1 = []            # (d m_u, hsum) of the load-balance terms: g_emb += sum d m_u (x) hsum
 
 
 def _on_tensors(name):
@@ -362,6 +363,11 @@ class _PoolPrepFn(torch.autograd.Function):
                 g_emb[:U] += hd.emb[:U].float() @ sym
         if d_esum is not None:
             g_emb[:U] += d_esum.unsqueeze(0)
+        if hd.rank1:
+            pairs, hd.rank1 = hd.rank1, []
+            count_launches(1)
+            ext().rank1_add(g_emb[:U], torch.stack([d for d, _ in pairs]),
+                            torch.stack([h for _, h in pairs]))
 
         def chain(g, w, nrm):
             if not ctx.normalize:
@@ -397,6 +403,31 @@ class _PoolMatVecFn(torch.autograd.Function):
         hd, U = ctx.holder, ctx.U
         hd.g_emb[:U].addr_(dm, v)
         return _emb_f32(hd)[:U].t() @ dm, torch.zeros_like(dm[:1]), None, None
+
+
+class _LoadBalanceFn(torch.autograd.Function):
+    """Load-balance term of one call from the column sums of h (see stats_kernels.cu: one pass
+    over the bf16 embedding rows each way).  The embedding gradient of a call is an outer
+    product; the pool's preparation node adds those of all layers at once."""
+    @staticmethod
+    def forward(ctx, hsum, anchor, holder, U, inv_n, units):
+        hsum = hsum.detach().contiguous()
+        lb, m_u, stat = ext().load_balance_fwd(holder.emb[:U], hsum, inv_n, units)
+        count_launches(2)
+        ctx.holder, ctx.args = holder, (U, inv_n, units)
+        ctx.save_for_backward(hsum, m_u, stat)
+        return lb
+
+    @staticmethod
+    def backward(ctx, g):
+        hsum, m_u, stat = ctx.saved_tensors
+        U, inv_n, units = ctx.args
+        hd = ctx.holder
+        dmn, d_hsum = ext().load_balance_bwd(hd.emb[:U], m_u, stat, g.float().contiguous(), inv_n, units)
+        count_launches(1)
+        if hd.g_emb is not None:
+            hd.rank1.append((dmn, hsum))
+        return d_hsum, None, None, None, None, None
 
 
 def _route_backward_core(x_bf, h_bf, tau, inv_sd, dy, d_den, hd, spec, U, xr=None):
@@ -1098,13 +1129,17 @@ class CudaBackend:
         x_bf = _bf16_2d(x)
         tau, inv_sd, hsum, h_bf3 = score_stats(h, tau_off, ex["gram"], ex["esum"], U_tot,
                                                ex["gram_split"])
-        hbar = hsum / float(T * Rr)
-        m_u = _PoolMatVecFn.apply(hbar, anchor, pool, U)
-        ns_sum = C.mean_over_group(m_u.sum(), pctx.dp_group)
-        ns_sq = C.mean_over_group((m_u * m_u).sum(), pctx.dp_group)
-        mean_score = ns_sum / U_tot
-        var_score = ns_sq / U_tot - mean_score ** 2
-        lb = var_score / (mean_score ** 2 + var_score + 1e-2)
+        if spec.has_dead_penalty or C.group_size(pctx.dp_group) > 1:
+            # the per-unit means are needed by themselves, or have to meet other ranks'
+            hbar = hsum / float(T * Rr)
+            m_u = _PoolMatVecFn.apply(hbar, anchor, pool, U)
+            ns_sum = C.mean_over_group(m_u.sum(), pctx.dp_group)
+            ns_sq = C.mean_over_group((m_u * m_u).sum(), pctx.dp_group)
+            mean_score = ns_sum / U_tot
+            var_score = ns_sq / U_tot - mean_score ** 2
+            lb = var_score / (mean_score ** 2 + var_score + 1e-2)
+        else:
+            lb = _LoadBalanceFn.apply(hsum, anchor, pool.tensors, U, 1.0 / (T * Rr), float(U_tot))
         alive = torch.zeros(U, dtype=torch.uint8, device=x.device) if spec.has_dead_penalty else None
         um = None if unit_mask is None else unit_mask[:U].float().contiguous()
         if out_scale is None:

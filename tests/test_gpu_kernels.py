@@ -752,3 +752,39 @@ def test_training_reduces_loss_on_gpu(cb):
 def test_graft_entry_smoke():
     import __graft_entry__ as g
     g.smoke()
+
+
+@pytest.mark.parametrize("U,r,layers", [(1, 8, 1), (7, 16, 2), (130, 128, 3), (1001, 256, 30), (2600, 384, 2),
+                                        (77, 512, 25)])
+def test_load_balance_term_and_its_gradients(cb, U, r, layers):
+    """One lane to a warp per unit, one or two chunks per lane, more layers than one launch of the
+    outer products takes.  fp32 sums of up to U terms against fp64: 1e-5 covers sqrt(U) roundings;
+    var is a difference of nearly equal numbers only where the mean dominates, which it does not."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(U + r)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    hd = cb._PoolTensors()
+    hd.emb = rn(U + 3, r).bfloat16()
+    hd.g_emb = rn(U + 3, r)
+    ref_e = hd.emb[:U].double().requires_grad_(True)
+    start = hd.g_emb.clone()
+    total = 0.0
+    for k in range(layers):
+        hsum = (rn(r) * 40).requires_grad_(True)
+        lb = cb._LoadBalanceFn.apply(hsum, torch.zeros(1, device=dev), hd, U, 1.0 / 96, float(U))
+        (lb * (k + 1.5)).backward()
+        hs = hsum.detach().double().requires_grad_(True)
+        m = ref_e @ (hs / 96)
+        mean = m.sum() / U
+        var = (m * m).sum() / U - mean ** 2
+        ref = var / (mean ** 2 + var + 1e-2)
+        (ref * (k + 1.5)).backward()
+        assert abs(float(lb) - float(ref)) < 1e-5
+        assert float((hsum.grad.double() - hs.grad).norm()) < 1e-4 * float(hs.grad.norm()) + 1e-6
+    pairs, hd.rank1 = hd.rank1, []
+    cb.ext().rank1_add(hd.g_emb[:U], torch.stack([d for d, _ in pairs]), torch.stack([h for _, h in pairs]))
+    added = (hd.g_emb - start).double()
+    assert float(added[U:].abs().max()) == 0.0
+    # every layer's product is added to a value of order one: 2^-24 of rounding per element each
+    rounding = 2.0 ** -24 * (layers * U * r) ** 0.5
+    assert float((added[:U] - ref_e.grad).norm()) < 1e-4 * float(ref_e.grad.norm()) + rounding + 1e-6
