@@ -642,12 +642,153 @@ std::vector<Tensor> score_stats_fwd(const Tensor& hg, const Tensor& h, const Ten
   auto o = hg.options();
   auto tau = torch::empty({N}, o), isd = torch::empty({N}, o), mu = torch::empty({N}, o),
        sd = torch::empty({N}, o), hsum = torch::zeros({r}, o);
-  int rc = dsb_score_stats_fwd(hg.data_ptr<float>(), h.data_ptr(), h.stride(0),
-                               esum.data_ptr<float>(), off.data_ptr<float>(), inv_u, N, r,
+  int rc = dsb_score_stats_fwd(hg.data_ptr<float>(), nullptr, r, h.data_ptr(), h.stride(0),
+                               esum.data_ptr<float>(), off.data_ptr<float>(), 1, 0, N, inv_u, N, r,
                                tau.data_ptr<float>(), isd.data_ptr<float>(), mu.data_ptr<float>(),
                                sd.data_ptr<float>(), hsum.data_ptr<float>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_score_stats_fwd failed with code ", rc);
   return {tau, isd, mu, sd, hsum};
+}
+
+bool f32(const Tensor& t) { return t.is_cuda() && t.scalar_type() == torch::kFloat32; }
+
+// Statistics of a pool call, routes stacked (row ri * T + t): h fp32 [T, R, r], off [T, R],
+// gcat bf16 [2r, r] = the two bf16 terms of G.  -> hb bf16 [R*T, r], hg fp32 [R*T, 2r] (its halves
+// add up to h . G), tau, isd, mu, sd [R*T], den [R, T] (zeros), hsum [r].
+std::vector<Tensor> srw_stats(const Tensor& h, const Tensor& off, const Tensor& gcat, const Tensor& esum,
+                              double inv_u, Tensor& status) {
+  TORCH_CHECK(f32(h) && h.dim() == 3 && h.stride(2) == 1 && f32(off) && off.dim() == 2 &&
+              off.size(0) == h.size(0) && off.size(1) == h.size(1), "srw_stats: bad h or off");
+  const int T = h.size(0), R = h.size(1), r = h.size(2), N = T * R;
+  check_bf16_2d(gcat, "gcat");
+  TORCH_CHECK(gcat.size(0) == 2 * r && gcat.size(1) == r && r % 8 == 0 && f32(esum) &&
+              esum.is_contiguous() && esum.numel() == r, "srw_stats: bad Gram matrix");
+  const c10::cuda::CUDAGuard guard(h.device());
+  auto o = h.options();
+  auto hb = torch::empty({N, r}, o.dtype(torch::kBFloat16)), hg = torch::empty({N, 2 * r}, o);
+  auto rows = torch::empty({4 * static_cast<int64_t>(N)}, o), den = torch::empty({R, T}, o),
+       hsum = torch::empty({r}, o);
+  float *tau = rows.data_ptr<float>(), *isd = tau + N, *mu = isd + N, *sd = mu + N;
+  int rc = dsb_score_pack(h.data_ptr<float>(), h.stride(0), h.stride(1), T, R, r, hb.data_ptr(),
+                          den.data_ptr<float>(), N, hsum.data_ptr<float>(), r, cur_stream());
+  if (rc == 0)
+    rc = dsb_gemm_bf16(hb.data_ptr(), 0, r, gcat.data_ptr(), 0, gcat.stride(0), N, 2 * r, r, hg.data_ptr(),
+                       2 * r, 0, 0, 1.f, nullptr, nullptr, 2 * r <= 128 ? 128 : 256,
+                       status.data_ptr<int>(), cur_stream());
+  if (rc == 0)
+    rc = dsb_score_stats_fwd(hg.data_ptr<float>(), hg.data_ptr<float>() + r, 2 * r, hb.data_ptr(), r,
+                             esum.data_ptr<float>(), off.data_ptr<float>(), off.stride(0), off.stride(1), T,
+                             inv_u, N, r, tau, isd, mu, sd, hsum.data_ptr<float>(), cur_stream());
+  TORCH_CHECK(rc == 0, "srw_stats failed with code ", rc);
+  auto part = [&](int k) { return rows.narrow(0, static_cast<int64_t>(k) * N, N); };
+  return {hb, hg, part(0), part(1), part(2), part(3), den, hsum};
+}
+
+// One route: gate kernel into p (scratch; xr too where given), then the write GEMM with the
+// normalisation in its epilogue into y fp32 [T, D] (accumulate: y is zeroed, splits of U add up).
+void srw_route_fwd(const Tensor& h, const Tensor& x, const Tensor& emb, const Tensor& read,
+                   const Tensor& write, Tensor& p, c10::optional<Tensor> xr, const Tensor& tau,
+                   const Tensor& isd, Tensor& den, c10::optional<Tensor> diag,
+                   c10::optional<Tensor> alive, c10::optional<Tensor> unit_mask, std::vector<double> gate,
+                   double scale, c10::optional<Tensor> scale_t, Tensor& y, bool accumulate,
+                   Tensor& status) {
+  check_bf16_2d(h, "h"); check_bf16_2d(x, "x"); check_bf16_2d(emb, "emb"); check_bf16_2d(read, "read");
+  check_bf16_2d(write, "write"); check_bf16_2d(p, "p");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int T = x.size(0), D = x.size(1), U = emb.size(0), r = emb.size(1);
+  TORCH_CHECK(h.size(0) == T && h.size(1) == r && read.size(0) == U && read.size(1) == D &&
+              write.size(0) == U && write.size(1) == D && p.size(0) >= T && p.size(1) >= U);
+  TORCH_CHECK(f32(y) && y.dim() == 2 && y.size(0) == T && y.size(1) == D && y.stride(1) == 1);
+  auto vec = [&](const Tensor& t) { return f32(t) && t.is_contiguous() && t.numel() == T; };
+  TORCH_CHECK(vec(tau) && vec(isd) && vec(den));
+  void* xr_p = nullptr;
+  long long ldxr = 0;
+  if (xr.has_value() && xr->defined()) {
+    check_bf16_2d(*xr, "xr");
+    TORCH_CHECK(xr->size(0) == T && xr->size(1) >= U);
+    xr_p = xr->data_ptr();
+    ldxr = xr->stride(0);
+  }
+  float* diag_p = nullptr;
+  if (diag.has_value() && diag->defined()) {
+    TORCH_CHECK(f32(*diag) && diag->is_contiguous() && diag->numel() >= static_cast<int64_t>(T) * 12 + 2);
+    diag_p = diag->data_ptr<float>();
+  }
+  unsigned char* alive_p = nullptr;
+  if (alive.has_value() && alive->defined()) {
+    TORCH_CHECK(alive->scalar_type() == torch::kUInt8 && alive->numel() >= U);
+    alive_p = alive->data_ptr<unsigned char>();
+  }
+  const float* sp = nullptr;
+  if (scale_t.has_value() && scale_t->defined()) {
+    TORCH_CHECK(f32(*scale_t) && scale_t->numel() == 1);
+    sp = scale_t->data_ptr<float>();
+  }
+  DsbGate g = to_gate(gate);
+  int rc = dsb_srw_fwd_gate_xr(h.data_ptr(), h.stride(0), emb.data_ptr(), emb.stride(0), x.data_ptr(),
+                               x.stride(0), read.data_ptr(), read.stride(0), T, U, r, D, p.data_ptr(),
+                               p.stride(0), xr_p, ldxr, tau.data_ptr<float>(), isd.data_ptr<float>(),
+                               nullptr, den.data_ptr<float>(), nullptr, diag_p, alive_p,
+                               opt_f32(unit_mask), &g, nullptr, status.data_ptr<int>(), cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_srw_fwd_gate_xr failed with code ", rc);
+  rc = dsb_srw_write(p.data_ptr(), p.stride(0), write.data_ptr(), write.stride(0), T, U, D,
+                     den.data_ptr<float>(), scale, sp, y.data_ptr<float>(), y.stride(0), accumulate,
+                     status.data_ptr<int>(), cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_srw_write failed with code ", rc);
+}
+
+// -> dy bf16 [T, D], d_den [T]; dtau [T] is zeroed, d_scale (optional) accumulated
+std::vector<Tensor> route_bwd_rows(const Tensor& dy, const Tensor& y, const Tensor& den, double scale,
+                                   c10::optional<Tensor> scale_t, c10::optional<Tensor> ext_dden,
+                                   Tensor& dtau, c10::optional<Tensor> d_scale) {
+  const int T = dy.size(0), D = dy.size(1);
+  auto ok = [&](const Tensor& t, int64_t n) {
+    return f32(t) && t.is_contiguous() && t.numel() == n && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 3) == 0;
+  };
+  TORCH_CHECK(dy.dim() == 2 && ok(dy, static_cast<int64_t>(T) * D) && ok(y, static_cast<int64_t>(T) * D) &&
+              ok(den, T) && ok(dtau, T));
+  TORCH_CHECK(((reinterpret_cast<uintptr_t>(dy.data_ptr()) | reinterpret_cast<uintptr_t>(y.data_ptr())) & 15) == 0,
+              "route_bwd_rows: dy and y must be 16-byte aligned");
+  const c10::cuda::CUDAGuard guard(dy.device());
+  auto dyb = torch::empty({T, D}, dy.options().dtype(torch::kBFloat16)), d_den = torch::empty({T}, dy.options());
+  int rc = dsb_route_bwd_rows(dy.data_ptr<float>(), y.data_ptr<float>(), den.data_ptr<float>(),
+                              opt_f32(scale_t), scale, opt_f32(ext_dden), dyb.data_ptr(),
+                              d_den.data_ptr<float>(), dtau.data_ptr<float>(), opt_f32_mut(d_scale), T, D,
+                              cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_route_bwd_rows failed with code ", rc);
+  return {dyb, d_den};
+}
+
+// Row part of a pool call's backward and its Gram gradient: -> dh [T, R, r], d_off [T, R];
+// g_gram [r, r] and g_esum [r] are accumulated into.
+std::vector<Tensor> srw_stats_bwd(const Tensor& dtau, const Tensor& dh32, c10::optional<Tensor> d_hsum,
+                                  const Tensor& off, const Tensor& tau, const Tensor& isd, const Tensor& mu,
+                                  const Tensor& sd, const Tensor& hg, const Tensor& hb, const Tensor& esum,
+                                  double inv_u, bool sigma_path, c10::optional<Tensor> g_gram,
+                                  Tensor& g_esum, Tensor& status) {
+  const int T = off.size(0), R = off.size(1), N = hb.size(0), r = hb.size(1);
+  check_bf16_2d(hb, "hb");
+  auto ok = [&](const Tensor& t, int64_t n) { return f32(t) && t.is_contiguous() && t.numel() == n; };
+  TORCH_CHECK(N == T * R && f32(off) && hb.is_contiguous() && ok(dtau, N) &&
+              ok(dh32, static_cast<int64_t>(N) * r) && ok(tau, N) && ok(isd, N) && ok(mu, N) && ok(sd, N) &&
+              ok(hg, static_cast<int64_t>(N) * 2 * r) && ok(esum, r) && ok(g_esum, r), "srw_stats_bwd: bad shapes");
+  const c10::cuda::CUDAGuard guard(hb.device());
+  auto o = hg.options();
+  auto dh = torch::empty({T, R, r}, o), d_off = torch::empty({T, R}, o),
+       w = torch::empty({N, r}, o.dtype(torch::kBFloat16));
+  int rc = dsb_score_route_bwd(dtau.data_ptr<float>(), dh32.data_ptr<float>(), opt_f32(d_hsum),
+                               off.data_ptr<float>(), off.stride(0), off.stride(1), tau.data_ptr<float>(),
+                               isd.data_ptr<float>(), mu.data_ptr<float>(), sd.data_ptr<float>(),
+                               hg.data_ptr<float>(), hg.data_ptr<float>() + r, 2 * r, hb.data_ptr(),
+                               esum.data_ptr<float>(), inv_u, sigma_path, T, R, r, dh.data_ptr<float>(),
+                               w.data_ptr(), d_off.data_ptr<float>(), g_esum.data_ptr<float>(), cur_stream());
+  if (rc == 0 && g_gram.has_value() && g_gram->defined()) {
+    TORCH_CHECK(ok(*g_gram, static_cast<int64_t>(r) * r));
+    rc = dsb_gemm_bf16(w.data_ptr(), 1, r, hb.data_ptr(), 1, r, r, r, N, g_gram->data_ptr(), r, 0, 1, inv_u,
+                       nullptr, nullptr, r <= 128 ? 128 : 256, status.data_ptr<int>(), cur_stream());
+  }
+  TORCH_CHECK(rc == 0, "srw_stats_bwd failed with code ", rc);
+  return {dh, d_off};
 }
 
 // SRW pool op for up to four token rows in one streaming pass (decoding).
@@ -912,6 +1053,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("load_balance_fwd", &load_balance_fwd);
   m.def("load_balance_bwd", &load_balance_bwd);
   m.def("rank1_add", &rank1_add);
+  m.def("srw_stats", &srw_stats);
+  m.def("srw_route_fwd", &srw_route_fwd);
+  m.def("route_bwd_rows", &route_bwd_rows);
+  m.def("srw_stats_bwd", &srw_stats_bwd);
   m.def("srw_rows", &srw_rows);
   m.def("gemv_rows", &gemv_rows);
   m.def("dropout", &dropout);

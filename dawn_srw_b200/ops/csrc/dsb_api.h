@@ -47,6 +47,12 @@ int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_m
                   float alpha, const float* row_scale, const float* bias, int block_n,
                   int* status, cudaStream_t stream);
 
+// Write GEMM of a route, normalised in its epilogue: y[T, D] (=|+=) (p[T, U] . write[U, D]) *
+// norm / max(den[t], 1), y fp32; norm_ptr (device scalar) overrides norm when not null.
+int dsb_srw_write(const void* p, long long ldp, const void* write, long long ldw, int T, int U, int D,
+                  const float* den, float norm, const float* norm_ptr, float* y, long long ldy,
+                  int accumulate, int* status, cudaStream_t stream);
+
 // SRW forward gate kernel: p[T,U] = gate(h.emb^T; tau, 1/sigma) * (x.read^T),
 // den_sum[T] += sum_U den_term.  gate_sum / alive / unit_mask may be null.
 int dsb_srw_fwd_gate(const void* h, long long ldh, const void* emb, long long lde, const void* x,

@@ -48,6 +48,13 @@ int dsb_offdiag_abs(const float* sim, long long ld, int m, void* sgn_bf16, long 
 int dsb_route_bwd_prologue(const float* dy, const float* y, const float* row_scale,
                            void* dy_bf16, float* rowdot, int T, int D, cudaStream_t stream);
 
+// With rs = s / max(den, 1), s = *scale_ptr or scale: dy_bf = bf16(dy * rs); with rowdot = <dy, y>:
+// d_den = -rowdot / den where den > 1, else 0 (+ ext_dden, nullable); dtau = 0;
+// d_scale[0] += sum_t rowdot / s (nullable).  dy, y fp32 [T, D], D % 4 == 0, 16-byte aligned.
+int dsb_route_bwd_rows(const float* dy, const float* y, const float* den, const float* scale_ptr,
+                       float scale, const float* ext_dden, void* dy_bf16, float* d_den, float* dtau,
+                       float* d_scale, int T, int D, cudaStream_t stream);
+
 // y = res + dropout(x) (res may be null: y = dropout(x)); fp32, n % 4 == 0.  An element is kept
 // (and scaled by 1 / (1 - p)) iff a hash of (seed, its index) is >= p * 2^32, so the gradient
 // of x is the same call with res = null on the incoming gradient.
@@ -57,9 +64,25 @@ int dsb_dropout(const float* res, const float* x, float* y, long long n, unsigne
 // Per-token score statistics from hg = h . (E^T E) (fp32 [N, r]) and bf16 h [N, ldh]:
 //   mu = <h, esum> * inv_u,  var = <hg, h> * inv_u - mu^2,  sd = sqrt(max(var, 1e-12)) + 1e-8,
 //   tau = mu + off * sd,  isd = 1 / sd;  hsum[r] += column sums of h (hsum may be null).
-int dsb_score_stats_fwd(const float* hg, const void* h_bf16, long long ldh, const float* esum,
-                        const float* off, float inv_u, int N, int r, float* tau, float* isd,
+// hg has row stride ldg; hg2 (nullable) is a second part of it, added on the fly.  Row n is token
+// n % T of route n / T; its offset is off[t * o_st + route * o_sr].
+int dsb_score_stats_fwd(const float* hg, const float* hg2, long long ldg, const void* h_bf16,
+                        long long ldh, const float* esum, const float* off, long long o_st,
+                        long long o_sr, int T, float inv_u, int N, int r, float* tau, float* isd,
                         float* mu, float* sd, float* hsum, cudaStream_t stream);
+// hb[ri * T + t, :] = bf16(h[t, ri, :]) (h fp32, strides h_st, h_sr, unit inner stride, r % 8 == 0);
+// z1[0 .. n1) = z2[0 .. n2) = 0.
+int dsb_score_pack(const float* h, long long h_st, long long h_sr, int T, int R, int r, void* hb_bf16,
+                   float* z1, int n1, float* z2, int n2, cudaStream_t stream);
+// Row part of a call's backward (rows route-major, N = R * T): from dtau [N] and dh32 [N, r] of the
+// gate step, the sigma path (sigma_path != 0) and the statistics: dh fp32 [T, R, r], d_off [T, R],
+// w = bf16(d_var * h) [N, r] (operand of dG = w^T h * inv_u); accumulates d_esum [r].
+int dsb_score_route_bwd(const float* dtau, const float* dh32, const float* d_hsum, const float* off,
+                        long long o_st, long long o_sr, const float* tau, const float* isd,
+                        const float* mu, const float* sd, const float* hg, const float* hg2,
+                        long long ldg, const void* h_bf16, const float* esum, float inv_u,
+                        int sigma_path, int T, int R, int r, float* dh, void* w_bf16, float* d_off,
+                        float* d_esum, cudaStream_t stream);
 // The same statistics for a handful of rows in one launch (generation), from fp32 h [T, R, r]
 // (strides h_st, h_sr in elements, unit inner stride), off [T, R] (strides o_st, o_sr) and the
 // fp32 Gram matrix.  Output rows are route-major: row ri * T + t; hb is bf16(h) [R * T, r].

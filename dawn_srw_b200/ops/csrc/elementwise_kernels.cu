@@ -393,6 +393,55 @@ __global__ void route_bwd_prologue_kernel(const float* __restrict__ dy, const fl
   if (lane == 0) rowdot[t] = acc;
 }
 
+// The same for a route whose denominator and scale are still separate, with all that follows per
+// row: row_scale = s / max(den, 1);  d_den = -rowdot / den where den > 1 (+ ext_dden);
+// d_scale += sum_t rowdot / s;  dtau = 0 (the gate kernel adds into it).  One pass over dy and y
+// instead of that plus nine tensor ops on [T].
+__global__ void __launch_bounds__(256) route_bwd_rows_kernel(
+    const float* __restrict__ dy, const float* __restrict__ y, const float* __restrict__ den,
+    const float* __restrict__ scale_ptr, float scale, const float* __restrict__ ext_dden,
+    __nv_bfloat16* __restrict__ dy_bf, float* __restrict__ d_den, float* __restrict__ dtau,
+    float* __restrict__ d_scale, int T, int D) {
+  __shared__ float s_dot[8];
+  const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  float acc = 0.f;
+  const float sc = scale_ptr != nullptr ? scale_ptr[0] : scale;
+  if (t < T) {
+    const float dn = den[t];
+    const float rs = sc / (dn < 1.f ? 1.f : dn);                 // a NaN stays one
+    const float4* g = reinterpret_cast<const float4*>(dy + static_cast<size_t>(t) * D);
+    const float4* yy = reinterpret_cast<const float4*>(y + static_cast<size_t>(t) * D);
+    uint2* o = reinterpret_cast<uint2*>(dy_bf + static_cast<size_t>(t) * D);
+#pragma unroll 4
+    for (int i = lane; i < (D >> 2); i += 32) {
+      const float4 a = g[i], b = yy[i];
+      acc += a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x * rs, a.y * rs);
+      const __nv_bfloat162 hi = __floats2bfloat162_rn(a.z * rs, a.w * rs);
+      uint2 w;
+      w.x = *reinterpret_cast<const uint32_t*>(&lo);
+      w.y = *reinterpret_cast<const uint32_t*>(&hi);
+      o[i] = w;
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) {
+      d_den[t] = (dn > 1.f ? -acc / dn : 0.f) + (ext_dden != nullptr ? ext_dden[t] : 0.f);
+      dtau[t] = 0.f;
+    }
+  }
+  if (d_scale != nullptr) {
+    if (lane == 0) s_dot[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float tot = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) tot += s_dot[k];
+      atomicAdd(d_scale, tot / sc);
+    }
+  }
+}
+
 inline int grid_for(long long n, int block, int cap) {
   long long g = (n + block - 1) / block;
   return static_cast<int>(g < cap ? (g < 1 ? 1 : g) : cap);
@@ -495,6 +544,18 @@ extern "C" int dsb_route_bwd_prologue(const float* dy, const float* y, const flo
   if (D & 3) return 2;
   route_bwd_prologue_kernel<<<(T + 7) / 8, 256, 0, stream>>>(
       dy, y, row_scale, reinterpret_cast<__nv_bfloat16*>(dy_bf16), rowdot, T, D);
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+
+extern "C" int dsb_route_bwd_rows(const float* dy, const float* y, const float* den,
+                                  const float* scale_ptr, float scale, const float* ext_dden,
+                                  void* dy_bf16, float* d_den, float* dtau, float* d_scale, int T, int D,
+                                  cudaStream_t stream) {
+  if (T <= 0) return 0;
+  if (D & 3) return 2;
+  route_bwd_rows_kernel<<<(T + 7) / 8, 256, 0, stream>>>(
+      dy, y, den, scale_ptr, scale, ext_dden, reinterpret_cast<__nv_bfloat16*>(dy_bf16), d_den, dtau,
+      d_scale, T, D);
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

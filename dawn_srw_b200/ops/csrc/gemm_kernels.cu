@@ -102,6 +102,11 @@ struct PlainEpi {
     // scatter_rows + local row] = aux_src[row], written by the tiles of the first column block.
     const float* aux_src;
     float* aux_dst[kMaxOut];
+    // Sum-normalised rows: with `den` the result row is multiplied by norm / max(den[row], 1),
+    // norm = *norm_ptr where given.
+    const float* den;
+    const float* norm_ptr;
+    float norm;
   };
   template <int BN, class Ctl>
   __device__ static void run(const Params& p, const CUtensorMap* maps, WarpStager& st, Ctl& ctl,
@@ -110,7 +115,11 @@ struct PlainEpi {
     if (r0 >= M) { ctl.skip(); return; }  // whole 32-row slab is outside the matrix (warp-uniform)
     const uint32_t acc0 = ctl.wait(0);
     const int row = r0 + lane;
-    const float scale = p.alpha * ((row < M && p.row_scale) ? p.row_scale[row] : 1.f);
+    float scale = p.alpha * ((row < M && p.row_scale) ? p.row_scale[row] : 1.f);
+    if (p.den != nullptr && row < M) {
+      const float d = p.den[row];
+      scale *= (p.norm_ptr != nullptr ? *p.norm_ptr : p.norm) / (d < 1.f ? 1.f : d);   // a NaN stays one
+    }
     if (p.scatter_rows > 0 && p.aux_src != nullptr && n0 == 0 && row < M) {
       const int owner = r0 / p.scatter_rows;
       p.aux_dst[owner][p.scatter_rank * p.scatter_rows + (row - owner * p.scatter_rows)] =
@@ -1429,10 +1438,10 @@ static int bwd_gate_wide(const void* h, long long ldh, const void* emb, long lon
 
 using namespace dsb;
 
-extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn,
-                             long long ldb, int M, int N, int K, void* C, long long ldc,
-                             int c_is_bf16, int accumulate, float alpha, const float* row_scale,
-                             const float* bias, int block_n, int* status, cudaStream_t stream) {
+static int gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn, long long ldb,
+                     int M, int N, int K, void* C, long long ldc, int c_is_bf16, int accumulate,
+                     float alpha, const float* row_scale, const float* bias, const float* den,
+                     const float* norm_ptr, float norm, int block_n, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   GemmParams<PlainEpi::Params> gp;
   memset(&gp, 0, sizeof(gp));
@@ -1450,7 +1459,7 @@ extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void*
   gp.status = status;
   rc = make_out_tmap(&gp.tma_out[0], C, M, N, ldc, c_is_bf16 ? 2 : 4);
   if (rc) return 300 + rc;
-  gp.epi = {alpha, row_scale, bias, c_is_bf16, accumulate, 0, 0, nullptr, {}};
+  gp.epi = {alpha, row_scale, bias, c_is_bf16, accumulate, 0, 0, nullptr, {}, den, norm_ptr, norm};
   if (accumulate && !c_is_bf16 && bias == nullptr) {
     // few output tiles but a long K (pool gradients of a small unit shard): cut K so
     // that every SM pair has work; the splits meet in the fp32 reduce-add epilogue
@@ -1485,6 +1494,21 @@ extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void*
                      : launch_engine_impl<256, PlainEpi, 1>(gp, stream);
   return BN == 128 ? launch_engine_impl<128, PlainEpi, 2>(gp, stream)
                    : launch_engine_impl<256, PlainEpi, 2>(gp, stream);
+}
+
+extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn,
+                             long long ldb, int M, int N, int K, void* C, long long ldc,
+                             int c_is_bf16, int accumulate, float alpha, const float* row_scale,
+                             const float* bias, int block_n, int* status, cudaStream_t stream) {
+  return gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, C, ldc, c_is_bf16, accumulate, alpha, row_scale,
+                   bias, nullptr, nullptr, 1.f, block_n, status, stream);
+}
+
+extern "C" int dsb_srw_write(const void* p, long long ldp, const void* write, long long ldw, int T, int U,
+                             int D, const float* den, float norm, const float* norm_ptr, float* y,
+                             long long ldy, int accumulate, int* status, cudaStream_t stream) {
+  return gemm_bf16(p, 0, ldp, write, 1, ldw, T, D, U, y, ldy, 0, accumulate, 1.f, nullptr, nullptr, den,
+                   norm_ptr, norm, D <= 128 ? 128 : 256, status, stream);
 }
 
 static GateConsts make_gc(const DsbGate* g) {

@@ -30,9 +30,13 @@ constexpr int kMaxR = 512;            // d_route of every supported model is <= 
 
 // One warp per row, grid-stride; a block adds its column sums of h into hsum
 // once at the end (shared-memory partials first).
-__global__ void score_stats_fwd_kernel(const float* __restrict__ hg, const __nv_bfloat16* __restrict__ h,
+// hg = g1 + g2 (row stride ldg): the products with the two bf16 terms of G, side by side in one
+// GEMM's output; g2 may be null.  Row n is token n % T of route n / T, off has strides (o_st, o_sr).
+__global__ void score_stats_fwd_kernel(const float* __restrict__ g1, const float* __restrict__ g2,
+                                       long long ldg, const __nv_bfloat16* __restrict__ h,
                                        long long ldh, const float* __restrict__ esum,
-                                       const float* __restrict__ off, float inv_u, int N, int r,
+                                       const float* __restrict__ off, long long o_st, long long o_sr,
+                                       int T, float inv_u, int N, int r,
                                        float* __restrict__ tau, float* __restrict__ isd,
                                        float* __restrict__ mu_out, float* __restrict__ sd_out,
                                        float* __restrict__ hsum) {
@@ -45,7 +49,8 @@ __global__ void score_stats_fwd_kernel(const float* __restrict__ hg, const __nv_
 #pragma unroll
   for (int k = 0; k < kMaxR / 32; ++k) csum[k] = 0.f;
   for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < N; row += gridDim.x * warps) {
-    const float* g = hg + static_cast<size_t>(row) * r;
+    const float* g = g1 + static_cast<size_t>(row) * ldg;
+    const float* gl = g2 != nullptr ? g2 + static_cast<size_t>(row) * ldg : nullptr;
     const __nv_bfloat16* hr = h + static_cast<size_t>(row) * ldh;
     float m2 = 0.f, m1 = 0.f;
 #pragma unroll
@@ -53,7 +58,7 @@ __global__ void score_stats_fwd_kernel(const float* __restrict__ hg, const __nv_
       const int j = lane + 32 * k;
       if (j < r) {
         const float hv = __bfloat162float(hr[j]);
-        m2 = fmaf(g[j], hv, m2);
+        m2 = fmaf(gl != nullptr ? g[j] + gl[j] : g[j], hv, m2);
         m1 = fmaf(esum[j], hv, m1);
         csum[k] += hv;
       }
@@ -62,7 +67,7 @@ __global__ void score_stats_fwd_kernel(const float* __restrict__ hg, const __nv_
     const float mu = warp_sum(m1) * inv_u;
     if (lane == 0) {
       const float sd = sqrtf(fmaxf(m2 - mu * mu, kVarFloor)) + kSdEps;
-      tau[row] = fmaf(off[row], sd, mu);
+      tau[row] = fmaf(off[(row % T) * o_st + (row / T) * o_sr], sd, mu);
       isd[row] = 1.f / sd;
       mu_out[row] = mu;
       sd_out[row] = sd;
@@ -130,6 +135,113 @@ __global__ void score_stats_bwd_kernel(const float* __restrict__ d_tau, const fl
         dr[j] = acc;
         wr[j] = __float2bfloat16(d_var * hv);
         csum[k] = fmaf(b, hv, csum[k]);
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kMaxR / 32; ++k) {
+    const int j = lane + 32 * k;
+    if (j < r) atomicAdd(&s_sum[j], csum[k]);
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < r; j += blockDim.x) atomicAdd(d_esum + j, s_sum[j]);
+}
+
+// The routes of one pool call, packed for the tensor engine: h fp32 [T, R, r] (strides h_st, h_sr)
+// -> bf16 [R * T, r], route-major, so that a route's rows are one operand.  The buffers that
+// the kernels after it add into (denominators, column sums) are cleared on the way.
+template <bool kVec>
+__global__ void __launch_bounds__(256) score_pack_kernel(const float* __restrict__ h, long long h_st,
+                                                         long long h_sr, int T, int R, int r,
+                                                         __nv_bfloat16* __restrict__ hb,
+                                                         float* __restrict__ z1, int n1,
+                                                         float* __restrict__ z2, int n2) {
+  const long long stride = static_cast<long long>(gridDim.x) * 256;
+  const long long first = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  for (long long i = first; i < n1; i += stride) z1[i] = 0.f;
+  for (long long i = first; i < n2; i += stride) z2[i] = 0.f;
+  const int per = r >> 3;                              // r % 8 == 0
+  const long long total = static_cast<long long>(T) * R * per;
+  for (long long i = first; i < total; i += stride) {
+    const int n = static_cast<int>(i / per), c = static_cast<int>(i - static_cast<long long>(n) * per);
+    const float* src = h + (n % T) * h_st + (n / T) * h_sr + 8 * c;
+    float v[8];
+    if constexpr (kVec) {
+      const float4 a = reinterpret_cast<const float4*>(src)[0], b = reinterpret_cast<const float4*>(src)[1];
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+      v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = src[j];
+    }
+    uint4 q;
+    uint32_t* w = reinterpret_cast<uint32_t*>(&q);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const __nv_bfloat162 p2 = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+      w[j] = *reinterpret_cast<const uint32_t*>(&p2);
+    }
+    *reinterpret_cast<uint4*>(hb + static_cast<size_t>(n) * r + 8 * c) = q;
+  }
+}
+
+// Everything of a call's backward pass that is a matter of token rows, one warp per row n
+// (route-major): the sigma path of the gate, the statistics, and the sum of what reaches h.
+//   dsz = (1/sigma) (<h, dh32> + tau dtau),  d_isd = dsz sigma^2      (gates that use sigma)
+//   then the row part above with d_tau = dtau; dh = ... + d_hsum + dh32.
+// dh32 (fp32 [N, r]) is ds . emb straight from its GEMM.  dh is [T, R, r], d_off [T, R].
+__global__ void __launch_bounds__(256) score_route_bwd_kernel(
+    const float* __restrict__ dtau, const float* __restrict__ dh32, const float* __restrict__ d_hsum,
+    const float* __restrict__ off, long long o_st, long long o_sr, const float* __restrict__ tau,
+    const float* __restrict__ isd, const float* __restrict__ mu_in, const float* __restrict__ sd_in,
+    const float* __restrict__ g1, const float* __restrict__ g2, long long ldg,
+    const __nv_bfloat16* __restrict__ h, const float* __restrict__ esum, float inv_u, int sigma_path,
+    int T, int R, int r, float* __restrict__ dh, __nv_bfloat16* __restrict__ w,
+    float* __restrict__ d_off, float* __restrict__ d_esum) {
+  __shared__ float s_sum[kMaxR];
+  for (int j = threadIdx.x; j < r; j += blockDim.x) s_sum[j] = 0.f;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5, N = T * R;
+  float csum[kMaxR / 32];
+#pragma unroll
+  for (int k = 0; k < kMaxR / 32; ++k) csum[k] = 0.f;
+  for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < N; row += gridDim.x * warps) {
+    const int t = row % T, ri = row / T;
+    const float sd = sd_in[row], mu = mu_in[row], dt = dtau[row];
+    const __nv_bfloat16* hr = h + static_cast<size_t>(row) * r;
+    const float* dr32 = dh32 + static_cast<size_t>(row) * r;
+    float hv[kMaxR / 32], dv[kMaxR / 32];
+    float dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < kMaxR / 32; ++k) {
+      const int j = lane + 32 * k;
+      hv[k] = j < r ? __bfloat162float(hr[j]) : 0.f;
+      dv[k] = j < r ? dr32[j] : 0.f;
+      dot = fmaf(hv[k], dv[k], dot);
+    }
+    float di = 0.f;
+    if (sigma_path) {
+      const float is = isd[row];
+      di = is * (warp_sum(dot) + tau[row] * dt) / (is * is);
+    }
+    const float d_sd = dt * off[t * o_st + ri * o_sr] - di / (sd * sd);
+    const float sq = sd - kSdEps;
+    const float d_var = sq > 1.5e-6f ? d_sd / (2.f * sq) : 0.f;   // sqrt(floor) = 1e-6
+    const float d_mu = dt - 2.f * mu * d_var;
+    if (lane == 0) d_off[static_cast<size_t>(t) * R + ri] = dt * sd;
+    const float a = 2.f * d_var * inv_u, b = d_mu * inv_u;
+    const float* gr1 = g1 + static_cast<size_t>(row) * ldg;
+    const float* gr2 = g2 + static_cast<size_t>(row) * ldg;
+    float* dr = dh + (static_cast<size_t>(t) * R + ri) * r;
+    __nv_bfloat16* wr = w + static_cast<size_t>(row) * r;
+#pragma unroll
+    for (int k = 0; k < kMaxR / 32; ++k) {
+      const int j = lane + 32 * k;
+      if (j < r) {
+        const float acc = fmaf(a, gr1[j] + gr2[j], fmaf(b, esum[j], d_hsum != nullptr ? d_hsum[j] : 0.f));
+        dr[j] = acc + dv[k];
+        wr[j] = __float2bfloat16(d_var * hv[k]);
+        csum[k] = fmaf(b, hv[k], csum[k]);
       }
     }
   }
@@ -423,15 +535,47 @@ int stats_grid(int N) {
 
 }  // namespace
 
-extern "C" int dsb_score_stats_fwd(const float* hg, const void* h_bf16, long long ldh,
-                                   const float* esum, const float* off, float inv_u, int N, int r,
+extern "C" int dsb_score_stats_fwd(const float* hg, const float* hg2, long long ldg, const void* h_bf16,
+                                   long long ldh, const float* esum, const float* off, long long o_st,
+                                   long long o_sr, int T, float inv_u, int N, int r,
                                    float* tau, float* isd, float* mu, float* sd, float* hsum,
                                    cudaStream_t stream) {
   if (N <= 0) return 0;
   if (r <= 0 || r > kMaxR) return 801;
   score_stats_fwd_kernel<<<stats_grid(N), 256, 0, stream>>>(
-      hg, static_cast<const __nv_bfloat16*>(h_bf16), ldh, esum, off, inv_u, N, r, tau, isd, mu, sd,
-      hsum);
+      hg, hg2, ldg, static_cast<const __nv_bfloat16*>(h_bf16), ldh, esum, off, o_st, o_sr, T, inv_u, N, r,
+      tau, isd, mu, sd, hsum);
+  return cudaGetLastError() == cudaSuccess ? 0 : 802;
+}
+
+extern "C" int dsb_score_pack(const float* h, long long h_st, long long h_sr, int T, int R, int r,
+                              void* hb_bf16, float* z1, int n1, float* z2, int n2,
+                              cudaStream_t stream) {
+  if (T <= 0 || R <= 0) return 0;
+  if (r <= 0 || r % 8 != 0 || r > kMaxR) return 801;
+  const long long n = static_cast<long long>(T) * R * (r >> 3);
+  const int blocks = static_cast<int>(n / 256 + 1 < 148 * 8 ? n / 256 + 1 : 148 * 8);
+  __nv_bfloat16* hb = static_cast<__nv_bfloat16*>(hb_bf16);
+  if (((reinterpret_cast<uintptr_t>(h) & 15) | (h_st & 3) | (h_sr & 3)) == 0)
+    score_pack_kernel<true><<<blocks, 256, 0, stream>>>(h, h_st, h_sr, T, R, r, hb, z1, n1, z2, n2);
+  else
+    score_pack_kernel<false><<<blocks, 256, 0, stream>>>(h, h_st, h_sr, T, R, r, hb, z1, n1, z2, n2);
+  return cudaGetLastError() == cudaSuccess ? 0 : 802;
+}
+
+extern "C" int dsb_score_route_bwd(const float* dtau, const float* dh32, const float* d_hsum,
+                                   const float* off, long long o_st, long long o_sr, const float* tau,
+                                   const float* isd, const float* mu, const float* sd, const float* hg,
+                                   const float* hg2, long long ldg, const void* h_bf16,
+                                   const float* esum, float inv_u, int sigma_path, int T, int R, int r,
+                                   float* dh, void* w_bf16, float* d_off, float* d_esum,
+                                   cudaStream_t stream) {
+  if (T <= 0 || R <= 0) return 0;
+  if (r <= 0 || r > kMaxR) return 801;
+  score_route_bwd_kernel<<<stats_grid(T * R), 256, 0, stream>>>(
+      dtau, dh32, d_hsum, off, o_st, o_sr, tau, isd, mu, sd, hg, hg2, ldg,
+      static_cast<const __nv_bfloat16*>(h_bf16), esum, inv_u, sigma_path, T, R, r, dh,
+      static_cast<__nv_bfloat16*>(w_bf16), d_off, d_esum);
   return cudaGetLastError() == cudaSuccess ? 0 : 802;
 }
 

@@ -277,12 +277,14 @@ class _LayerNormFn(torch.autograd.Function):
 # ---------------------------------------------------------------------------
 class _PoolTensors:
     """bf16 compute copies of a pool and the fp32 gradient accumulators of the current step."""
-    __slots__ = ("emb", "read", "write", "g_emb", "g_read", "g_write", "emb_f", "rank1", "__weakref__")
+    __slots__ = ("emb", "read", "write", "g_emb", "g_read", "g_write", "emb_f", "rank1",
+                 "g_gram", "g_esum", "__weakref__")
 
     def __init__(self):
         self.emb = self.read = self.write = None
         self.g_emb = self.g_read = self.g_write = None
         self.emb_f = None          # fp32 copy of emb for the per-unit mat-vecs (made on first use)
+        self.g_gram = self.g_esum = None
         self.rank1 = []            # (d m_u, hsum) of the load-balance terms: g_emb += sum d m_u (x) hsum
 
 
@@ -336,12 +338,16 @@ class _PoolPrepFn(torch.autograd.Function):
             gram = ef.t() @ ef
         esum = emb_c[:U].sum(0, dtype=torch.float32)
         holder.emb, holder.read, holder.write = emb_c, read_c, write_c
+        holder.rank1, holder.g_gram, holder.g_esum = [], None, None
         if any(ctx.needs_input_grad[:3]):
             holder.g_emb = torch.zeros_like(emb, dtype=torch.float32)
             holder.g_read = torch.zeros_like(read, dtype=torch.float32)
             holder.g_write = torch.zeros_like(write, dtype=torch.float32)
+            stat = torch.zeros(r * r + r, dtype=torch.float32, device=emb.device)
+            holder.g_gram, holder.g_esum = stat[:r * r].view(r, r), stat[r * r:]
         ctx.save_for_backward(emb, read, write, n_e, n_r, n_w)
         ctx.U = U
+        ctx.set_materialize_grads(False)
         anchor = torch.zeros(1, device=emb.device)
         return anchor, gram, esum
 
@@ -351,6 +357,10 @@ class _PoolPrepFn(torch.autograd.Function):
         hd = ctx.holder
         U = ctx.U
         g_emb, g_read, g_write = hd.g_emb, hd.g_read, hd.g_write
+        # what reached the statistics through autograd, and what unsharded calls accumulated
+        if hd.g_gram is not None:
+            d_gram = hd.g_gram if d_gram is None else d_gram + hd.g_gram
+            d_esum = hd.g_esum if d_esum is None else d_esum + hd.g_esum
         if d_gram is not None:
             # d emb = E (dG + dG^T): engine GEMMs on a two-term bf16 split of the symmetric
             # factor, accumulated into the shared gradient buffer
@@ -375,7 +385,7 @@ class _PoolPrepFn(torch.autograd.Function):
             n = w / nrm
             return (g - n * (n * g).sum(-1, keepdim=True)) / nrm
         out = (chain(g_emb, emb, n_e), chain(g_read, read, n_r), chain(g_write, write, n_w))
-        hd.g_emb = hd.g_read = hd.g_write = None
+        hd.g_emb = hd.g_read = hd.g_write = hd.g_gram = hd.g_esum = None
         return out + (None, None, None)
 
 
@@ -439,11 +449,27 @@ def _route_backward_core(x_bf, h_bf, tau, inv_sd, dy, d_den, hd, spec, U, xr=Non
     are recomputed.  Either way it emits p, dxr, ds and dtau.  Pool gradients
     are accumulated into the holder's fp32 buffers.
     Returns (dx bf16, dh bf16, dtau, d_inv_sigma or None)."""
+    dev = x_bf.device
+    T = x_bf.shape[0]
+    dtau = torch.zeros(T, dtype=torch.float32, device=dev)
+    dh32 = torch.empty(T, hd.emb.shape[1], dtype=torch.float32, device=dev)
+    dx = _route_backward_gemms(x_bf, h_bf, tau, inv_sd, dy, d_den, dtau, hd, spec, U, xr, dh32)
+    d_isd = None
+    if spec.kind == GATE_GELU_Z:
+        # sum_u ds_u z_u = (1/sigma) (<h, ds.emb> + tau * dtau): the sigma path needs no
+        # reduction of its own in the kernel
+        dsz = inv_sd * ((h_bf.float() * dh32).sum(-1) + tau * dtau)
+        d_isd = dsz / (inv_sd * inv_sd)
+    return dx, dh32.to(torch.bfloat16), dtau, d_isd
+
+
+def _route_backward_gemms(x_bf, h_bf, tau, inv_sd, dy, d_den, dtau, hd, spec, U, xr, dh32, want_dx=True):
+    """Gate step and GEMMs of one route's backward: adds into the zeroed ``dtau`` [T] and the
+    pool's gradient buffers, fills ``dh32`` [T, r] = ds . emb; returns dx (bf16)."""
     e = ext()
     dev = x_bf.device
     T = x_bf.shape[0]
     Up = _round_up(U, 8)
-    dtau = torch.zeros(T, dtype=torch.float32, device=dev)
     emb, read, write = hd.emb[:U], hd.read[:U], hd.write[:U]
     if xr is not None:
         p = xr
@@ -456,23 +482,16 @@ def _route_backward_core(x_bf, h_bf, tau, inv_sd, dy, d_den, hd, spec, U, xr=Non
         p = torch.empty(T, Up, dtype=torch.bfloat16, device=dev)
         dxr = torch.empty_like(p)
         ds = torch.empty_like(p)
-        dsz = torch.zeros(T, dtype=torch.float32, device=dev)
         count_launches(2)
-        e.srw_bwd_gate(h_bf, emb, x_bf, read, dy, write, p, dxr, ds, tau, inv_sd, d_den, dtau, dsz,
-                       _gate_list(spec), status_word(dev))
+        # the sigma sum is derived from dh32 and dtau: the kernel's own output for it is unused
+        e.srw_bwd_gate(h_bf, emb, x_bf, read, dy, write, p, dxr, ds, tau, inv_sd, d_den, dtau,
+                       torch.empty_like(dtau), _gate_list(spec), status_word(dev))
     pv, dxrv, dsv = p[:, :U], dxr[:, :U], ds[:, :U]
     gemm(pv, True, dy, True, out=hd.g_write[:U], accumulate=True)       # p^T dy
     gemm(dxrv, True, x_bf, True, out=hd.g_read[:U], accumulate=True)    # dxr^T x
     gemm(dsv, True, h_bf, True, out=hd.g_emb[:U], accumulate=True)      # ds^T h
-    dx = gemm(dxrv, False, read, True, out_dtype=torch.bfloat16)        # dxr . read
-    dh32 = gemm(dsv, False, emb, True, out_dtype=torch.float32)         # ds . emb
-    d_isd = None
-    if spec.kind == GATE_GELU_Z:
-        # sum_u ds_u z_u = (1/sigma) (<h, ds.emb> + tau * dtau): the sigma path needs no
-        # reduction of its own in the kernel
-        dsz = inv_sd * ((h_bf.float() * dh32).sum(-1) + tau * dtau)
-        d_isd = dsz / (inv_sd * inv_sd)
-    return dx, dh32.to(torch.bfloat16), dtau, d_isd
+    gemm(dsv, False, emb, True, out=dh32)                               # ds . emb
+    return gemm(dxrv, False, read, True, out_dtype=torch.bfloat16) if want_dx else None   # dxr . read
 
 
 class _SRWRouteFn(torch.autograd.Function):
@@ -503,54 +522,84 @@ class _SRWRouteFn(torch.autograd.Function):
         return (dx, dh, dtau, d_isd, torch.zeros(1, device=dev), None, None, None, None, None)
 
 
-class _SRWRouteScaledFn(torch.autograd.Function):
-    """One SRW route with the sum-normalisation and the pool scale folded into
-    the write GEMM's epilogue: ``y = scale * (p . write) / max(den, 1)`` leaves
-    the engine as the final fp32 output (no [T, D] pass for the divide or the
-    scale).  Backward starts with one row kernel that produces the bf16
-    ``dy * scale / max(den, 1)`` operand and ``<dy, y>`` per row, from which the
-    denominator and scale gradients follow:
+class _SRWCallFn(torch.autograd.Function):
+    """One call of an unsharded pool, all its routes: score statistics, gate kernels and write
+    GEMMs, ``y_r = scale * (p_r . write) / max(den_r, 1)`` leaving the engine as the final fp32
+    output.  One node per call, the routes stacked route-major ([R * T] rows), so that every
+    per-row step of the forward and of the backward pass is one launch for all of them; the
+    gradients of the Gram matrix and of the pool tensors go straight into the buffers that the
+    pool's preparation node chains on.  (A node per route between statistics, selects and clamps
+    was some 160 launches a layer more: a training step of 4 x 128 tokens on the 40M model took
+    57.8 ms for 41.6, a forward of 16 x 512 tokens 18.2 for 13.6.)  Backward per route starts with one row kernel that makes
+    the bf16 ``dy * scale / max(den, 1)`` operand and, from <dy, y>,
         d_den = -<dy, y> / den  (den > 1),   d_scale = sum_t <dy, y> / scale.
-    Only for unsharded pools (the denominator is complete on this rank)."""
+    Returns y_0 .. y_{R-1} [T, D], hsum [r], den [R, T], tau and 1/sigma [R, T] (not
+    differentiable)."""
 
     @staticmethod
-    def forward(ctx, x_bf, h_bf, tau, inv_sd, anchor, holder, spec, U, alive, unit_mask, scale,
-                diag=None):
-        e = ext()
-        dev = x_bf.device
-        T, D = x_bf.shape
-        Up = _round_up(U, 8)
-        p = torch.empty(T, Up, dtype=torch.bfloat16, device=dev)           # scratch
-        den = torch.zeros(T, dtype=torch.float32, device=dev)
-        xr = _alloc_saved_xr(dev, T, Up, U, getattr(holder, "keep_xr", True) and unit_mask is None
-                             and any(ctx.needs_input_grad))
-        count_launches(2)
-        e.srw_fwd_gate_xr(h_bf, holder.emb[:U], x_bf, holder.read[:U], p, xr, tau, inv_sd, None, den,
-                          diag, alive, unit_mask, _gate_list(spec), status_word(dev), *NO_GATHER)
-        rs = (scale.detach().float() / den.clamp(min=1.0)).contiguous()
-        y = gemm(p[:, :U], False, holder.write[:U], True, out_dtype=torch.float32, row_scale=rs)
-        ctx.save_for_backward(x_bf, h_bf, tau, inv_sd, y, den, rs, scale)
-        ctx.holder, ctx.spec, ctx.U = holder, spec, U
-        ctx.xr = xr
-        return y, den
+    def forward(ctx, x_bf, h, off, scale, anchor, hd, ex, spec, U, inv_u, alive, unit_mask, diag, keep):
+        e, dev, st = ext(), x_bf.device, status_word(x_bf.device)
+        T, R, r = h.shape
+        D, Up = x_bf.shape[1], _round_up(U, 8)
+        hb, hg, tau, isd, mu, sd, den, hsum = e.srw_stats(h.detach(), off.detach(), ex["gram_cat"],
+                                                          ex["esum"].detach(), inv_u, st)
+        p = torch.empty(T, Up, dtype=torch.bfloat16, device=dev)           # scratch of every route
+        emb, read, write = hd.emb[:U], hd.read[:U], hd.write[:U]
+        sc_t = scale.detach() if isinstance(scale, torch.Tensor) else None
+        sc_f = 1.0 if sc_t is not None else float(scale)
+        gl = _gate_list(spec)
+        ys, xrs = [], []
+        for i in range(R):
+            rows = slice(i * T, (i + 1) * T)
+            xr = _alloc_saved_xr(dev, T, Up, U, keep)
+            y = torch.empty(T, D, dtype=torch.float32, device=dev)
+            e.srw_route_fwd(hb[rows], x_bf, emb, read, write, p, xr, tau[rows], isd[rows], den[i],
+                            None if diag is None else diag[i], alive, unit_mask, gl, sc_f, sc_t, y, False, st)
+            ys.append(y)
+            xrs.append(xr)
+        count_launches(3 + 2 * R)
+        ctx.save_for_backward(x_bf, off, hb, hg, tau, isd, mu, sd, den, sc_t, *ys)
+        ctx.hd, ctx.esum, ctx.spec, ctx.args = hd, ex["esum"].detach(), spec, (T, R, r, U, inv_u, sc_f)
+        ctx.xrs, ctx.h_shape = xrs, h.shape
+        ctx.set_materialize_grads(False)
+        tau_o, isd_o = tau.view(R, T), isd.view(R, T)
+        ctx.mark_non_differentiable(tau_o, isd_o)
+        return (*ys, hsum, den, tau_o, isd_o)
 
     @staticmethod
-    def backward(ctx, d_y, d_den_ext):
-        x_bf, h_bf, tau, inv_sd, y, den, rs, scale = ctx.saved_tensors
-        hd, spec, U = ctx.holder, ctx.spec, ctx.U
-        dev = x_bf.device
-        dy, rowdot = ext().route_bwd_prologue(d_y.contiguous().float(), y, rs)
-        count_launches(1)
-        d_den = torch.where(den > 1.0, -rowdot / den.clamp(min=1.0), torch.zeros_like(rowdot))
+    def backward(ctx, *grads):
+        x_bf, off, hb, hg, tau, isd, mu, sd, den, sc_t, *ys = ctx.saved_tensors
+        T, R, r, U, inv_u, sc_f = ctx.args
+        hd, spec = ctx.hd, ctx.spec
+        e, dev, st = ext(), x_bf.device, status_word(x_bf.device)
+        d_hsum, d_den_ext = grads[R], grads[R + 1]
+        if d_hsum is not None:
+            d_hsum = d_hsum.contiguous()
         if d_den_ext is not None:
-            d_den = d_den + d_den_ext.float()
-        d_scale = (rowdot.sum() / scale.detach().float()).reshape(scale.shape).to(scale.dtype) \
-            if ctx.needs_input_grad[10] else None
-        xr, ctx.xr = ctx.xr, None
-        dx, dh, dtau, d_isd = _route_backward_core(x_bf, h_bf, tau, inv_sd, dy, d_den.contiguous(), hd,
-                                                   spec, U, xr)
-        return (dx, dh, dtau, d_isd, torch.zeros(1, device=dev), None, None, None, None, None,
-                d_scale, None)
+            d_den_ext = d_den_ext.float().contiguous()
+        dtau = torch.empty(R * T, dtype=torch.float32, device=dev)
+        dh32 = torch.empty(R * T, r, dtype=torch.float32, device=dev)
+        d_scale = torch.zeros_like(sc_t) if sc_t is not None and ctx.needs_input_grad[3] else None
+        xrs, ctx.xrs = ctx.xrs, [None] * R
+        dx = None
+        for i in range(R):
+            rows = slice(i * T, (i + 1) * T)
+            dy = grads[i]
+            dy = torch.zeros_like(ys[i]) if dy is None else dy.float().contiguous()
+            if dy.data_ptr() % 16:
+                dy = dy.clone()
+            dyb, d_den = e.route_bwd_rows(dy, ys[i], den[i], sc_f, sc_t,
+                                          None if d_den_ext is None else d_den_ext[i], dtau[rows], d_scale)
+            dxi = _route_backward_gemms(x_bf, hb[rows], tau[rows], isd[rows], dyb, d_den, dtau[rows],
+                                        hd, spec, U, xrs[i], dh32[rows], ctx.needs_input_grad[0])
+            xrs[i] = None
+            if dxi is not None:
+                dx = dxi if dx is None else dx.add_(dxi)
+        g_esum = hd.g_esum if hd.g_esum is not None else torch.zeros_like(ctx.esum)
+        dh, d_off = e.srw_stats_bwd(dtau, dh32, d_hsum, off.detach(), tau, isd, mu, sd, hg, hb, ctx.esum,
+                                    inv_u, spec.kind == GATE_GELU_Z, hd.g_gram, g_esum, st)
+        count_launches(R + 2)
+        return (dx, dh, d_off, d_scale, None, None, None, None, None, None, None, None, None, None)
 
 
 # ---------------------------------------------------------------------------
@@ -906,8 +955,10 @@ class CudaBackend:
         gram = C.sum_over_shards(gram, pctx.shard_group)
         esum = C.sum_over_shards(esum, pctx.shard_group)
         from .score_stats import split_bf16
+        cat = torch.cat(split_bf16(gram.detach()))           # the two bf16 terms, one operand
+        r = gram.shape[0]
         pool.extra = {"anchor": anchor, "gram": gram, "esum": esum, "U": U,
-                      "gram_split": split_bf16(gram.detach())}
+                      "gram_split": (cat[:r], cat[r:]), "gram_cat": cat}
         return pool
 
     def srw(self, x, h, tau_off, pool: CudaPool, spec: GateSpec, *,
@@ -949,7 +1000,6 @@ class CudaBackend:
         else:
             scale = out_scale.detach().float() if isinstance(out_scale, torch.Tensor) else float(out_scale)
         gl = _gate_list(spec)
-        wide = bool(e.srw_wide_tiles(U))
         # Routes of one pool are independent token rows as far as the kernels care: with few
         # tokens (decoding) they are stacked into one call, so the pool is streamed once.
         stack = Rr * T <= 128
@@ -964,30 +1014,30 @@ class CudaBackend:
             return list(out.reshape(Rr, T, D).unbind(0))
         if stack:
             tau, inv_sd, h_rm = score_stats_rows(h, tau_off, ex["gram"], ex["esum"], U_tot)
-            calls = [(h_rm, x_bf.repeat(Rr, 1) if Rr > 1 else x_bf, tau, inv_sd)]
+            x_rm = x_bf.repeat(Rr, 1) if Rr > 1 else x_bf
+            calls = [(h_rm, x_rm, tau, inv_sd)]
         else:
-            tau, inv_sd, _, h_bf3 = score_stats(h, tau_off, ex["gram"], ex["esum"], U_tot,
-                                                ex["gram_split"])
-            calls = [(_bf16_2d(h_bf3[:, ri]), x_bf, tau[:, ri].contiguous(), inv_sd[:, ri].contiguous())
-                     for ri in range(Rr)]
-        outs = []
-        for h_r, x_r, tau_r, isd_r in calls:
-            Tr = h_r.shape[0]
-            p = torch.empty(Tr, Up, dtype=torch.bfloat16, device=dev)
-            work = torch.zeros(Tr * (D + 1), dtype=torch.float32, device=dev)   # y and den, one fill
-            y, den = work[:Tr * D].view(Tr, D), work[Tr * D:]
-            if wide:
-                e.srw_fwd_gate_xr(h_r, pool.emb[:U], x_r, pool.read[:U], p, None, tau_r, isd_r, None,
-                                  den, None, None, None, gl, st, *NO_GATHER)
-            else:
-                e.srw_fwd_gate(h_r, pool.emb[:U], x_r, pool.read[:U], p, tau_r, isd_r, den, None, None,
-                               None, gl, st)
-            gemm(p[:, :U], False, pool.write[:U], True, out=y, accumulate=True)
-            outs.append(y * (scale / den.clamp(min=1.0)).unsqueeze(-1))
-        count_launches(len(calls))
+            hf = h if h.dtype == torch.float32 and h.stride(2) == 1 else h.float().contiguous()
+            hb, _, tau, inv_sd, *_ = e.srw_stats(hf, tau_off.float(), ex["gram_cat"], ex["esum"].detach(),
+                                                 1.0 / float(U_tot), st)
+            count_launches(3)
+            calls = [(hb[i * T:(i + 1) * T], x_bf, tau[i * T:(i + 1) * T], inv_sd[i * T:(i + 1) * T])
+                     for i in range(Rr)]
+        # y and den of all calls, cleared by one fill (the splits of the write GEMM add up in y)
+        Tr = calls[0][0].shape[0]
+        work = torch.zeros(len(calls) * Tr * (D + 1), dtype=torch.float32, device=dev)
+        ys = work[:len(calls) * Tr * D].view(len(calls), Tr, D)
+        dens = work[len(calls) * Tr * D:].view(len(calls), Tr)
+        p = torch.empty(Tr, Up, dtype=torch.bfloat16, device=dev)
+        sc_t = scale.reshape(1) if isinstance(scale, torch.Tensor) else None
+        sc_f = 1.0 if sc_t is not None else scale
+        for i, (h_r, x_r, tau_r, isd_r) in enumerate(calls):
+            e.srw_route_fwd(h_r, x_r, pool.emb[:U], pool.read[:U], pool.write[:U], p, None, tau_r, isd_r,
+                            dens[i], None, None, None, gl, sc_f, sc_t, ys[i], True, st)
+        count_launches(2 * len(calls))
         if stack:
-            return list(outs[0].reshape(Rr, T, D).unbind(0))
-        return outs
+            return list(ys[0].reshape(Rr, T, D).unbind(0))
+        return list(ys.unbind(0))
 
     def srw_group(self, x, calls, spec: GateSpec, *, want_diag: bool = True):
         """Several SRW calls on the same ``x``.  Sequence- and pool-sharded calls on
@@ -1127,8 +1177,20 @@ class CudaBackend:
         U_tot = pctx.n_total if pctx.n_total is not None else U
         T, Rr, r = h.shape
         x_bf = _bf16_2d(x)
-        tau, inv_sd, hsum, h_bf3 = score_stats(h, tau_off, ex["gram"], ex["esum"], U_tot,
-                                               ex["gram_split"])
+        alive = torch.zeros(U, dtype=torch.uint8, device=x.device) if spec.has_dead_penalty else None
+        um = None if unit_mask is None else unit_mask[:U].float().contiguous()
+        scale = 1.0 if out_scale is None else out_scale
+        if isinstance(scale, torch.Tensor):
+            scale = scale.to(device=x.device, dtype=torch.float32)
+        # routing diagnostics ride in the gate kernel's epilogue (wide kernels); pools too
+        # small for those take the library path below
+        dg = torch.zeros(Rr, T * DIAG_COLS + 2, dtype=torch.float32, device=x.device) \
+            if want_diag and ext().srw_wide_tiles(U) else None
+        hf = h if h.dtype == torch.float32 and h.stride(2) == 1 else h.float().contiguous()
+        keep = getattr(pool, "keep_xr", True) and um is None and torch.is_grad_enabled()
+        res = _SRWCallFn.apply(x_bf, hf, tau_off.float(), scale, anchor, pool.tensors, ex, spec, U,
+                               1.0 / float(U_tot), alive, um, dg, keep)
+        outs, (hsum, den, tau, inv_sd) = list(res[:Rr]), res[Rr:]
         if spec.has_dead_penalty or C.group_size(pctx.dp_group) > 1:
             # the per-unit means are needed by themselves, or have to meet other ranks'
             hbar = hsum / float(T * Rr)
@@ -1140,26 +1202,7 @@ class CudaBackend:
             lb = var_score / (mean_score ** 2 + var_score + 1e-2)
         else:
             lb = _LoadBalanceFn.apply(hsum, anchor, pool.tensors, U, 1.0 / (T * Rr), float(U_tot))
-        alive = torch.zeros(U, dtype=torch.uint8, device=x.device) if spec.has_dead_penalty else None
-        um = None if unit_mask is None else unit_mask[:U].float().contiguous()
-        if out_scale is None:
-            scale = torch.ones((), device=x.device)
-        elif isinstance(out_scale, torch.Tensor):
-            scale = out_scale
-        else:
-            scale = torch.full((), float(out_scale), device=x.device)
-        outs, dens = [], []
-        # routing diagnostics ride in the gate kernel's epilogue (wide kernels); pools too
-        # small for those take the library path below
-        dg = torch.zeros(Rr, T * DIAG_COLS + 2, dtype=torch.float32, device=x.device) \
-            if want_diag and ext().srw_wide_tiles(U) else None
-        for ri in range(Rr):
-            y, den = _SRWRouteScaledFn.apply(x_bf, _bf16_2d(h_bf3[:, ri]), tau[:, ri].contiguous(),
-                                             inv_sd[:, ri].contiguous(), anchor, pool, spec, U,
-                                             alive, um, scale, None if dg is None else dg[ri])
-            outs.append(y)
-            dens.append(den)
-        den = torch.stack(dens, dim=1).clamp(min=1.0)
+        den = den.t().clamp(min=1.0)
         dead_pen = x.new_zeros(())
         if spec.has_dead_penalty:
             al = C.all_reduce_nograd(alive.float(), pctx.dp_group, "max")
@@ -1170,8 +1213,8 @@ class CudaBackend:
         if want_diag:
             with torch.no_grad():
                 if dg is not None:
-                    diag = diag_from_kernel(spec, dg, tau.detach(), inv_sd.detach(), tau_off.detach(),
-                                            U_tot, alive, None)
+                    diag = diag_from_kernel(spec, dg, tau.t(), inv_sd.t(), tau_off.detach(), U_tot, alive,
+                                            None)
                 else:
                     diag = self._srw_library(x.detach(), h.detach(), tau_off.detach(), pool, spec,
                                              ParallelCtx(None, pctx.dp_group, pctx.n_total,

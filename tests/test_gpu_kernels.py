@@ -788,3 +788,62 @@ def test_load_balance_term_and_its_gradients(cb, U, r, layers):
     # every layer's product is added to a value of order one: 2^-24 of rounding per element each
     rounding = 2.0 ** -24 * (layers * U * r) ** 0.5
     assert float((added[:U] - ref_e.grad).norm()) < 1e-4 * float(ref_e.grad.norm()) + rounding + 1e-6
+
+
+@pytest.mark.parametrize("T,R,r,wide", [(1, 1, 8, 24), (5, 2, 16, 35), (129, 2, 64, 131), (300, 1, 384, 387)])
+def test_stacked_call_statistics_and_row_steps(cb, T, R, r, wide):
+    """Routes that are strided (and here unaligned) slices of a router output, stacked for one
+    call: bf16 copy exact, statistics and their gradients against fp64 of the same bf16 values;
+    2e-5 covers the two-term Gram split (2^-17), 3e-3 gradients through bf16(d_var h)."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(T + r)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    U, e, st = 600, cb.ext(), cb.status_word(dev)
+    h = rn(T, R * r + wide)[:, 3:3 + R * r].unflatten(1, (R, r))
+    off = (rn(T, R + 2) * 0.3)[:, 1:1 + R]
+    emb = torch.nn.functional.normalize(rn(U, r), dim=-1).bfloat16().double()
+    gram, esum = emb.t() @ emb, emb.sum(0)
+    hi = gram.float().bfloat16()
+    gcat = torch.cat([hi, (gram.float() - hi.float()).bfloat16()])
+    hb, hg, tau, isd, mu, sd, den, hsum = e.srw_stats(h, off, gcat, esum.float(), 1.0 / U, st)
+    assert torch.equal(hb.view(R, T, r), h.transpose(0, 1).bfloat16())
+    assert float(den.abs().max()) == 0.0
+    h64, o64 = hb.double().requires_grad_(True), off.t().reshape(-1).double().requires_grad_(True)
+    gr64, es64 = gram.clone().requires_grad_(True), esum.clone().requires_grad_(True)
+    m = (h64 @ es64) / U
+    s = (((h64 @ gr64) * h64).sum(-1) / U - m * m).sqrt()
+    t64 = m + o64 * s
+    assert _rel(tau, t64) < 2e-5 and _rel(isd, 1 / s) < 2e-5 and _rel(hsum, h64.sum(0)) < 1e-5
+    dtau, dh32, d_hsum = rn(R * T), rn(R * T, r), rn(r)
+    d_isd = (((hb.double() * dh32.double()).sum(-1) + t64.detach() * dtau) * s.detach())     # dsz / isd^2
+    ((t64 * dtau).sum() + (d_isd / s).sum() + (h64 * (dh32 + d_hsum).double()).sum()).backward()
+    g_gram, g_esum = torch.zeros(r, r, device=dev), torch.zeros(r, device=dev)
+    dh, d_off = e.srw_stats_bwd(dtau, dh32, d_hsum, off, tau, isd, mu, sd, hg, hb, esum.float(), 1.0 / U,
+                                True, g_gram, g_esum, st)
+    cb.check_status()
+    assert _rel(dh.transpose(0, 1).reshape(R * T, r), h64.grad) < 1e-4
+    assert _rel(d_off.t().reshape(-1), o64.grad) < 1e-4 and _rel(g_esum, es64.grad) < 1e-4
+    assert _rel(g_gram + g_gram.t(), gr64.grad + gr64.grad.t()) < 2 * 3e-3
+
+
+@pytest.mark.parametrize("T,D", [(1, 8), (9, 136), (64, 2048)])
+def test_route_backward_row_step(cb, T, D):
+    """Denominators below, at and above one, and NaN (which has to reach the operand, as with
+    clamp); fp32 sums of D terms, so 1e-5, and one bf16 rounding of the operand."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(T)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    dy, y, den = rn(T, D), rn(T, D), rn(T).abs() * 2
+    den[0] = 1.0
+    scale, ext_dden = torch.full((), 1.7, device=dev), rn(T)
+    dtau, d_scale = rn(T), torch.zeros((), device=dev)
+    dyb, d_den = cb.ext().route_bwd_rows(dy, y, den, 1.0, scale, ext_dden, dtau, d_scale)
+    dot = (dy.double() * y.double()).sum(-1)
+    assert torch.equal(dyb, (dy * (scale / den.clamp(min=1.0))[:, None]).bfloat16()) or \
+        _rel(dyb, dy * (scale / den.clamp(min=1.0))[:, None]) < 4e-3
+    want = torch.where(den > 1.0, -dot / den, torch.zeros_like(dot)) + ext_dden
+    assert float((d_den - want).abs().max()) < 1e-5 * D and float(dtau.abs().max()) == 0.0
+    assert abs(float(d_scale) - float(dot.sum() / 1.7)) < 1e-5 * T * D
+    den[0] = float("nan")
+    dyb, _ = cb.ext().route_bwd_rows(dy, y, den, 1.5, None, None, dtau, None)
+    assert bool(dyb[0].isnan().all()) and bool(dyb[1:].isfinite().all())
