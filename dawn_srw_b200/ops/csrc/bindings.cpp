@@ -881,7 +881,7 @@ Tensor kv_decode_attention(const Tensor& q, const Tensor& k, const Tensor& v, Te
 
 // Route-major tau, isd [R*T] and bf16(h) [R*T, r] for a handful of rows (one launch).
 std::vector<Tensor> score_stats_rows(const Tensor& h, const Tensor& off, const Tensor& gram,
-                                     const Tensor& esum, double inv_u) {
+                                     const Tensor& esum, double inv_u, int64_t n_zero) {
   TORCH_CHECK(h.is_cuda() && h.dim() == 3 && h.scalar_type() == torch::kFloat32 && h.stride(2) == 1);
   const int T = h.size(0), R = h.size(1), r = h.size(2);
   TORCH_CHECK(off.is_cuda() && off.dim() == 2 && off.scalar_type() == torch::kFloat32 &&
@@ -892,13 +892,14 @@ std::vector<Tensor> score_stats_rows(const Tensor& h, const Tensor& off, const T
   const c10::cuda::CUDAGuard guard(h.device());
   auto o = gram.options();
   auto tau = torch::empty({R * T}, o), isd = torch::empty({R * T}, o);
-  auto hb = torch::empty({R * T, r}, o.dtype(torch::kBFloat16));
+  auto hb = torch::empty({R * T, r}, o.dtype(torch::kBFloat16)), zero = torch::empty({n_zero}, o);
   int rc = dsb_score_stats_rows(h.data_ptr<float>(), h.stride(0), h.stride(1), off.data_ptr<float>(),
                                 off.stride(0), off.stride(1), gram.data_ptr<float>(),
                                 esum.data_ptr<float>(), inv_u, T, R, r, tau.data_ptr<float>(),
-                                isd.data_ptr<float>(), hb.data_ptr(), cur_stream());
+                                isd.data_ptr<float>(), hb.data_ptr(), n_zero > 0 ? zero.data_ptr<float>() : nullptr,
+                                n_zero, cur_stream());
   TORCH_CHECK(rc == 0, "dsb_score_stats_rows failed with code ", rc);
-  return {tau, isd, hb};
+  return {tau, isd, hb, zero};
 }
 
 // dh fp32 [N, r], w bf16 [N, r] (row stride padded to 8), d_off [N], d_esum [r].

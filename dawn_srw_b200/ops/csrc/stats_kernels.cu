@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "common/ptx.cuh"
 #include "dsb_api_ops.h"
 
 namespace {
@@ -254,70 +255,71 @@ __global__ void __launch_bounds__(256) score_route_bwd_kernel(
   for (int j = threadIdx.x; j < r; j += blockDim.x) atomicAdd(d_esum + j, s_sum[j]);
 }
 
-constexpr int kRowGroups = 8;      // thread groups that share the rows of G
-constexpr int kRowThreads = 128;   // threads of a group: one column of G each (strided)
-
 // A handful of rows (decoding): the whole statistic in one launch, fp32 throughout.
-// Block n handles token t = n % T of route ri = n / T (route-major output rows, the
-// order in which the routes of one pool are stacked into one gate-kernel call).
-// Thread j owns column j of the symmetric G: consecutive threads read consecutive
-// addresses of every row of G.
-__global__ void score_stats_rows_kernel(const float* __restrict__ h, long long h_st, long long h_sr,
-                                        const float* __restrict__ off, long long o_st, long long o_sr,
-                                        const float* __restrict__ gram, const float* __restrict__ esum,
-                                        float inv_u, int T, int r, float* __restrict__ tau,
-                                        float* __restrict__ isd, __nv_bfloat16* __restrict__ hb) {
+// Row n is token t = n % T of route ri = n / T (route-major output rows, the order in which
+// the routes of one pool are stacked into one gate-kernel call).  h G h^T is a sum over the rows of
+// G, so a cluster of eight CTAs shares them and only scalars meet in the first CTA; thread j owns
+// column j of the symmetric G (consecutive addresses), sixteen loads in flight.  One block per row
+// pulled all of G through one SM: 7.2 us at r = 256 (256 KB) and 15 us at r = 384, a tenth of a
+// decoded token (400M, one sequence: 3.03 ms a token, 2.80 with this; 1B, six: 9.25 and 8.58).  `zero` is scratch of the launch that follows (partial sums, counters).
+constexpr int kRowCtas = 8, kRowThreads = 256;
+__global__ void __cluster_dims__(kRowCtas, 1, 1) __launch_bounds__(kRowThreads)
+score_stats_rows_kernel(const float* __restrict__ h, long long h_st, long long h_sr,
+                        const float* __restrict__ off, long long o_st, long long o_sr,
+                        const float* __restrict__ gram, const float* __restrict__ esum, float inv_u,
+                        int T, int r, float* __restrict__ tau, float* __restrict__ isd,
+                        __nv_bfloat16* __restrict__ hb, float* __restrict__ zero, long long n_zero) {
   __shared__ float s_h[kMaxR];
-  __shared__ float s_part[kRowGroups][kMaxR];
-  __shared__ float s_red[2][32];
-  const int n = blockIdx.x, t = n % T, ri = n / T;
+  __shared__ float s_red[2][kRowThreads / 32];
+  __shared__ float s_m2;
+  const int cta = blockIdx.x, n = blockIdx.y, t = n % T, ri = n / T, tid = threadIdx.x;
   const float* hr = h + t * h_st + ri * h_sr;
-  for (int j = threadIdx.x; j < r; j += blockDim.x) {
+  for (long long i = (static_cast<long long>(n) * kRowCtas + cta) * kRowThreads + tid; i < n_zero;
+       i += static_cast<long long>(gridDim.y) * kRowCtas * kRowThreads)
+    zero[i] = 0.f;
+  for (int j = tid; j < r; j += kRowThreads) {
     const __nv_bfloat16 q = __float2bfloat16(hr[j]);     // the gate kernels see bf16(h)
-    hb[static_cast<size_t>(n) * r + j] = q;
+    if (cta == 0) hb[static_cast<size_t>(n) * r + j] = q;
     s_h[j] = __bfloat162float(q);
   }
   __syncthreads();
-  // (G h)_j: the rows of G are dealt to kRowGroups thread groups, eight independent
-  // accumulators per thread keep the loads in flight
-  const int grp = threadIdx.x / kRowThreads, tj = threadIdx.x % kRowThreads;
-  const int rows_per = (r + kRowGroups - 1) / kRowGroups;
-  const int i0 = grp * rows_per, i1 = min(r, i0 + rows_per);
-  for (int j = tj; j < r; j += kRowThreads) {
-    float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    int i = i0;
-    for (; i + 8 <= i1; i += 8) {
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        a[k] = fmaf(gram[static_cast<size_t>(i + k) * r + j], s_h[i + k], a[k]);
-    }
-    for (; i < i1; ++i) a[0] = fmaf(gram[static_cast<size_t>(i) * r + j], s_h[i], a[0]);
-    s_part[grp][j] = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
-  }
-  __syncthreads();
+  const int per = (r + kRowCtas - 1) / kRowCtas;
+  const int i0 = cta * per, i1 = min(r, i0 + per);
   float m2 = 0.f, m1 = 0.f;
-  for (int j = threadIdx.x; j < r; j += blockDim.x) {
-    float acc = 0.f;
+  for (int j = tid; j < r; j += kRowThreads) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* col = gram + j;
+    int i = i0;
+    for (; i + 16 <= i1; i += 16) {
+      float v[16];
 #pragma unroll
-    for (int g = 0; g < kRowGroups; ++g) acc += s_part[g][j];
-    m2 = fmaf(acc, s_h[j], m2);
-    m1 = fmaf(esum[j], s_h[j], m1);
+      for (int k = 0; k < 16; ++k) v[k] = col[static_cast<size_t>(i + k) * r];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) a[k & 3] = fmaf(v[k], s_h[i + k], a[k & 3]);
+    }
+    for (; i < i1; ++i) a[0] = fmaf(col[static_cast<size_t>(i) * r], s_h[i], a[0]);
+    m2 = fmaf((a[0] + a[1]) + (a[2] + a[3]), s_h[j], m2);
+    if (cta == 0) m1 = fmaf(esum[j], s_h[j], m1);
   }
   m2 = warp_sum(m2);
   m1 = warp_sum(m1);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) { s_red[0][warp] = m2; s_red[1][warp] = m1; }
+  if ((tid & 31) == 0) { s_red[0][tid >> 5] = m2; s_red[1][tid >> 5] = m1; }
   __syncthreads();
-  if (warp == 0) {
-    const int nw = blockDim.x >> 5;
-    m2 = warp_sum(lane < nw ? s_red[0][lane] : 0.f) * inv_u;
-    const float mu = warp_sum(lane < nw ? s_red[1][lane] : 0.f) * inv_u;
-    if (lane == 0) {
-      const float sd = sqrtf(fmaxf(m2 - mu * mu, kVarFloor)) + kSdEps;
-      tau[n] = fmaf(off[t * o_st + ri * o_sr], sd, mu);
-      isd[n] = 1.f / sd;
-    }
+  m2 = m1 = 0.f;
+#pragma unroll
+  for (int w = 0; w < kRowThreads / 32; ++w) { m2 += s_red[0][w]; m1 += s_red[1][w]; }
+  if (tid == 0) s_m2 = m2;
+  dsb::cluster_sync_all();
+  if (cta == 0 && tid == 0) {
+    m2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < kRowCtas; ++k) m2 += dsb::ld_cluster_f32(dsb::mapa_shared(dsb::smem_u32(&s_m2), k));
+    const float mu = m1 * inv_u;
+    const float sd = sqrtf(fmaxf(m2 * inv_u - mu * mu, kVarFloor)) + kSdEps;
+    tau[n] = fmaf(off[t * o_st + ri * o_sr], sd, mu);
+    isd[n] = 1.f / sd;
   }
+  dsb::cluster_sync_all();   // nobody leaves while its shared memory may still be read
 }
 
 // ------------------------------------------------------------ load balance
@@ -598,12 +600,14 @@ extern "C" int dsb_score_stats_bwd(const float* d_tau, const float* d_isd, const
 extern "C" int dsb_score_stats_rows(const float* h, long long h_st, long long h_sr, const float* off,
                                     long long o_st, long long o_sr, const float* gram,
                                     const float* esum, float inv_u, int T, int R, int r, float* tau,
-                                    float* isd, void* hb_bf16, cudaStream_t stream) {
+                                    float* isd, void* hb_bf16, float* zero, long long n_zero,
+                                    cudaStream_t stream) {
   if (T <= 0 || R <= 0) return 0;
   if (r <= 0 || r > kMaxR) return 801;
-  score_stats_rows_kernel<<<T * R, kRowGroups * kRowThreads, 0, stream>>>(h, h_st, h_sr, off, o_st, o_sr, gram, esum, inv_u,
-                                                     T, r, tau, isd,
-                                                     static_cast<__nv_bfloat16*>(hb_bf16));
+  if (static_cast<long long>(T) * R > 65535) return 804;
+  score_stats_rows_kernel<<<dim3(kRowCtas, T * R), kRowThreads, 0, stream>>>(
+      h, h_st, h_sr, off, o_st, o_sr, gram, esum, inv_u, T, r, tau, isd,
+      static_cast<__nv_bfloat16*>(hb_bf16), zero, n_zero);
   return cudaGetLastError() == cudaSuccess ? 0 : 802;
 }
 

@@ -1013,7 +1013,9 @@ class CudaBackend:
             count_launches(2)
             return list(out.reshape(Rr, T, D).unbind(0))
         if stack:
-            tau, inv_sd, h_rm = score_stats_rows(h, tau_off, ex["gram"], ex["esum"], U_tot)
+            # y and den, cleared by the same launch (the splits of the write GEMM add up in y)
+            tau, inv_sd, h_rm, work = score_stats_rows(h, tau_off, ex["gram"], ex["esum"], U_tot,
+                                                       Rr * T * (D + 1))
             x_rm = x_bf.repeat(Rr, 1) if Rr > 1 else x_bf
             calls = [(h_rm, x_rm, tau, inv_sd)]
         else:
@@ -1023,9 +1025,9 @@ class CudaBackend:
             count_launches(3)
             calls = [(hb[i * T:(i + 1) * T], x_bf, tau[i * T:(i + 1) * T], inv_sd[i * T:(i + 1) * T])
                      for i in range(Rr)]
-        # y and den of all calls, cleared by one fill (the splits of the write GEMM add up in y)
         Tr = calls[0][0].shape[0]
-        work = torch.zeros(len(calls) * Tr * (D + 1), dtype=torch.float32, device=dev)
+        if not stack:
+            work = torch.zeros(len(calls) * Tr * (D + 1), dtype=torch.float32, device=dev)
         ys = work[:len(calls) * Tr * D].view(len(calls), Tr, D)
         dens = work[len(calls) * Tr * D:].view(len(calls), Tr)
         p = torch.empty(Tr, Up, dtype=torch.bfloat16, device=dev)

@@ -114,23 +114,25 @@ def score_stats(h, tau_off, gram, esum, n_units: int, gram_split=None):
 
 
 @torch.no_grad()
-def score_stats_rows(h, tau_off, gram, esum, n_units: int):
+def score_stats_rows(h, tau_off, gram, esum, n_units: int, n_zero: int = 0):
     """Forward-only statistics of a handful of rows (generation) in one launch:
     h [T, R, r], tau_off [T, R] -> route-major (row ``ri * T + t``) tau [R*T],
-    inv_sigma [R*T] and the bf16 copy of h [R*T, r]."""
+    inv_sigma [R*T] and the bf16 copy of h [R*T, r].  With ``n_zero``, a fourth result: that
+    many fp32 zeros, cleared by the same launch (what the next launches add into)."""
     T, Rr, r = h.shape
     inv_u = 1.0 / float(n_units)
     if h.is_cuda:
         from . import cuda_backend as CB
         hf = h if h.dtype == torch.float32 and h.stride(2) == 1 else h.float().contiguous()
         off = tau_off if tau_off.dtype == torch.float32 else tau_off.float()
-        tau, isd, hb = CB.ext().score_stats_rows(hf, off, gram.detach().float().contiguous(),
-                                                 esum.detach().float().contiguous(), inv_u)
+        tau, isd, hb, zero = CB.ext().score_stats_rows(hf, off, gram.detach().float().contiguous(),
+                                                       esum.detach().float().contiguous(), inv_u, n_zero)
         CB.count_launches(1)
-        return tau, isd, hb
+        return (tau, isd, hb, zero) if n_zero else (tau, isd, hb)
     hb = h.detach().to(torch.bfloat16).transpose(0, 1).reshape(Rr * T, r)
     hf = hb.float()
     mu = (hf @ esum.float()) * inv_u
     m2 = ((hf @ gram.float()) * hf).sum(-1) * inv_u
     sd = torch.sqrt((m2 - mu * mu).clamp_min(VAR_FLOOR)) + SD_EPS
-    return mu + tau_off.float().t().reshape(-1) * sd, 1.0 / sd, hb
+    out = (mu + tau_off.float().t().reshape(-1) * sd, 1.0 / sd, hb)
+    return out + (torch.zeros(n_zero, device=h.device),) if n_zero else out

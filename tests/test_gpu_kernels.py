@@ -847,3 +847,23 @@ def test_route_backward_row_step(cb, T, D):
     den[0] = float("nan")
     dyb, _ = cb.ext().route_bwd_rows(dy, y, den, 1.5, None, None, dtau, None)
     assert bool(dyb[0].isnan().all()) and bool(dyb[1:].isfinite().all())
+
+
+@pytest.mark.parametrize("T,R,r", [(1, 1, 8), (2, 2, 120), (1, 2, 136), (64, 2, 384), (5, 1, 512)])
+def test_score_statistics_of_a_few_rows_over_a_cluster(cb, T, R, r):
+    """CTAs with no row of G, with fewer and with more than sixteen; strided inputs; the scratch
+    that the launch clears.  fp32 sums of r^2 terms against fp64: 2e-5."""
+    from dawn_srw_b200.ops.score_stats import score_stats_rows
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(r)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    h, off = rn(T, R * r + 5)[:, 2:2 + R * r].unflatten(1, (R, r)), rn(T, R + 1)[:, :R]
+    emb = rn(700, r).double() / r ** 0.5
+    gram, esum = emb.t() @ emb, emb.sum(0)
+    tau, isd, hb, zero = score_stats_rows(h, off, gram.float(), esum.float(), 700, 10007)
+    assert torch.equal(hb, h.transpose(0, 1).reshape(R * T, r).bfloat16())
+    assert zero.numel() == 10007 and float(zero.abs().max()) == 0.0
+    hd = hb.double()
+    mu = hd @ esum / 700
+    sd = (((hd @ gram) * hd).sum(-1) / 700 - mu * mu).sqrt()
+    assert _rel(tau, mu + off.t().reshape(-1).double() * sd) < 2e-5 and _rel(isd, 1 / sd) < 2e-5
