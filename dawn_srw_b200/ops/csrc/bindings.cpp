@@ -796,20 +796,20 @@ std::vector<Tensor> srw_stats_bwd(const Tensor& dtau, const Tensor& dh32, c10::o
 std::vector<Tensor> srw_rows(const Tensor& h, const Tensor& x, const Tensor& tau, const Tensor& isd,
                              const Tensor& emb, const Tensor& read, const Tensor& write,
                              c10::optional<Tensor> unit_mask, std::vector<double> gate, double scale,
-                             c10::optional<Tensor> scale_t) {
+                             c10::optional<Tensor> scale_t, c10::optional<Tensor> work) {
   check_bf16_2d(h, "h"); check_bf16_2d(x, "x"); check_bf16_2d(emb, "emb");
   check_bf16_2d(read, "read"); check_bf16_2d(write, "write");
   const int N = h.size(0), r = h.size(1), D = x.size(1), U = emb.size(0);
-  TORCH_CHECK(h.is_contiguous() && x.is_contiguous() && x.size(0) == N && emb.size(1) == r &&
+  TORCH_CHECK(h.is_contiguous() && x.is_contiguous() && x.size(0) >= 1 && N % x.size(0) == 0 && emb.size(1) == r &&
               read.size(0) == U && read.size(1) == D && write.size(0) == U && write.size(1) == D);
   TORCH_CHECK(N >= 1 && N <= dsb_srw_rows_max(D), "srw_rows: too many rows for this d_model");
   TORCH_CHECK(tau.scalar_type() == torch::kFloat32 && tau.is_contiguous() && tau.numel() == N &&
               isd.scalar_type() == torch::kFloat32 && isd.is_contiguous() && isd.numel() == N);
   const c10::cuda::CUDAGuard guard(x.device());
-  const int NR = N <= 1 ? 1 : N <= 2 ? 2 : 4;
-  const int blocks = dsb_srw_rows_blocks(N, D);
   auto o = tau.options();
-  auto part = torch::empty({static_cast<int64_t>(blocks) * NR * (D + 1)}, o);
+  const int64_t n_work = static_cast<int64_t>(N) * (D + 1) + 1;
+  auto wk = work.has_value() && work->defined() ? *work : torch::zeros({n_work}, o);
+  TORCH_CHECK(f32(wk) && wk.is_contiguous() && wk.numel() >= n_work, "srw_rows: bad scratch");
   auto out = torch::empty({N, D}, o), den = torch::empty({N}, o);
   DsbGate g = to_gate(gate);
   const float* sp = nullptr;
@@ -817,12 +817,10 @@ std::vector<Tensor> srw_rows(const Tensor& h, const Tensor& x, const Tensor& tau
     TORCH_CHECK(scale_t->is_cuda() && scale_t->scalar_type() == torch::kFloat32 && scale_t->numel() == 1);
     sp = scale_t->data_ptr<float>();
   }
-  float* part_p = part.data_ptr<float>();
-  int rc = dsb_srw_rows(h.data_ptr(), x.data_ptr(), tau.data_ptr<float>(), isd.data_ptr<float>(),
+  int rc = dsb_srw_rows(h.data_ptr(), x.data_ptr(), x.size(0), tau.data_ptr<float>(), isd.data_ptr<float>(),
                         emb.data_ptr(), emb.stride(0), read.data_ptr(), read.stride(0),
                         write.data_ptr(), write.stride(0), opt_f32(unit_mask), N, U, r, D, &g,
-                        static_cast<float>(scale), sp, part_p,
-                        part_p + static_cast<size_t>(blocks) * NR * D, out.data_ptr<float>(),
+                        static_cast<float>(scale), sp, wk.data_ptr<float>(), out.data_ptr<float>(),
                         den.data_ptr<float>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_srw_rows failed with code ", rc);
   return {out, den};
@@ -1058,7 +1056,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("srw_route_fwd", &srw_route_fwd);
   m.def("route_bwd_rows", &route_bwd_rows);
   m.def("srw_stats_bwd", &srw_stats_bwd);
-  m.def("srw_rows", &srw_rows);
+  m.def("srw_rows", &srw_rows, py::arg("h"), py::arg("x"), py::arg("tau"), py::arg("isd"), py::arg("emb"),
+        py::arg("read"), py::arg("write"), py::arg("unit_mask"), py::arg("gate"), py::arg("scale"),
+        py::arg("scale_t"), py::arg("work") = py::none());
   m.def("gemv_rows", &gemv_rows);
   m.def("dropout", &dropout);
   m.def("kv_decode_attention", &kv_decode_attention);

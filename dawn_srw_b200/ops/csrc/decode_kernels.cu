@@ -1,18 +1,22 @@
 // SRW pool op for a handful of token rows (KV-cache decoding at batch 1..4).
 //
 // With one to four rows the op is a stream over the pool: per unit u it needs
-// e_u (r values), r_u and w_u (d_model values each), about 5.6 KB at the 400M
-// shapes, and a few hundred FMAs.  A tensor-core tile would spend a 128-row MMA on
-// those rows, so this path is plain SIMT and bound by HBM: one warp per unit,
-//   s_t  = <h_t, e_u>           (warp reduction)
-//   g_t  = gate(s_t; tau_t, 1/sigma_t),   den_t += den_term
-//   xr_t = <x_t, r_u>           (only if some g_t != 0: the relu-type gates of
-//                                v3.9.4 / v4.0.1 are exactly zero below the
-//                                threshold, and then r_u and w_u are not read)
-//   acc_t += bf16(g_t * xr_t) * w_u
-// Each block keeps its partial outputs; a second kernel adds the blocks' partials
-// and applies scale / max(sum den, 1).  The reference runs the generic chunked
-// kernels for decoding (models/dawn_spatial_v41_exp.py:1713-1739, 1913-1957).
+// e_u (r values), and r_u and w_u (d_model values each) where some row's gate is not
+// zero (the relu-type gates of v3.9.4 / v4.0.1 are exactly zero below the threshold),
+//   s_t  = <h_t, e_u>,   g_t = gate(s_t; tau_t, 1/sigma_t),   den_t += den_term
+//   acc_t += bf16(g_t * <x_t, r_u>) * w_u
+// and a few hundred FMAs.  A tensor-core tile would spend a 128-row MMA on those rows, so
+// this path is plain SIMT and bound by HBM - if enough loads are in flight.  A block
+// therefore takes its units in two phases: all scores first, four embedding rows in flight
+// per group of lanes, the units with a gate going on a list in shared memory; then the
+// listed units, dealt evenly to the warps, with the next unit's read row and this unit's
+// write row in flight.  (A warp that took a unit from score to write waited out the latency of
+// HBM twice for every active one.)  Blocks add their sums to global memory with vector
+// reductions; the last one to arrive applies scale / max(sum den, 1).  One row, 28 % of the units
+// active: 100 000 units of 256 + 2 x 1280 and 10 400 of them in 35.5 us on average, 43.6 before (with
+// the kernel that added the blocks' partials); 25 200 and 2 600 units of 128 + 2 x 384 in 11.3, 15.9.
+// The reference runs the generic chunked kernels for decoding
+// (models/dawn_spatial_v41_exp.py:1713-1739, 1913-1957).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -55,7 +59,7 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {
 
 struct RowsParams {
   const __nv_bfloat16* h;       // [N, r]   contiguous
-  const __nv_bfloat16* x;       // [N, D]   contiguous
+  const __nv_bfloat16* x;       // [N / x_rep, D] contiguous: row n of h goes with row n % (N / x_rep)
   const float* tau;             // [N]
   const float* isd;             // [N]
   const __nv_bfloat16* emb;     // [U, lde]
@@ -63,38 +67,57 @@ struct RowsParams {
   const __nv_bfloat16* write;   // [U, ldw]
   const float* unit_mask;       // [U] or null
   long long lde, ldr, ldw;
-  int N, U, r, D;
-  float* part;                  // [blocks, NR, D] partial outputs
-  float* den_part;              // [blocks, NR]
+  int N, x_rows, U, r, D;
+  int lpu;                      // lanes that share a unit's embedding row (power of two)
+  float* acc;                   // zeroed scratch: [N, D] sums, [N] denominators, then the arrival counter
+  float* out;                   // [N, D]
+  float* den_out;               // [N] or null
+  float scale;
+  const float* scale_ptr;
   GateConsts gc;
 };
 
-// NR: rows handled (N <= NR); KC: 16-byte chunks of a d_model row per lane.
-template <int KIND, int NR, int KC>
+__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+               : "memory");
+}
+
+constexpr int kListUnits = 512;     // units of a block between two list phases
+
+// NR: rows handled (N <= NR); KC: 16-byte chunks of a d_model row per lane; EC: of an embedding row.
+template <int KIND, int NR, int KC, int EC>
 __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) srw_rows_kernel(const RowsParams p) {
+  // registers allow the next read row to be in flight beside the accumulators
+  constexpr bool kAhead = NR * KC <= 10;
+  constexpr int kScoreUnroll = NR * EC == 1 ? 8 : 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __nv_bfloat16* s_x = reinterpret_cast<__nv_bfloat16*>(smem_raw);                  // [NR][D]
+  float* s_acc = reinterpret_cast<float*>(smem_raw);                                // [warps][NR][D]
+  __nv_bfloat16* s_x = reinterpret_cast<__nv_bfloat16*>(s_acc + kRowWarps * NR * p.D);   // [NR][D]
   __nv_bfloat16* s_h = s_x + NR * p.D;                                              // [NR][r]
-  float* s_acc = reinterpret_cast<float*>(s_h + NR * p.r);                          // [NR][D]
-  float* s_den = s_acc + NR * p.D;                                                  // [NR]
+  float* s_g = reinterpret_cast<float*>(s_h + NR * p.r);                            // [kListUnits][NR]
+  int* s_u = reinterpret_cast<int*>(s_g + kListUnits * NR);                         // [kListUnits]
+  __shared__ float s_den[kRowWarps][NR];
+  __shared__ int s_count, s_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int i = tid; i < NR * p.D; i += blockDim.x) {
-    const int t = i / p.D;
-    s_x[i] = t < p.N ? p.x[i] : __float2bfloat16(0.f);
-    s_acc[i] = 0.f;
+  const int d_chunks = p.D >> 3, r_chunks = p.r >> 3;
+  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+  for (int t = 0; t < NR; ++t) {
+    const uint4* xs = reinterpret_cast<const uint4*>(p.x) + static_cast<size_t>(t % p.x_rows) * d_chunks;
+    const uint4* hs = reinterpret_cast<const uint4*>(p.h) + static_cast<size_t>(t) * r_chunks;
+    for (int c = tid; c < d_chunks; c += kRowWarps * 32)
+      reinterpret_cast<uint4*>(s_x)[t * d_chunks + c] = t < p.N ? xs[c] : none;
+    for (int c = tid; c < r_chunks; c += kRowWarps * 32)
+      reinterpret_cast<uint4*>(s_h)[t * r_chunks + c] = t < p.N ? hs[c] : none;
   }
-  for (int i = tid; i < NR * p.r; i += blockDim.x) {
-    const int t = i / p.r;
-    s_h[i] = t < p.N ? p.h[i] : __float2bfloat16(0.f);
-  }
-  if (tid < NR) s_den[tid] = 0.f;
+  if (tid == 0) s_count = 0;
   __syncthreads();
   RowGate rg[NR];
 #pragma unroll
   for (int t = 0; t < NR; ++t)
     rg[t] = row_gate<KIND>(p.gc, t < p.N ? p.tau[t] : 0.f, t < p.N ? p.isd[t] : 1.f);
 
-  const int d_chunks = p.D >> 3, r_chunks = p.r >> 3;
+  const int lpu = p.lpu, sub = lane & (lpu - 1), groups = kRowWarps * 32 / lpu, grp = tid / lpu;
   float acc[NR][KC * 8];
   float den[NR];
 #pragma unroll
@@ -103,156 +126,189 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
 #pragma unroll
     for (int j = 0; j < KC * 8; ++j) acc[t][j] = 0.f;
   }
-  const int warps_total = gridDim.x * kRowWarps;
-  constexpr int kEC = kMaxRouteDim / 256;      // 16-byte chunks of an embedding row per lane
-  auto load_emb = [&](int u, uint4 (&eq)[kEC]) {
+  const int per = (p.U + gridDim.x - 1) / gridDim.x;
+  const int u_lo = blockIdx.x * per, u_hi = min(p.U, u_lo + per);
+  for (int base = u_lo; base < u_hi; base += kListUnits) {
+    const int end = min(u_hi, base + kListUnits);
+    // ---- scores and gates of units [base, end)
+    for (int u0 = base; u0 < end; u0 += kScoreUnroll * groups) {          // block-uniform trip count
+      uint4 eq[kScoreUnroll][EC];
 #pragma unroll
-    for (int k = 0; k < kEC; ++k) {
-      const int c = lane + 32 * k;
-      eq[k] = (u < p.U && c < r_chunks) ? ldg_stream(p.emb + static_cast<size_t>(u) * p.lde + 8 * c)
-                                        : make_uint4(0u, 0u, 0u, 0u);
-    }
-  };
-  uint4 e_next[kEC];
-  load_emb(blockIdx.x * kRowWarps + warp, e_next);
-  for (int u = blockIdx.x * kRowWarps + warp; u < p.U; u += warps_total) {
-    // ---- scores of this unit for all rows; the next unit's embedding row is already on its way
-    uint4 e_cur[kEC];
+      for (int i = 0; i < kScoreUnroll; ++i) {
+        const int u = u0 + i * groups + grp;
 #pragma unroll
-    for (int k = 0; k < kEC; ++k) e_cur[k] = e_next[k];
-    load_emb(u + warps_total, e_next);
-    float s[NR];
+        for (int k = 0; k < EC; ++k) {
+          const int c = sub + lpu * k;
+          eq[i][k] = u < end && c < r_chunks ? ldg_stream(p.emb + static_cast<size_t>(u) * p.lde + 8 * c)
+                                             : make_uint4(0u, 0u, 0u, 0u);
+        }
+      }
+      float s[kScoreUnroll][NR];
 #pragma unroll
-    for (int t = 0; t < NR; ++t) s[t] = 0.f;
+      for (int i = 0; i < kScoreUnroll; ++i)
 #pragma unroll
-    for (int k = 0; k < kEC; ++k) {
-      const int c = lane + 32 * k;
-      if (c < r_chunks) {
-        float e[8];
-        unpack8(e_cur[k], e);
+        for (int t = 0; t < NR; ++t) s[i][t] = 0.f;
 #pragma unroll
-        for (int t = 0; t < NR; ++t) {
-          float hv[8];
-          unpack8(*reinterpret_cast<const uint4*>(s_h + t * p.r + 8 * c), hv);
+      for (int k = 0; k < EC; ++k) {
+        const int c = sub + lpu * k;
+        if (c < r_chunks) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) s[t] = fmaf(e[j], hv[j], s[t]);
+          for (int t = 0; t < NR; ++t) {
+            float hv[8];
+            unpack8(*reinterpret_cast<const uint4*>(s_h + t * p.r + 8 * c), hv);
+#pragma unroll
+            for (int i = 0; i < kScoreUnroll; ++i) {
+              float e[8];
+              unpack8(eq[i][k], e);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) s[i][t] = fmaf(e[j], hv[j], s[i][t]);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kScoreUnroll; ++i) {
+        const int u = u0 + i * groups + grp;
+#pragma unroll
+        for (int t = 0; t < NR; ++t)
+          for (int o = lpu >> 1; o > 0; o >>= 1) s[i][t] += __shfl_xor_sync(0xffffffffu, s[i][t], o);
+        if (sub == 0 && u < end) {
+          const float um = p.unit_mask != nullptr ? p.unit_mask[u] : 1.f;
+          float g[NR];
+          bool any = false;
+#pragma unroll
+          for (int t = 0; t < NR; ++t) {
+            float dt;
+            gate_fwd_shifted<KIND>(p.gc, fmaf(s[i][t], rg[t].a, rg[t].b), g[t], dt);
+            g[t] *= um;
+            if (t < p.N) {
+              den[t] = fmaf(dt, um, den[t]);
+              any = any || g[t] != 0.f;
+            }
+          }
+          if (any) {
+            const int slot = atomicAdd(&s_count, 1);
+            s_u[slot] = u;
+#pragma unroll
+            for (int t = 0; t < NR; ++t) s_g[slot * NR + t] = g[t];
+          }
         }
       }
     }
-    float g[NR];
-    bool any = false;
-    const float um = p.unit_mask != nullptr ? p.unit_mask[u] : 1.f;
+    __syncthreads();
+    // ---- read scalars and gated writes of the listed units
+    const int n = s_count;
+    auto load_row = [&](const __nv_bfloat16* m, long long ld, int i, uint4 (&q)[KC]) {
+      const __nv_bfloat16* row = m + static_cast<size_t>(i < n ? s_u[i] : 0) * ld;
 #pragma unroll
-    for (int t = 0; t < NR; ++t) {
-      const float st = warp_sum(s[t]);
-      float dt;
-      gate_fwd_shifted<KIND>(p.gc, fmaf(st, rg[t].a, rg[t].b), g[t], dt);
-      g[t] *= um;
-      dt *= um;
-      if (t < p.N) {
-        den[t] += dt;
-        any = any || g[t] != 0.f;
+      for (int k = 0; k < KC; ++k) {
+        const int c = lane + 32 * k;
+        q[k] = i < n && c < d_chunks ? ldg_stream(row + 8 * c) : make_uint4(0u, 0u, 0u, 0u);
       }
-    }
-    if (!any) continue;                                   // warp-uniform: nothing to read or write
-    // ---- read scalars and the gated write, both rows of the unit in flight together
+    };
     uint4 rq[KC], wq[KC];
-#pragma unroll
-    for (int k = 0; k < KC; ++k) {
-      const int c = lane + 32 * k;
-      if (c < d_chunks) {
-        rq[k] = ldg_stream(p.read + static_cast<size_t>(u) * p.ldr + 8 * c);
-        wq[k] = ldg_stream(p.write + static_cast<size_t>(u) * p.ldw + 8 * c);
-      } else {
-        rq[k] = make_uint4(0u, 0u, 0u, 0u);
-        wq[k] = make_uint4(0u, 0u, 0u, 0u);
-      }
+    if (warp < n) {
+      load_row(p.read, p.ldr, warp, rq);
+      load_row(p.write, p.ldw, warp, wq);
     }
-    float xr[NR];
+    for (int i = warp; i < n; i += kRowWarps) {
+      uint4 rn[kAhead ? KC : 1];
+      if constexpr (kAhead) load_row(p.read, p.ldr, i + kRowWarps, rn);
+      float xr[NR];
 #pragma unroll
-    for (int t = 0; t < NR; ++t) xr[t] = 0.f;
+      for (int t = 0; t < NR; ++t) xr[t] = 0.f;
 #pragma unroll
-    for (int k = 0; k < KC; ++k) {
-      const int c = lane + 32 * k;
-      if (c < d_chunks) {
-        float rv[8];
-        unpack8(rq[k], rv);
+      for (int k = 0; k < KC; ++k) {
+        const int c = lane + 32 * k;
+        if (c < d_chunks) {
+          float rv[8];
+          unpack8(rq[k], rv);
 #pragma unroll
-        for (int t = 0; t < NR; ++t) {
-          float xv[8];
-          unpack8(*reinterpret_cast<const uint4*>(s_x + t * p.D + 8 * c), xv);
+          for (int t = 0; t < NR; ++t) {
+            float xv[8];
+            unpack8(*reinterpret_cast<const uint4*>(s_x + t * p.D + 8 * c), xv);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) xr[t] = fmaf(rv[j], xv[j], xr[t]);
+            for (int j = 0; j < 8; ++j) xr[t] = fmaf(rv[j], xv[j], xr[t]);
+          }
         }
       }
+      if constexpr (!kAhead) load_row(p.read, p.ldr, i + kRowWarps, rq);
+      float pv[NR];
+#pragma unroll
+      for (int t = 0; t < NR; ++t)   // p is rounded to bf16, as the tile kernels store it
+        pv[t] = __bfloat162float(__float2bfloat16(s_g[i * NR + t] * warp_sum(xr[t])));
+#pragma unroll
+      for (int k = 0; k < KC; ++k) {
+        float wv[8];
+        unpack8(wq[k], wv);
+#pragma unroll
+        for (int t = 0; t < NR; ++t)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[t][8 * k + j] = fmaf(pv[t], wv[j], acc[t][8 * k + j]);
+      }
+      load_row(p.write, p.ldw, i + kRowWarps, wq);
+      if constexpr (kAhead) {
+#pragma unroll
+        for (int k = 0; k < KC; ++k) rq[k] = rn[k];
+      }
     }
-    float pv[NR];
-#pragma unroll
-    for (int t = 0; t < NR; ++t)   // p is rounded to bf16, as the tile kernels store it
-      pv[t] = __bfloat162float(__float2bfloat16(g[t] * warp_sum(xr[t])));
-#pragma unroll
-    for (int k = 0; k < KC; ++k) {
-      float wv[8];
-      unpack8(wq[k], wv);
-#pragma unroll
-      for (int t = 0; t < NR; ++t)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[t][8 * k + j] = fmaf(pv[t], wv[j], acc[t][8 * k + j]);
-    }
+    __syncthreads();               // the list has been read
+    if (tid == 0) s_count = 0;
+    __syncthreads();
   }
-  // ---- block partials: warps add into shared memory, the block writes one slab
+  // ---- the block's sums: a slab of shared memory per warp (floating-point atomics on shared memory
+  // are compare-and-swap loops, and eight warps on the same words cost more than a small pool's
+  // whole stream), summed on the way to global memory
+  float* slab = s_acc + warp * NR * p.D;
 #pragma unroll
   for (int t = 0; t < NR; ++t) {
 #pragma unroll
     for (int k = 0; k < KC; ++k) {
       const int c = lane + 32 * k;
       if (c < d_chunks) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) atomicAdd(&s_acc[t * p.D + 8 * c + j], acc[t][8 * k + j]);
+        float4* dst = reinterpret_cast<float4*>(slab + t * p.D + 8 * c);
+        const float* a = &acc[t][8 * k];
+        dst[0] = make_float4(a[0], a[1], a[2], a[3]);
+        dst[1] = make_float4(a[4], a[5], a[6], a[7]);
       }
     }
-    if (lane == 0) atomicAdd(&s_den[t], den[t]);
+    const float d = warp_sum(den[t]);
+    if (lane == 0) s_den[warp][t] = d;
   }
   __syncthreads();
-  float* out = p.part + static_cast<size_t>(blockIdx.x) * NR * p.D;
-  for (int i = tid; i < NR * p.D; i += blockDim.x) out[i] = s_acc[i];
-  if (tid < NR) p.den_part[blockIdx.x * NR + tid] = s_den[tid];
-}
-
-// out[t, :] = (sum_b part[b, t, :]) * scale / max(sum_b den_part[b, t], 1).
-// A block covers 32 columns of one row: 8 groups of 32 threads share the blocks'
-// partials (coalesced 128-byte reads), then meet in shared memory.
-__global__ void __launch_bounds__(256) srw_rows_finish_kernel(
-    const float* __restrict__ part, const float* __restrict__ den_part, int blocks, int NR, int N,
-    int D, float scale, const float* __restrict__ scale_ptr, float* __restrict__ out,
-    float* __restrict__ den_out) {
-  __shared__ float s_col[8][32];
-  __shared__ float s_den[8];
-  const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, grp = tid >> 5;
-  const int j = blockIdx.x * 32 + lane;
-  float d = 0.f;
-  for (int b = tid; b < blocks; b += 256) d += den_part[b * NR + t];
-  d = warp_sum(d);
-  if (lane == 0) s_den[grp] = d;
-  float a0 = 0.f, a1 = 0.f;
-  if (j < D) {
-    int b = grp;
-    for (; b + 8 < blocks; b += 16) {
-      a0 += part[(static_cast<size_t>(b) * NR + t) * D + j];
-      a1 += part[(static_cast<size_t>(b + 8) * NR + t) * D + j];
-    }
-    if (b < blocks) a0 += part[(static_cast<size_t>(b) * NR + t) * D + j];
-  }
-  s_col[grp][lane] = a0 + a1;
-  __syncthreads();
-  if (grp == 0) {
-    float den = 0.f, a = 0.f;
+  const int total = p.N * p.D;                                     // D % 8 == 0
+  for (int i = 4 * tid; i < total; i += 4 * kRowWarps * 32) {
+    float4 v = *reinterpret_cast<const float4*>(s_acc + i);
 #pragma unroll
-    for (int g = 0; g < 8; ++g) { den += s_den[g]; a += s_col[g][lane]; }
-    const float sc = (scale_ptr != nullptr ? scale_ptr[0] : scale) / fmaxf(den, 1.f);
-    if (j < D) out[static_cast<size_t>(t) * D + j] = a * sc;
-    if (den_out != nullptr && blockIdx.x == 0 && lane == 0) den_out[t] = den;
+    for (int w = 1; w < kRowWarps; ++w) {
+      const float4 o = *reinterpret_cast<const float4*>(s_acc + w * NR * p.D + i);
+      v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+    }
+    red_add_v4(p.acc + i, v.x, v.y, v.z, v.w);
   }
+  float* den_sum = p.acc + total;
+  if (tid < p.N) {
+    float d = 0.f;
+#pragma unroll
+    for (int w = 0; w < kRowWarps; ++w) d += s_den[w][tid];
+    atomicAdd(den_sum + tid, d);
+  }
+  __threadfence();
+  __syncthreads();
+  unsigned int* counter = reinterpret_cast<unsigned int*>(den_sum + p.N);
+  if (tid == 0) s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const float sc = p.scale_ptr != nullptr ? p.scale_ptr[0] : p.scale;
+  for (int i = 4 * tid; i < total; i += 4 * kRowWarps * 32) {
+    const int t = i / p.D;
+    const float dn = __ldcg(den_sum + t);
+    const float f = sc / fmaxf(dn, 1.f);
+    const float4 v = __ldcg(reinterpret_cast<const float4*>(p.acc + i));
+    *reinterpret_cast<float4*>(p.out + i) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+  }
+  if (p.den_out != nullptr && tid < p.N) p.den_out[tid] = __ldcg(den_sum + tid);
 }
 
 // ------------------------------------------------- attention over the KV cache
@@ -557,31 +613,38 @@ int launch_kv(const KvParams& p, int B, cudaStream_t stream) {
   return launch_kv_nv<8>(p, splits, B, stream);
 }
 
-template <int KIND, int NR, int KC>
+template <int KIND, int NR, int KC, int EC>
 int launch_rows(const RowsParams& p, int blocks, cudaStream_t stream) {
-  const size_t smem = static_cast<size_t>(NR) * (p.D + p.r) * 2 + static_cast<size_t>(NR) * p.D * 4 + NR * 4 + 16;
+  const size_t smem = static_cast<size_t>(NR) * (p.D + p.r) * 2 +
+                      static_cast<size_t>(kRowWarps) * NR * p.D * 4 + static_cast<size_t>(kListUnits) * (NR + 1) * 4;
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(srw_rows_kernel<KIND, NR, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             96 * 1024) != cudaSuccess)
+    if (cudaFuncSetAttribute(srw_rows_kernel<KIND, NR, KC, EC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             200 * 1024) != cudaSuccess)
       return 902;
     attr_set = true;
   }
-  if (smem > 96 * 1024) return 903;
-  srw_rows_kernel<KIND, NR, KC><<<blocks, kRowWarps * 32, smem, stream>>>(p);
+  if (smem > 200 * 1024) return 903;
+  srw_rows_kernel<KIND, NR, KC, EC><<<blocks, kRowWarps * 32, smem, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : 904;
+}
+
+template <int KIND, int EC>
+int dispatch_rows(const RowsParams& p, int NR, int KC, int blocks, cudaStream_t stream) {
+  if (KC == 5) {
+    if (NR == 1) return launch_rows<KIND, 1, 5, EC>(p, blocks, stream);
+    if (NR == 2) return launch_rows<KIND, 2, 5, EC>(p, blocks, stream);
+    return launch_rows<KIND, 4, 5, EC>(p, blocks, stream);
+  }
+  if (NR == 1) return launch_rows<KIND, 1, 8, EC>(p, blocks, stream);
+  if (NR == 2) return launch_rows<KIND, 2, 8, EC>(p, blocks, stream);
+  return 905;
 }
 
 template <int KIND>
 int dispatch_rows(const RowsParams& p, int NR, int KC, int blocks, cudaStream_t stream) {
-  if (KC == 5) {
-    if (NR == 1) return launch_rows<KIND, 1, 5>(p, blocks, stream);
-    if (NR == 2) return launch_rows<KIND, 2, 5>(p, blocks, stream);
-    return launch_rows<KIND, 4, 5>(p, blocks, stream);
-  }
-  if (NR == 1) return launch_rows<KIND, 1, 8>(p, blocks, stream);
-  if (NR == 2) return launch_rows<KIND, 2, 8>(p, blocks, stream);
-  return 905;
+  return p.r <= 256 ? dispatch_rows<KIND, 1>(p, NR, KC, blocks, stream)
+                    : dispatch_rows<KIND, 2>(p, NR, KC, blocks, stream);
 }
 
 }  // namespace
@@ -599,13 +662,14 @@ extern "C" int dsb_srw_rows_blocks(int N, int D) {
   return (N <= 1 && D <= 1280) ? 2 * n : n;   // one row needs 128 registers: two blocks per SM
 }
 
-extern "C" int dsb_srw_rows(const void* h, const void* x, const float* tau, const float* isd,
+extern "C" int dsb_srw_rows(const void* h, const void* x, int x_rows, const float* tau, const float* isd,
                             const void* emb, long long lde, const void* read, long long ldr,
                             const void* write, long long ldw, const float* unit_mask, int N, int U,
                             int r, int D, const DsbGate* gate, float scale, const float* scale_ptr,
-                            float* part, float* den_part, float* out, float* den_out,
-                            cudaStream_t stream) {
+                            float* work, float* out, float* den_out, cudaStream_t stream) {
   if (N <= 0 || U <= 0) return 0;
+  if (x_rows <= 0 || (reinterpret_cast<uintptr_t>(work) & 15) != 0 || (reinterpret_cast<uintptr_t>(out) & 15) != 0)
+    return 907;
   const int max_rows = dsb_srw_rows_max(D);
   if (N > max_rows || r % 8 != 0 || r > kMaxRouteDim || lde % 8 != 0 || ldr % 8 != 0 || ldw % 8 != 0)
     return 901;
@@ -622,20 +686,19 @@ extern "C" int dsb_srw_rows(const void* h, const void* x, const float* tau, cons
   p.write = static_cast<const __nv_bfloat16*>(write);
   p.unit_mask = unit_mask;
   p.lde = lde; p.ldr = ldr; p.ldw = ldw;
-  p.N = N; p.U = U; p.r = r; p.D = D;
-  p.part = part;
-  p.den_part = den_part;
+  p.N = N; p.x_rows = x_rows; p.U = U; p.r = r; p.D = D;
+  p.lpu = 1;
+  while (p.lpu < 32 && 8 * p.lpu < r) p.lpu *= 2;
+  p.acc = work;
+  p.out = out;
+  p.den_out = den_out;
+  p.scale = scale;
+  p.scale_ptr = scale_ptr;
   p.gc = {gate->kind, gate->sharpness, gate->act_threshold, gate->act_cutoff, gate->epsilon,
           gate->max_intensity, gate->clip_max, gate->dead_threshold};
-  int rc;
-  if (gate->kind == 0) rc = dispatch_rows<0>(p, NR, KC, blocks, stream);
-  else if (gate->kind == 1) rc = dispatch_rows<1>(p, NR, KC, blocks, stream);
-  else rc = dispatch_rows<2>(p, NR, KC, blocks, stream);
-  if (rc) return rc;
-  const dim3 grid((D + 31) / 32, N);
-  srw_rows_finish_kernel<<<grid, 256, 0, stream>>>(part, den_part, blocks, NR, N, D, scale, scale_ptr,
-                                                   out, den_out);
-  return cudaGetLastError() == cudaSuccess ? 0 : 906;
+  if (gate->kind == 0) return dispatch_rows<0>(p, NR, KC, blocks, stream);
+  if (gate->kind == 1) return dispatch_rows<1>(p, NR, KC, blocks, stream);
+  return dispatch_rows<2>(p, NR, KC, blocks, stream);
 }
 
 extern "C" int dsb_kv_decode_attention(const float* q, const float* k, const float* v, float* cache_k,

@@ -117,19 +117,19 @@ int dsb_rank1_add(float* g, long long ldg, const float* dm, const float* hs, int
                   cudaStream_t stream);
 
 // SRW pool op for a handful of token rows (decoding): one streaming pass over the pool.
-// h [N, r], x [N, D] bf16 contiguous (row n of x belongs to row n of h), tau / isd [N];
+// h [N, r], x [x_rows, D] bf16 contiguous (row n % x_rows of x belongs to row n of h), tau / isd [N];
 // emb / read / write bf16 with row strides in elements (multiples of 8); unit_mask [U] or null.
 // out[n, :] = (sum_u bf16(g * <x_n, r_u>) w_u) * scale / max(sum_u den_term, 1), fp32 [N, D];
 // scale_ptr (device scalar) overrides scale when not null; den_out [N] may be null.
-// part / den_part: scratch of dsb_srw_rows_blocks(N, D) * NR * D and * NR floats, NR = N rounded
-// up to 1, 2 or 4.  N <= dsb_srw_rows_max(D) (4 up to d_model 1280, 2 up to 2048, else 0).
+// work: N * (D + 1) + 1 zeroed floats of scratch; work and out 16-byte aligned.
+// N <= dsb_srw_rows_max(D) (4 up to d_model 1280, 2 up to 2048, else 0).
 int dsb_srw_rows_max(int D);
 int dsb_srw_rows_blocks(int N, int D);
 struct DsbGate;
-int dsb_srw_rows(const void* h, const void* x, const float* tau, const float* isd, const void* emb,
-                 long long lde, const void* read, long long ldr, const void* write, long long ldw,
-                 const float* unit_mask, int N, int U, int r, int D, const struct DsbGate* gate,
-                 float scale, const float* scale_ptr, float* part, float* den_part, float* out,
+int dsb_srw_rows(const void* h, const void* x, int x_rows, const float* tau, const float* isd,
+                 const void* emb, long long lde, const void* read, long long ldr, const void* write,
+                 long long ldw, const float* unit_mask, int N, int U, int r, int D,
+                 const struct DsbGate* gate, float scale, const float* scale_ptr, float* work, float* out,
                  float* den_out, cudaStream_t stream);
 
 // One decoded token: k, v [B, H*dh] are appended to the fp32 caches [B, H, s_max, dh] at

@@ -132,7 +132,7 @@ def test_forward_gate_kernel_with_few_rows(cb, kind, T):
                                    (2, 2048, 384)])
 def test_streaming_pool_op_for_a_few_rows(cb, kind, N, D, r):
     """The SIMT decode kernel (one pass over the pool, normalisation and scale applied by its
-    second kernel) against the fp32 formula with p rounded to bf16."""
+    last block) against the fp32 formula with p rounded to bf16."""
     from dawn_srw_b200.ops.gates import GateSpec, gate_forward
     dev = torch.device("cuda")
     torch.manual_seed(100 * N + kind)
@@ -867,3 +867,29 @@ def test_score_statistics_of_a_few_rows_over_a_cluster(cb, T, R, r):
     mu = hd @ esum / 700
     sd = (((hd @ gram) * hd).sum(-1) / 700 - mu * mu).sqrt()
     assert _rel(tau, mu + off.t().reshape(-1).double() * sd) < 2e-5 and _rel(isd, 1 / sd) < 2e-5
+
+
+@pytest.mark.parametrize("N,x_rows,U,D,r", [(1, 1, 1, 8, 8), (2, 1, 300, 128, 16), (4, 2, 2999, 256, 264),
+                                            (2, 2, 160000, 64, 8), (1, 1, 6400, 2048, 512)])
+def test_streaming_pool_op_over_unit_counts(cb, N, x_rows, U, D, r):
+    """Blocks without a unit, lanes shared by several units, more units per block than its list
+    holds, rows that share an x row, a mask; against the formula with p rounded to bf16 (3e-3)."""
+    from dawn_srw_b200.ops.gates import GateSpec, gate_forward
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(U)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    spec = GateSpec(kind=1)
+    h, x = rn(N, r).bfloat16(), rn(x_rows, D).bfloat16()
+    emb, read, write = rn(U, r).bfloat16(), rn(U, D).bfloat16(), rn(U, D).bfloat16()
+    mask = (torch.rand(U, device=dev, generator=g) < 0.8).float()
+    s = h.float() @ emb.float().t()
+    sd = s.std(-1, unbiased=False, keepdim=True) + 1.0
+    tau = s.mean(-1, keepdim=True) - 0.1
+    gate, dt, _ = gate_forward(spec, s, tau, sd)
+    xn = x.repeat(N // x_rows, 1).float()
+    p = (gate * mask * (xn @ read.float().t())).bfloat16().float()
+    ref = (p @ write.float()) * (0.7 / (dt * mask).sum(-1).clamp(min=1.0))[:, None]
+    for _ in range(2):
+        out, den = cb.ext().srw_rows(h, x, tau.squeeze(-1).contiguous(), (1 / sd).squeeze(-1).contiguous(),
+                                     emb, read, write, mask, cb._gate_list(spec), 0.7, None)
+        assert _rel(out, ref) < 3e-3 and _rel(den, (dt * mask).sum(-1)) < 1e-4
