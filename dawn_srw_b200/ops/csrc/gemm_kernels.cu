@@ -479,6 +479,137 @@ struct FwdGateEpi {
   }
 };
 
+// ---------------------------------------------- a few token rows (decoding), operands swapped
+// With up to 64 token rows both products of a pool call are a stream over the pool, and a tile with
+// the tokens as its 128 rows fills most of its A operand with zeros: a 16 KB share of every stage
+// that moves nothing.  Here the pool's rows are the M side (128 units, or 128 output columns, a
+// tile) and the 16 to 64 tokens the N side, so a stage is 16 KB of pool and 2 to 8 KB of tokens, eight of
+// them in flight per SM, and a tile is half the work of a 256-wide one, which evens out the last wave.
+// Lanes of an epilogue warp own consecutive units: stores of one token are consecutive addresses.
+// The 1B model's gate kernels, averaged over its pools: 52 us for 75 at 6 sequences; its write GEMMs
+// and projections 27 for 33; a decoded token 6.78 ms for 8.58, with 32 sequences (64 stacked rows of
+// Q and K) 7.90 for 8.73.  Above 64 rows the zeros are the smaller part and the wide tile stays.
+constexpr int kFewRows = 64;
+
+// Column sums over the 32 lanes of 16 values each; lane l gets the sum of value l & 15.
+__device__ __forceinline__ float warp_column_sums16(float (&d)[16], int lane) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) d[j] += __shfl_xor_sync(0xffffffffu, d[j], 16);
+#pragma unroll
+  for (int w = 8; w > 0; w >>= 1) {
+    const bool up = (lane & w) != 0;
+#pragma unroll
+    for (int j = 0; j < w; ++j) {
+      const float keep = up ? d[j + w] : d[j], give = up ? d[j] : d[j + w];
+      d[j] = keep + __shfl_xor_sync(0xffffffffu, give, w);
+    }
+  }
+  return d[0];
+}
+
+struct FewRowsGateParams {
+  const float* tau;        // [T]
+  const float* inv_sigma;  // [T]
+  float* den_sum;          // [T] += sum_U den_term
+  const float* unit_mask;  // optional [U]
+  __nv_bfloat16* p;        // [T, ldp]
+  long long ldp;
+  GateConsts gc;
+};
+template <int KIND>
+struct FewRowsGateEpi {
+  static constexpr int kNumAcc = 2;
+  static constexpr int kNumOut = 0;
+  static constexpr int kOutBufs = 0;
+  static constexpr int kEpiWarps = 4;
+  __host__ __device__ static constexpr int acc_bufs(int) { return 2; }
+  using Params = FewRowsGateParams;
+  template <int BN, class Ctl>
+  __device__ static void run(const Params& p, const CUtensorMap*, WarpStager&, Ctl& ctl, int m0, int n0,
+                             int M, int N, int warp, int lane) {
+    if (m0 + warp * 32 >= M) { ctl.skip(); return; }   // warp-uniform
+    const int u = m0 + warp * 32 + lane;
+    const bool u_ok = u < M;
+    const float um = u_ok ? (p.unit_mask != nullptr ? p.unit_mask[u] : 1.f) : 0.f;
+    const uint32_t acc_s = ctl.wait(0), acc_xr = ctl.wait(1);
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 16) {
+      const int t0 = n0 + c;
+      if (t0 >= N) break;
+      float s[16], xr[16];
+      tmem_ld16(acc_s + c, s);
+      tmem_ld16(acc_xr + c, xr);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int t = t0 + j;
+        const bool ok = u_ok && t < N;
+        const RowGate rg = row_gate<KIND>(p.gc, t < N ? p.tau[t] : 0.f, t < N ? p.inv_sigma[t] : 1.f);
+        float g, dt;
+        gate_fwd_shifted<KIND>(p.gc, fmaf(s[j], rg.a, rg.b), g, dt);
+        if (ok) p.p[static_cast<size_t>(t) * p.ldp + u] = __float2bfloat16(g * um * xr[j]);
+        s[j] = ok ? dt * um : 0.f;
+      }
+      const float d = warp_column_sums16(s, lane);
+      if (lane < 16 && t0 + lane < N) atomicAdd(p.den_sum + t0 + lane, d);
+    }
+    ctl.release(0);
+    ctl.release(1);
+  }
+};
+
+// out[t, n] (=|+=) (x . w^T)[t, n] * norm / max(den[t], 1) + bias[n]; rows of a tile are columns n.
+struct FewRowsEpi {
+  static constexpr int kNumAcc = 1;
+  static constexpr int kNumOut = 0;
+  static constexpr int kOutBufs = 0;
+  static constexpr int kEpiWarps = 4;
+  __host__ __device__ static constexpr int acc_bufs(int) { return 2; }
+  struct Params {
+    float* out;
+    long long ldo;
+    const float* bias;       // optional
+    const float* den;        // optional [T]
+    const float* norm_ptr;   // optional
+    float norm;
+    int accumulate;
+  };
+  template <int BN, class Ctl>
+  __device__ static void run(const Params& p, const CUtensorMap*, WarpStager&, Ctl& ctl, int m0, int n0,
+                             int M, int N, int warp, int lane) {
+    if (m0 + warp * 32 >= M) { ctl.skip(); return; }   // warp-uniform
+    const int n = m0 + warp * 32 + lane;
+    const float norm = p.norm_ptr != nullptr ? *p.norm_ptr : p.norm;
+    const float b = p.bias != nullptr && n < M ? p.bias[n] : 0.f;
+    const uint32_t acc = ctl.wait(0);
+#pragma unroll 1
+    for (int c = 0; c < BN; c += 16) {
+      const int t0 = n0 + c;
+      if (t0 >= N) break;
+      float v[16];
+      tmem_ld16(acc + c, v);
+      tmem_ld_wait();
+      if (n < M) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int t = t0 + j;
+          if (t < N) {
+            float f = norm;
+            if (p.den != nullptr) {
+              const float d = p.den[t];
+              f /= d < 1.f ? 1.f : d;                  // a NaN stays one
+            }
+            float* dst = p.out + static_cast<size_t>(t) * p.ldo + n;
+            if (p.accumulate) atomicAdd(dst, v[j] * f);
+            else *dst = fmaf(v[j], f, b);
+          }
+        }
+      }
+    }
+    ctl.release(0);
+  }
+};
+
 template <int KIND>
 __device__ __forceinline__ float gate_shifted(const GateConsts& gc, float s, float tau, float isg) {
   if constexpr (KIND == 0) return s - tau;
@@ -1438,6 +1569,58 @@ static int bwd_gate_wide(const void* h, long long ldh, const void* emb, long lon
 
 using namespace dsb;
 
+namespace dsb {
+// Splits of K so that tiles * splits fill a whole number of waves (1..3) of `units`; a longer wave
+// count is taken only if it fills the machine 5 % better.
+static int choose_k_splits(long long tiles, int units, int k_tiles, int max_by_k) {
+  int want = 1;
+  double best = static_cast<double>(tiles) / ((tiles + units - 1) / units * units);
+  for (int w = 1; w <= 3; ++w) {
+    int s = static_cast<int>(static_cast<long long>(w) * units / tiles);
+    if (s > max_by_k) s = max_by_k;
+    if (s < 2) continue;
+    const long long items = tiles * s;
+    const double fill = static_cast<double>(items) / ((items + units - 1) / units * units);
+    if (fill > best + 0.05) { best = fill; want = s; }
+  }
+  // Every split has to have K tiles of its own: one without would add whatever its CTA's
+  // accumulator still holds (163 tiles in 20 splits of 9 leave the last one empty).
+  const int per_split = (k_tiles + want - 1) / want;
+  return (k_tiles + per_split - 1) / per_split;
+}
+
+template <class Epi>
+static int launch_few_rows(GemmParams<typename Epi::Params>& gp, int T, cudaStream_t stream) {
+  if (T <= 16) return launch_engine_impl<16, Epi, 1>(gp, stream);
+  if (T <= 32) return launch_engine_impl<32, Epi, 1>(gp, stream);
+  return launch_engine_impl<64, Epi, 1>(gp, stream);
+}
+static int few_rows_tile(int T) { return T <= 16 ? 16 : T <= 32 ? 32 : 64; }
+
+// w: [N, K] rows (w_mn == 0) or stored [K, N] (w_mn == 1).
+static int few_rows_gemm(const void* x, long long ldx, const void* w, int w_mn, long long ldw, int T, int N,
+                         int K, const FewRowsEpi::Params& epi, int* status, cudaStream_t stream) {
+  GemmParams<FewRowsEpi::Params> gp;
+  memset(&gp, 0, sizeof(gp));
+  int rc = fill_operand(&gp.tma_a[0], {w, w_mn, ldw}, N, K, kBlockM);
+  if (rc) return 100 + rc;
+  rc = fill_operand(&gp.tma_b[0], {x, 0, ldx}, T, K, few_rows_tile(T));
+  if (rc) return 200 + rc;
+  gp.seg[0] = {(K + kBlockK - 1) / kBlockK, 0, w_mn, 0};
+  gp.n_seg = 1;
+  gp.M = N;
+  gp.N = T;
+  gp.status = status;
+  gp.epi = epi;
+  if (epi.accumulate) {
+    const int k_tiles = gp.seg[0].k_tiles;
+    const int s = k_tiles >= 16 ? choose_k_splits((N + kBlockM - 1) / kBlockM, sm_count(), k_tiles, k_tiles / 8) : 1;
+    if (s > 1) gp.k_splits = s;
+  }
+  return launch_few_rows<FewRowsEpi>(gp, T, stream);
+}
+}  // namespace dsb
+
 static int gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn, long long ldb,
                      int M, int N, int K, void* C, long long ldc, int c_is_bf16, int accumulate,
                      float alpha, const float* row_scale, const float* bias, const float* den,
@@ -1468,24 +1651,8 @@ static int gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int 
     const int units = sm_count() / (pairs ? 2 : 1);
     const int k_tiles = gp.seg[0].k_tiles;
     if (tiles < 2 * units && k_tiles >= 64) {
-      // tiles * splits should fill a whole number of waves (1..3) of SM pairs; a
-      // longer wave count is taken only if it fills the machine 5 % better
       // every split reduce-adds a whole output tile: long splits unless the output is a few rows
-      const int max_by_k = k_tiles / (M <= tm ? 8 : 32);
-      int want = 1;
-      double best = static_cast<double>(tiles) / ((tiles + units - 1) / units * units);
-      for (int w = 1; w <= 3; ++w) {
-        int s = static_cast<int>(static_cast<long long>(w) * units / tiles);
-        if (s > max_by_k) s = max_by_k;
-        if (s < 2) continue;
-        const long long items = tiles * s;
-        const double fill = static_cast<double>(items) / ((items + units - 1) / units * units);
-        if (fill > best + 0.05) { best = fill; want = s; }
-      }
-      // Every split has to have K tiles of its own: one without would add whatever its CTA's
-      // accumulator still holds (163 tiles in 20 splits of 9 leave the last one empty).
-      const int per_split = (k_tiles + want - 1) / want;
-      want = (k_tiles + per_split - 1) / per_split;
+      const int want = choose_k_splits(tiles, units, k_tiles, k_tiles / (M <= tm ? 8 : 32));
       if (want > 1) gp.k_splits = want;
     }
   }
@@ -1500,6 +1667,10 @@ extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void*
                              long long ldb, int M, int N, int K, void* C, long long ldc,
                              int c_is_bf16, int accumulate, float alpha, const float* row_scale,
                              const float* bias, int block_n, int* status, cudaStream_t stream) {
+  if (M > 0 && M <= kFewRows && N > 0 && K > 0 && !a_mn && !b_mn && !c_is_bf16 && !accumulate &&
+      row_scale == nullptr)
+    return few_rows_gemm(A, lda, B, 0, ldb, M, N, K,
+                         {static_cast<float*>(C), ldc, bias, nullptr, nullptr, alpha, 0}, status, stream);
   return gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, C, ldc, c_is_bf16, accumulate, alpha, row_scale,
                    bias, nullptr, nullptr, 1.f, block_n, status, stream);
 }
@@ -1507,6 +1678,10 @@ extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void*
 extern "C" int dsb_srw_write(const void* p, long long ldp, const void* write, long long ldw, int T, int U,
                              int D, const float* den, float norm, const float* norm_ptr, float* y,
                              long long ldy, int accumulate, int* status, cudaStream_t stream) {
+  if (T <= 0 || U <= 0 || D <= 0) return 0;
+  if (T <= kFewRows && accumulate)
+    return few_rows_gemm(p, ldp, write, 1, ldw, T, D, U, {y, ldy, nullptr, den, norm_ptr, norm, 1}, status,
+                         stream);
   return gemm_bf16(p, 0, ldp, write, 1, ldw, T, D, U, y, ldy, 0, accumulate, 1.f, nullptr, nullptr, den,
                    norm_ptr, norm, D <= 128 ? 128 : 256, status, stream);
 }
@@ -1584,6 +1759,26 @@ extern "C" int dsb_srw_fwd_gate_xr(const void* h, long long ldh, const void* emb
   // single CTAs take 128 x 256 tiles and twice as many of them stream the pool.
   const bool solo = wide && T <= kBlockM && xr_out == nullptr && diag == nullptr &&
                     !(gather != nullptr && gather->n_ranks > 1);
+  if (solo && T <= kFewRows && stats == nullptr && alive == nullptr && gate_sum == nullptr) {
+    GemmParams<FewRowsGateParams> fp;
+    memset(&fp, 0, sizeof(fp));
+    const int bn = few_rows_tile(T);
+    int rc = fill_operand(&fp.tma_a[0], {emb, 0, lde}, U, r, kBlockM);
+    rc |= fill_operand(&fp.tma_b[0], {h, 0, ldh}, T, r, bn);
+    rc |= fill_operand(&fp.tma_a[1], {read, 0, ldr}, U, D, kBlockM);
+    rc |= fill_operand(&fp.tma_b[1], {x, 0, ldx}, T, D, bn);
+    if (rc) return 100 + rc;
+    fp.seg[0] = {(r + kBlockK - 1) / kBlockK, 0, 0, 0};
+    fp.seg[1] = {(D + kBlockK - 1) / kBlockK, 1, 0, 0};
+    fp.n_seg = 2;
+    fp.M = U;
+    fp.N = T;
+    fp.status = status;
+    fp.epi = {tau, inv_sigma, den_sum, unit_mask, static_cast<__nv_bfloat16*>(p_out), ldp, make_gc(gate)};
+    if (gate->kind == 0) return launch_few_rows<FewRowsGateEpi<0>>(fp, T, stream);
+    if (gate->kind == 1) return launch_few_rows<FewRowsGateEpi<1>>(fp, T, stream);
+    return launch_few_rows<FewRowsGateEpi<2>>(fp, T, stream);
+  }
   const int brows = solo ? 256 : wide ? 128 : (use_cta_pairs() ? BN / 2 : BN);
   int rc = fill_operand(&gp.tma_a[0], {h, 0, ldh}, T, r, kBlockM);
   rc |= fill_operand(&gp.tma_b[0], {emb, 0, lde}, U, r, brows);

@@ -893,3 +893,50 @@ def test_streaming_pool_op_over_unit_counts(cb, N, x_rows, U, D, r):
         out, den = cb.ext().srw_rows(h, x, tau.squeeze(-1).contiguous(), (1 / sd).squeeze(-1).contiguous(),
                                      emb, read, write, mask, cb._gate_list(spec), 0.7, None)
         assert _rel(out, ref) < 3e-3 and _rel(den, (dt * mask).sum(-1)) < 1e-4
+
+
+@pytest.mark.parametrize("kind", [0, 1, 2])
+@pytest.mark.parametrize("T,U,D,r", [(5, 520, 136, 64), (16, 1000, 384, 128), (17, 5003, 256, 72),
+                                     (33, 16100, 2048, 384), (64, 1580, 1280, 256), (65, 700, 128, 64)])
+def test_route_of_a_few_rows_on_the_tensor_engine(cb, kind, T, U, D, r):
+    """Token tiles of 16, 32 and 64 with ragged rows, units and columns, a mask, K cut into splits,
+    and one row too many for the swapped form; the formula with p rounded to bf16, so 6e-3."""
+    from dawn_srw_b200.ops.gates import GateSpec, gate_forward
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(U + kind)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    spec, Up = GateSpec(kind=kind), (U + 7) // 8 * 8
+    nz = lambda *s: torch.nn.functional.normalize(rn(*s), dim=-1).bfloat16()
+    h, x, emb, read, write = rn(T, r).bfloat16(), rn(T, D).bfloat16(), nz(U, r), nz(U, D), nz(U, D)
+    mask = (torch.rand(U, device=dev, generator=g) < 0.9).float()
+    s = h.float() @ emb.float().t()
+    sd = s.std(-1, unbiased=False, keepdim=True)
+    tau = s.mean(-1, keepdim=True) + 0.6 * sd
+    gate, dt, _ = gate_forward(spec, s, tau, sd)
+    p_ref = (gate * mask * (x.float() @ read.float().t())).bfloat16().float()
+    ref = (p_ref @ write.float()) * (1.3 / (dt * mask).sum(-1).clamp(min=1.0))[:, None]
+    st, scale = cb.status_word(dev), torch.full((1,), 1.3, device=dev)
+    for sc_f, sc_t in ((1.3, None), (1.0, scale)):
+        p = torch.empty(T, Up, device=dev, dtype=torch.bfloat16)
+        y, den = torch.zeros(T, D, device=dev), torch.zeros(T, device=dev)
+        cb.ext().srw_route_fwd(h, x, emb, read, write, p, None, tau.squeeze(-1).contiguous(),
+                               (1 / sd).squeeze(-1).contiguous(), den, None, None, mask,
+                               cb._gate_list(spec), sc_f, sc_t, y, True, st)
+        cb.check_status()
+        assert _rel(den, (dt * mask).sum(-1)) < 1e-4
+        assert _rel(p[:, :U], p_ref) < 8e-3 and _rel(y, ref) < 6e-3
+
+
+@pytest.mark.parametrize("M", [5, 16, 31, 64])
+def test_gemm_of_a_few_rows_with_swapped_operands(cb, M):
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(M)
+    for K, N in ((64, 8), (200, 131), (2048, 1283)):
+        Kp = (K + 7) // 8 * 8
+        x = torch.randn(M, Kp, device=dev, generator=g).bfloat16()[:, :K]
+        w = torch.randn(N, Kp, device=dev, generator=g).bfloat16()[:, :K]
+        bias = torch.randn(N, device=dev, generator=g)
+        ref = 0.5 * (x.double() @ w.double().t()) + bias
+        out = cb.gemm(x, False, w, False, out_dtype=torch.float32, bias=bias, alpha=0.5)
+        assert out.shape == (M, N) and _rel(out, ref) < 1e-5
+    cb.check_status()
