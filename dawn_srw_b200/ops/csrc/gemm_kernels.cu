@@ -1643,17 +1643,26 @@ static int gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int 
   rc = make_out_tmap(&gp.tma_out[0], C, M, N, ldc, c_is_bf16 ? 2 : 4);
   if (rc) return 300 + rc;
   gp.epi = {alpha, row_scale, bias, c_is_bf16, accumulate, 0, 0, nullptr, {}, den, norm_ptr, norm};
-  if (accumulate && !c_is_bf16 && bias == nullptr) {
-    // few output tiles but a long K (pool gradients of a small unit shard): cut K so
-    // that every SM pair has work; the splits meet in the fp32 reduce-add epilogue
+  if (!c_is_bf16 && bias == nullptr) {
+    // few output tiles but a long K (weight gradients, the write GEMM of a small batch): cut K so
+    // that every SM pair has work; the splits meet in the fp32 reduce-add epilogue, in an output
+    // that is cleared first where the caller did not ask to add to it.  Every split reduce-adds a
+    // whole output tile, so splits are long (32 K tiles; 16 where the tiles would leave most of
+    // the chip idle, 8 for a few rows).  384 x 384 from K = 8192 is 4 tiles.
     const int tm = pairs ? 2 * kBlockM : kBlockM;
     const long long tiles = static_cast<long long>((M + tm - 1) / tm) * ((N + BN - 1) / BN);
     const int units = sm_count() / (pairs ? 2 : 1);
     const int k_tiles = gp.seg[0].k_tiles;
     if (tiles < 2 * units && k_tiles >= 64) {
-      // every split reduce-adds a whole output tile: long splits unless the output is a few rows
-      const int want = choose_k_splits(tiles, units, k_tiles, k_tiles / (M <= tm ? 8 : 32));
-      if (want > 1) gp.k_splits = want;
+      const int min_len = M <= tm ? 8 : 4 * tiles <= units ? 16 : 32;
+      const int want = choose_k_splits(tiles, units, k_tiles, k_tiles / min_len);
+      if (want > 1) {
+        gp.k_splits = want;
+        if (!accumulate) {
+          if (cudaMemset2DAsync(C, ldc * sizeof(float), 0, N * sizeof(float), M, stream) != cudaSuccess) return 12;
+          gp.epi.accumulate = 1;
+        }
+      }
     }
   }
   if (!pairs)

@@ -463,9 +463,11 @@ def _route_backward_core(x_bf, h_bf, tau, inv_sd, dy, d_den, hd, spec, U, xr=Non
     return dx, dh32.to(torch.bfloat16), dtau, d_isd
 
 
-def _route_backward_gemms(x_bf, h_bf, tau, inv_sd, dy, d_den, dtau, hd, spec, U, xr, dh32, want_dx=True):
+def _route_backward_gemms(x_bf, h_bf, tau, inv_sd, dy, d_den, dtau, hd, spec, U, xr, dh32, want_dx=True,
+                          dx32=None):
     """Gate step and GEMMs of one route's backward: adds into the zeroed ``dtau`` [T] and the
-    pool's gradient buffers, fills ``dh32`` [T, r] = ds . emb; returns dx (bf16)."""
+    pool's gradient buffers, fills ``dh32`` [T, r] = ds . emb; returns dx (bf16, or fp32 added
+    into ``dx32``)."""
     e = ext()
     dev = x_bf.device
     T = x_bf.shape[0]
@@ -491,7 +493,11 @@ def _route_backward_gemms(x_bf, h_bf, tau, inv_sd, dy, d_den, dtau, hd, spec, U,
     gemm(dxrv, True, x_bf, True, out=hd.g_read[:U], accumulate=True)    # dxr^T x
     gemm(dsv, True, h_bf, True, out=hd.g_emb[:U], accumulate=True)      # ds^T h
     gemm(dsv, False, emb, True, out=dh32)                               # ds . emb
-    return gemm(dxrv, False, read, True, out_dtype=torch.bfloat16) if want_dx else None   # dxr . read
+    if not want_dx:
+        return None
+    if dx32 is not None:
+        return gemm(dxrv, False, read, True, out=dx32, accumulate=True)  # dxr . read
+    return gemm(dxrv, False, read, True, out_dtype=torch.bfloat16)
 
 
 class _SRWRouteFn(torch.autograd.Function):
@@ -581,7 +587,11 @@ class _SRWCallFn(torch.autograd.Function):
         dh32 = torch.empty(R * T, r, dtype=torch.float32, device=dev)
         d_scale = torch.zeros_like(sc_t) if sc_t is not None and ctx.needs_input_grad[3] else None
         xrs, ctx.xrs = ctx.xrs, [None] * R
-        dx = None
+        # few tokens: dx is a handful of tiles with K = U, which only an fp32 output lets the SM
+        # pairs share; the routes then add up there too
+        D = x_bf.shape[1]
+        few = ctx.needs_input_grad[0] and 2 * (-(-T // 256)) * (-(-D // 256)) <= 74
+        dx = torch.zeros(T, D, dtype=torch.float32, device=dev) if few else None
         for i in range(R):
             rows = slice(i * T, (i + 1) * T)
             dy = grads[i]
@@ -591,10 +601,13 @@ class _SRWCallFn(torch.autograd.Function):
             dyb, d_den = e.route_bwd_rows(dy, ys[i], den[i], sc_f, sc_t,
                                           None if d_den_ext is None else d_den_ext[i], dtau[rows], d_scale)
             dxi = _route_backward_gemms(x_bf, hb[rows], tau[rows], isd[rows], dyb, d_den, dtau[rows],
-                                        hd, spec, U, xrs[i], dh32[rows], ctx.needs_input_grad[0])
+                                        hd, spec, U, xrs[i], dh32[rows], ctx.needs_input_grad[0],
+                                        dx if few else None)
             xrs[i] = None
             if dxi is not None:
-                dx = dxi if dx is None else dx.add_(dxi)
+                dx = dxi if dx is None or few else dx.add_(dxi)
+        if few:
+            dx = dx.to(torch.bfloat16)
         g_esum = hd.g_esum if hd.g_esum is not None else torch.zeros_like(ctx.esum)
         dh, d_off = e.srw_stats_bwd(dtau, dh32, d_hsum, off.detach(), tau, isd, mu, sd, hg, hb, ctx.esum,
                                     inv_u, spec.kind == GATE_GELU_Z, hd.g_gram, g_esum, st)

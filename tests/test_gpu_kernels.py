@@ -940,3 +940,20 @@ def test_gemm_of_a_few_rows_with_swapped_operands(cb, M):
         out = cb.gemm(x, False, w, False, out_dtype=torch.float32, bias=bias, alpha=0.5)
         assert out.shape == (M, N) and _rel(out, ref) < 1e-5
     cb.check_status()
+
+
+@pytest.mark.parametrize("M,N,K,a_mn", [(384, 384, 8192, True), (8, 384, 8200, True), (512, 384, 25200, False),
+                                        (300, 131, 10400, False), (256, 128, 4096, True)])
+def test_plain_gemm_with_few_tiles_and_a_long_k(cb, M, N, K, a_mn):
+    """K is cut although the caller does not accumulate: whatever the output held is gone, rows
+    beyond its width stay, and a row scale applies once per split part (fp32 sums: 1e-5)."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(K + M)
+    A = torch.randn(M, K, device=dev, generator=g).bfloat16()
+    B = torch.randn((N + 7) // 8 * 8, K, device=dev, generator=g).bfloat16()[:N]
+    rs = torch.rand(M, device=dev, generator=g)
+    buf = torch.full((M, (N + 7) // 8 * 8 + 8), float("nan"), device=dev)
+    ref = 0.3 * (A.double() @ B.double().t()) * rs[:, None]
+    cb.gemm(A.t().contiguous() if a_mn else A, a_mn, B, False, out=buf[:, :N], alpha=0.3, row_scale=rs)
+    cb.check_status()
+    assert _rel(buf[:, :N], ref) < 1e-5 and bool(buf[:, N:].isnan().all())
