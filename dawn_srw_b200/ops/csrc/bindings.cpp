@@ -796,7 +796,7 @@ std::vector<Tensor> srw_stats_bwd(const Tensor& dtau, const Tensor& dh32, c10::o
 std::vector<Tensor> srw_rows(const Tensor& h, const Tensor& x, const Tensor& tau, const Tensor& isd,
                              const Tensor& emb, const Tensor& read, const Tensor& write,
                              c10::optional<Tensor> unit_mask, std::vector<double> gate, double scale,
-                             c10::optional<Tensor> scale_t, c10::optional<Tensor> work) {
+                             c10::optional<Tensor> scale_t) {
   check_bf16_2d(h, "h"); check_bf16_2d(x, "x"); check_bf16_2d(emb, "emb");
   check_bf16_2d(read, "read"); check_bf16_2d(write, "write");
   const int N = h.size(0), r = h.size(1), D = x.size(1), U = emb.size(0);
@@ -807,9 +807,7 @@ std::vector<Tensor> srw_rows(const Tensor& h, const Tensor& x, const Tensor& tau
               isd.scalar_type() == torch::kFloat32 && isd.is_contiguous() && isd.numel() == N);
   const c10::cuda::CUDAGuard guard(x.device());
   auto o = tau.options();
-  const int64_t n_work = static_cast<int64_t>(N) * (D + 1) + 1;
-  auto wk = work.has_value() && work->defined() ? *work : torch::zeros({n_work}, o);
-  TORCH_CHECK(f32(wk) && wk.is_contiguous() && wk.numel() >= n_work, "srw_rows: bad scratch");
+  auto part = torch::empty({static_cast<int64_t>(dsb_srw_rows_blocks(N, D)) * N * (D + 1)}, o);
   auto out = torch::empty({N, D}, o), den = torch::empty({N}, o);
   DsbGate g = to_gate(gate);
   const float* sp = nullptr;
@@ -820,7 +818,7 @@ std::vector<Tensor> srw_rows(const Tensor& h, const Tensor& x, const Tensor& tau
   int rc = dsb_srw_rows(h.data_ptr(), x.data_ptr(), x.size(0), tau.data_ptr<float>(), isd.data_ptr<float>(),
                         emb.data_ptr(), emb.stride(0), read.data_ptr(), read.stride(0),
                         write.data_ptr(), write.stride(0), opt_f32(unit_mask), N, U, r, D, &g,
-                        static_cast<float>(scale), sp, wk.data_ptr<float>(), out.data_ptr<float>(),
+                        static_cast<float>(scale), sp, part.data_ptr<float>(), out.data_ptr<float>(),
                         den.data_ptr<float>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_srw_rows failed with code ", rc);
   return {out, den};
@@ -1056,9 +1054,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("srw_route_fwd", &srw_route_fwd);
   m.def("route_bwd_rows", &route_bwd_rows);
   m.def("srw_stats_bwd", &srw_stats_bwd);
-  m.def("srw_rows", &srw_rows, py::arg("h"), py::arg("x"), py::arg("tau"), py::arg("isd"), py::arg("emb"),
-        py::arg("read"), py::arg("write"), py::arg("unit_mask"), py::arg("gate"), py::arg("scale"),
-        py::arg("scale_t"), py::arg("work") = py::none());
+  m.def("srw_rows", &srw_rows);
   m.def("gemv_rows", &gemv_rows);
   m.def("dropout", &dropout);
   m.def("kv_decode_attention", &kv_decode_attention);

@@ -11,8 +11,10 @@
 // per group of lanes, the units with a gate going on a list in shared memory; then the
 // listed units, dealt evenly to the warps, with the next unit's read row and this unit's
 // write row in flight.  (A warp that took a unit from score to write waited out the latency of
-// HBM twice for every active one.)  Blocks add their sums to global memory with vector
-// reductions; the last one to arrive applies scale / max(sum den, 1).  One row, 28 % of the units
+// HBM twice for every active one.)  Every sum has a fixed order: lists are compacted in unit order,
+// blocks write partial outputs, and a second kernel adds those and applies scale / max(sum den, 1);
+// adding them up with global reductions would save that launch, but a decoded token would no longer
+// repeat bit by bit.  One row, 28 % of the units
 // active: 100 000 units of 256 + 2 x 1280 and 10 400 of them in 35.5 us on average, 43.6 before (with
 // the kernel that added the blocks' partials); 25 200 and 2 600 units of 128 + 2 x 384 in 11.3, 15.9.
 // The reference runs the generic chunked kernels for decoding
@@ -69,18 +71,10 @@ struct RowsParams {
   long long lde, ldr, ldw;
   int N, x_rows, U, r, D;
   int lpu;                      // lanes that share a unit's embedding row (power of two)
-  float* acc;                   // zeroed scratch: [N, D] sums, [N] denominators, then the arrival counter
-  float* out;                   // [N, D]
-  float* den_out;               // [N] or null
-  float scale;
-  const float* scale_ptr;
+  float* part;                  // [blocks, N, D] partial outputs
+  float* den_part;              // [blocks, N]
   GateConsts gc;
 };
-
-__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
-}
 
 constexpr int kListUnits = 512;     // units of a block between two list phases
 
@@ -95,9 +89,9 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
   __nv_bfloat16* s_x = reinterpret_cast<__nv_bfloat16*>(s_acc + kRowWarps * NR * p.D);   // [NR][D]
   __nv_bfloat16* s_h = s_x + NR * p.D;                                              // [NR][r]
   float* s_g = reinterpret_cast<float*>(s_h + NR * p.r);                            // [kListUnits][NR]
-  int* s_u = reinterpret_cast<int*>(s_g + kListUnits * NR);                         // [kListUnits]
+  int* s_u = reinterpret_cast<int*>(s_g + kListUnits * NR);                         // [kListUnits] active units
   __shared__ float s_den[kRowWarps][NR];
-  __shared__ int s_count, s_last;
+  __shared__ int s_cnt[kRowWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int d_chunks = p.D >> 3, r_chunks = p.r >> 3;
   const uint4 none = make_uint4(0u, 0u, 0u, 0u);
@@ -110,7 +104,6 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
     for (int c = tid; c < r_chunks; c += kRowWarps * 32)
       reinterpret_cast<uint4*>(s_h)[t * r_chunks + c] = t < p.N ? hs[c] : none;
   }
-  if (tid == 0) s_count = 0;
   __syncthreads();
   RowGate rg[NR];
 #pragma unroll
@@ -174,32 +167,50 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
           for (int o = lpu >> 1; o > 0; o >>= 1) s[i][t] += __shfl_xor_sync(0xffffffffu, s[i][t], o);
         if (sub == 0 && u < end) {
           const float um = p.unit_mask != nullptr ? p.unit_mask[u] : 1.f;
-          float g[NR];
-          bool any = false;
 #pragma unroll
           for (int t = 0; t < NR; ++t) {
-            float dt;
-            gate_fwd_shifted<KIND>(p.gc, fmaf(s[i][t], rg[t].a, rg[t].b), g[t], dt);
-            g[t] *= um;
-            if (t < p.N) {
-              den[t] = fmaf(dt, um, den[t]);
-              any = any || g[t] != 0.f;
-            }
-          }
-          if (any) {
-            const int slot = atomicAdd(&s_count, 1);
-            s_u[slot] = u;
-#pragma unroll
-            for (int t = 0; t < NR; ++t) s_g[slot * NR + t] = g[t];
+            float g, dt;
+            gate_fwd_shifted<KIND>(p.gc, fmaf(s[i][t], rg[t].a, rg[t].b), g, dt);
+            if (t < p.N) den[t] = fmaf(dt, um, den[t]);
+            s_g[(u - base) * NR + t] = t < p.N ? g * um : 0.f;
           }
         }
       }
     }
     __syncthreads();
+    // ---- the active units, in unit order: a warp compacts kListUnits / kRowWarps of them
+    constexpr int kRounds = kListUnits / kRowWarps / 32;
+    unsigned act[kRounds];
+    int cnt = 0;
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k) {
+      const int l = (warp * kRounds + k) * 32 + lane;
+      bool any = false;
+      if (l < end - base) {
+#pragma unroll
+        for (int t = 0; t < NR; ++t) any = any || s_g[l * NR + t] != 0.f;
+      }
+      act[k] = __ballot_sync(0xffffffffu, any);
+      cnt += __popc(act[k]);
+    }
+    if (lane == 0) s_cnt[warp] = cnt;
+    __syncthreads();
+    int n = 0, slot = 0;
+#pragma unroll
+    for (int w = 0; w < kRowWarps; ++w) {
+      if (w == warp) slot = n;
+      n += s_cnt[w];
+    }
+#pragma unroll
+    for (int k = 0; k < kRounds; ++k) {
+      if ((act[k] >> lane) & 1u)
+        s_u[slot + __popc(act[k] & ((1u << lane) - 1u))] = (warp * kRounds + k) * 32 + lane;
+      slot += __popc(act[k]);
+    }
+    __syncthreads();
     // ---- read scalars and gated writes of the listed units
-    const int n = s_count;
     auto load_row = [&](const __nv_bfloat16* m, long long ld, int i, uint4 (&q)[KC]) {
-      const __nv_bfloat16* row = m + static_cast<size_t>(i < n ? s_u[i] : 0) * ld;
+      const __nv_bfloat16* row = m + static_cast<size_t>(i < n ? base + s_u[i] : 0) * ld;
 #pragma unroll
       for (int k = 0; k < KC; ++k) {
         const int c = lane + 32 * k;
@@ -236,7 +247,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
       float pv[NR];
 #pragma unroll
       for (int t = 0; t < NR; ++t)   // p is rounded to bf16, as the tile kernels store it
-        pv[t] = __bfloat162float(__float2bfloat16(s_g[i * NR + t] * warp_sum(xr[t])));
+        pv[t] = __bfloat162float(__float2bfloat16(s_g[s_u[i] * NR + t] * warp_sum(xr[t])));
 #pragma unroll
       for (int k = 0; k < KC; ++k) {
         float wv[8];
@@ -253,8 +264,6 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
       }
     }
     __syncthreads();               // the list has been read
-    if (tid == 0) s_count = 0;
-    __syncthreads();
   }
   // ---- the block's sums: a slab of shared memory per warp (floating-point atomics on shared memory
   // are compare-and-swap loops, and eight warps on the same words cost more than a small pool's
@@ -284,31 +293,54 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
       const float4 o = *reinterpret_cast<const float4*>(s_acc + w * NR * p.D + i);
       v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
     }
-    red_add_v4(p.acc + i, v.x, v.y, v.z, v.w);
+    *reinterpret_cast<float4*>(p.part + static_cast<size_t>(blockIdx.x) * total + i) = v;
   }
-  float* den_sum = p.acc + total;
   if (tid < p.N) {
     float d = 0.f;
 #pragma unroll
     for (int w = 0; w < kRowWarps; ++w) d += s_den[w][tid];
-    atomicAdd(den_sum + tid, d);
+    p.den_part[blockIdx.x * p.N + tid] = d;
   }
-  __threadfence();
-  __syncthreads();
-  unsigned int* counter = reinterpret_cast<unsigned int*>(den_sum + p.N);
-  if (tid == 0) s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  const float sc = p.scale_ptr != nullptr ? p.scale_ptr[0] : p.scale;
-  for (int i = 4 * tid; i < total; i += 4 * kRowWarps * 32) {
-    const int t = i / p.D;
-    const float dn = __ldcg(den_sum + t);
-    const float f = sc / fmaxf(dn, 1.f);
-    const float4 v = __ldcg(reinterpret_cast<const float4*>(p.acc + i));
-    *reinterpret_cast<float4*>(p.out + i) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+}
+
+// out[t, :] = (sum_b part[b, t, :]) * scale / max(sum_b den_part[b, t], 1).  A block covers 32
+// columns of one row; sixteen warps share the blocks' partials (128-byte reads, eight in flight:
+// with two in flight the launch was bound by their latency, 4.4 us for 1.5 MB).
+constexpr int kFinishWarps = 16;
+__global__ void __launch_bounds__(32 * kFinishWarps) srw_rows_finish_kernel(
+    const float* __restrict__ part, const float* __restrict__ den_part, int blocks, int N, int D,
+    float scale, const float* __restrict__ scale_ptr, float* __restrict__ out, float* __restrict__ den_out) {
+  __shared__ float s_col[kFinishWarps][32];
+  __shared__ float s_den[kFinishWarps];
+  const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int j = blockIdx.x * 32 + lane;
+  float d = 0.f;
+  for (int b = tid; b < blocks; b += 32 * kFinishWarps) d += den_part[b * N + t];
+  d = warp_sum(d);
+  if (lane == 0) s_den[warp] = d;
+  float a = 0.f;
+  if (j < D) {
+    const float* col = part + static_cast<size_t>(t) * D + j;
+    const size_t ld = static_cast<size_t>(N) * D;
+    for (int b = warp; b < blocks; b += 8 * kFinishWarps) {
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = b + k * kFinishWarps < blocks ? col[(b + k * kFinishWarps) * ld] : 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) a += v[k];
+    }
   }
-  if (p.den_out != nullptr && tid < p.N) p.den_out[tid] = __ldcg(den_sum + tid);
+  s_col[warp][lane] = a;
+  __syncthreads();
+  if (warp == 0) {
+    float den = 0.f;
+    a = 0.f;
+#pragma unroll
+    for (int g = 0; g < kFinishWarps; ++g) { den += s_den[g]; a += s_col[g][lane]; }
+    const float sc = (scale_ptr != nullptr ? scale_ptr[0] : scale) / fmaxf(den, 1.f);
+    if (j < D) out[static_cast<size_t>(t) * D + j] = a * sc;
+    if (den_out != nullptr && blockIdx.x == 0 && lane == 0) den_out[t] = den;
+  }
 }
 
 // ------------------------------------------------- attention over the KV cache
@@ -666,10 +698,9 @@ extern "C" int dsb_srw_rows(const void* h, const void* x, int x_rows, const floa
                             const void* emb, long long lde, const void* read, long long ldr,
                             const void* write, long long ldw, const float* unit_mask, int N, int U,
                             int r, int D, const DsbGate* gate, float scale, const float* scale_ptr,
-                            float* work, float* out, float* den_out, cudaStream_t stream) {
+                            float* part, float* out, float* den_out, cudaStream_t stream) {
   if (N <= 0 || U <= 0) return 0;
-  if (x_rows <= 0 || (reinterpret_cast<uintptr_t>(work) & 15) != 0 || (reinterpret_cast<uintptr_t>(out) & 15) != 0)
-    return 907;
+  if (x_rows <= 0 || (reinterpret_cast<uintptr_t>(part) & 15) != 0) return 907;
   const int max_rows = dsb_srw_rows_max(D);
   if (N > max_rows || r % 8 != 0 || r > kMaxRouteDim || lde % 8 != 0 || ldr % 8 != 0 || ldw % 8 != 0)
     return 901;
@@ -689,16 +720,18 @@ extern "C" int dsb_srw_rows(const void* h, const void* x, int x_rows, const floa
   p.N = N; p.x_rows = x_rows; p.U = U; p.r = r; p.D = D;
   p.lpu = 1;
   while (p.lpu < 32 && 8 * p.lpu < r) p.lpu *= 2;
-  p.acc = work;
-  p.out = out;
-  p.den_out = den_out;
-  p.scale = scale;
-  p.scale_ptr = scale_ptr;
+  p.part = part;
+  p.den_part = part + static_cast<size_t>(blocks) * N * D;
   p.gc = {gate->kind, gate->sharpness, gate->act_threshold, gate->act_cutoff, gate->epsilon,
           gate->max_intensity, gate->clip_max, gate->dead_threshold};
-  if (gate->kind == 0) return dispatch_rows<0>(p, NR, KC, blocks, stream);
-  if (gate->kind == 1) return dispatch_rows<1>(p, NR, KC, blocks, stream);
-  return dispatch_rows<2>(p, NR, KC, blocks, stream);
+  int rc;
+  if (gate->kind == 0) rc = dispatch_rows<0>(p, NR, KC, blocks, stream);
+  else if (gate->kind == 1) rc = dispatch_rows<1>(p, NR, KC, blocks, stream);
+  else rc = dispatch_rows<2>(p, NR, KC, blocks, stream);
+  if (rc) return rc;
+  srw_rows_finish_kernel<<<dim3((D + 31) / 32, N), 32 * kFinishWarps, 0, stream>>>(
+      part, p.den_part, blocks, N, D, scale, scale_ptr, out, den_out);
+  return cudaGetLastError() == cudaSuccess ? 0 : 906;
 }
 
 extern "C" int dsb_kv_decode_attention(const float* q, const float* k, const float* v, float* cache_k,

@@ -121,7 +121,7 @@ int dsb_rank1_add(float* g, long long ldg, const float* dm, const float* hs, int
 // emb / read / write bf16 with row strides in elements (multiples of 8); unit_mask [U] or null.
 // out[n, :] = (sum_u bf16(g * <x_n, r_u>) w_u) * scale / max(sum_u den_term, 1), fp32 [N, D];
 // scale_ptr (device scalar) overrides scale when not null; den_out [N] may be null.
-// work: N * (D + 1) + 1 zeroed floats of scratch; work and out 16-byte aligned.
+// part: dsb_srw_rows_blocks(N, D) * N * (D + 1) floats of scratch, 16-byte aligned.
 // N <= dsb_srw_rows_max(D) (4 up to d_model 1280, 2 up to 2048, else 0).
 int dsb_srw_rows_max(int D);
 int dsb_srw_rows_blocks(int N, int D);
@@ -129,7 +129,7 @@ struct DsbGate;
 int dsb_srw_rows(const void* h, const void* x, int x_rows, const float* tau, const float* isd,
                  const void* emb, long long lde, const void* read, long long ldr, const void* write,
                  long long ldw, const float* unit_mask, int N, int U, int r, int D,
-                 const struct DsbGate* gate, float scale, const float* scale_ptr, float* work, float* out,
+                 const struct DsbGate* gate, float scale, const float* scale_ptr, float* part, float* out,
                  float* den_out, cudaStream_t stream);
 
 // One decoded token: k, v [B, H*dh] are appended to the fp32 caches [B, H, s_max, dh] at

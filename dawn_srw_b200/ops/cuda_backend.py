@@ -1018,13 +1018,11 @@ class CudaBackend:
         stack = Rr * T <= 128
         if Rr * T <= e.srw_rows_max(D):
             # one to four rows: a single streaming pass over the pool (SIMT, bound by HBM)
-            tau, inv_sd, h_rm, work = score_stats_rows(h, tau_off, ex["gram"], ex["esum"], U_tot,
-                                                       Rr * T * (D + 1) + 1)
+            tau, inv_sd, h_rm = score_stats_rows(h, tau_off, ex["gram"], ex["esum"], U_tot)
             sc_t = scale.reshape(1) if isinstance(scale, torch.Tensor) else None
             out, _ = e.srw_rows(h_rm, x_bf.contiguous(), tau, inv_sd, pool.emb[:U], pool.read[:U],
-                                pool.write[:U], None, gl, 1.0 if sc_t is not None else float(scale), sc_t,
-                                work)
-            count_launches(1)
+                                pool.write[:U], None, gl, 1.0 if sc_t is not None else float(scale), sc_t)
+            count_launches(2)
             return list(out.reshape(Rr, T, D).unbind(0))
         if stack:
             # y and den, cleared by the same launch (the splits of the write GEMM add up in y)
