@@ -224,18 +224,23 @@ class DAWN(nn.Module):
         rt = self.router
         xf = x.reshape(T, D)
         with trace("attn/router"):
-            h_all = be.linear(xf, rt.proj_attn.weight, rt.proj_attn.bias)
-            h_all = be.dropout(h_all, self.router_dropout, training)
-            tau_all = be.linear(xf, rt.tau_attn.weight, rt.tau_attn.bias).float()    # [T,3]
-        h_qk = h_all[:, : 2 * r].reshape(T, 2, r)
-        h_v = h_all[:, 2 * r:].reshape(T, 1, r)
+            if hasattr(be, "router"):
+                (h_qk, h_v), (tau_qk, tau_v), tau_all = be.router(
+                    xf, rt.proj_attn, rt.tau_attn, self.router_dropout, training, (2 * r, r), (2, 1))
+            else:
+                h_all = be.linear(xf, rt.proj_attn.weight, rt.proj_attn.bias)
+                h_all = be.dropout(h_all, self.router_dropout, training)
+                tau_all = be.linear(xf, rt.tau_attn.weight, rt.tau_attn.bias).float()    # [T,3]
+                h_qk, h_v = h_all[:, : 2 * r], h_all[:, 2 * r:]
+                tau_qk, tau_v = tau_all[:, 0:2], tau_all[:, 2:3]
+        h_qk, h_v = h_qk.reshape(T, 2, r), h_v.reshape(T, 1, r)
         qk_scale, v_scale = self.pool_scale("qk"), self.pool_scale("v")
         with trace("attn/srw_qkv"):
             # the paired Q/K call and the V call read the same activations: one group
             res_qk, res_v = be.srw_group(xf, [
-                dict(h=h_qk, tau_off=tau_all[:, 0:2], pool=pools["qk"], pctx=self.pctx("qk"),
+                dict(h=h_qk, tau_off=tau_qk, pool=pools["qk"], pctx=self.pctx("qk"),
                      out_scale=qk_scale),
-                dict(h=h_v, tau_off=tau_all[:, 2:3], pool=pools["v"], pctx=self.pctx("v"),
+                dict(h=h_v, tau_off=tau_v, pool=pools["v"], pctx=self.pctx("v"),
                      out_scale=v_scale)], self.gate, want_diag=want_diag)
         Q, K, V = res_qk.route(0), res_qk.route(1), res_v.route(0)
         dh = D // H
@@ -265,9 +270,13 @@ class DAWN(nn.Module):
         rt = self.router
         xf = x.reshape(T, D)
         with trace("know/router"):
-            h = be.linear(xf, rt.proj_know.weight, rt.proj_know.bias)
-            h = be.dropout(h, self.router_dropout, training)
-            tau = be.linear(xf, rt.tau_know.weight, rt.tau_know.bias).float()         # [T,1]
+            if hasattr(be, "router"):
+                (h,), _, tau = be.router(xf, rt.proj_know, rt.tau_know, self.router_dropout, training,
+                                         (self.d_route,), (1,))
+            else:
+                h = be.linear(xf, rt.proj_know.weight, rt.proj_know.bias)
+                h = be.dropout(h, self.router_dropout, training)
+                tau = be.linear(xf, rt.tau_know.weight, rt.tau_know.bias).float()     # [T,1]
         k_scale = self.pool_scale("know")
         with trace("know/srw"):
             (res,) = be.srw_group(xf, [dict(h=h.reshape(T, 1, self.d_route), tau_off=tau,

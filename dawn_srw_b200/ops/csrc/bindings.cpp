@@ -842,6 +842,39 @@ Tensor dropout(c10::optional<Tensor> res, const Tensor& x, int64_t seed, double 
   return y;
 }
 
+Tensor dropout_rows(const Tensor& x, int64_t seed, double p) {
+  TORCH_CHECK(f32(x) && x.dim() == 2 && x.stride(1) == 1, "dropout_rows: fp32 rows");
+  const c10::cuda::CUDAGuard guard(x.device());
+  auto y = torch::empty({x.size(0), x.size(1)}, x.options());
+  int rc = dsb_dropout_rows(x.data_ptr<float>(), x.stride(0), y.data_ptr<float>(), x.size(0), x.size(1),
+                            static_cast<unsigned long long>(seed), static_cast<float>(p), cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_dropout_rows failed with code ", rc);
+  return y;
+}
+
+// sources fp32 [T, cols_i] at columns cols0[i] -> bf16 [T, n] and, if wanted, its column sums [n]
+std::vector<Tensor> linear_pack(std::vector<Tensor> srcs, std::vector<int64_t> cols0, int64_t T, int64_t n,
+                                bool want_sum, int64_t seed, double p, int64_t n_drop) {
+  TORCH_CHECK(!srcs.empty() && srcs.size() <= 5 && srcs.size() == cols0.size());
+  DsbPackSrc s[5];
+  for (size_t i = 0; i < srcs.size(); ++i) {
+    const Tensor& t = srcs[i];
+    TORCH_CHECK(f32(t) && t.dim() == 2 && t.stride(1) == 1 && t.size(0) == T && cols0[i] >= 0 &&
+                cols0[i] + t.size(1) <= n, "linear_pack: bad source");
+    s[i] = {t.data_ptr<float>(), t.stride(0), static_cast<int>(cols0[i]), static_cast<int>(t.size(1)), 0};
+  }
+  const c10::cuda::CUDAGuard guard(srcs[0].device());
+  auto o = srcs[0].options();
+  auto dst = torch::empty({T, n}, o.dtype(torch::kBFloat16));
+  auto sum = want_sum ? torch::zeros({n}, o) : Tensor();
+  int rc = dsb_linear_pack(s, static_cast<int>(srcs.size()), T, n, dst.data_ptr(),
+                           want_sum ? sum.data_ptr<float>() : nullptr, static_cast<unsigned long long>(seed),
+                           static_cast<float>(p), n_drop, cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_linear_pack failed with code ", rc);
+  if (want_sum) return {dst, sum};
+  return {dst};
+}
+
 // y = x . W^T + bias for up to four rows (SIMT, one pass over W).
 void gemv_rows(const Tensor& x, const Tensor& w, c10::optional<Tensor> bias, Tensor& y) {
   check_bf16_2d(x, "x"); check_bf16_2d(w, "w");
@@ -1057,6 +1090,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("srw_rows", &srw_rows);
   m.def("gemv_rows", &gemv_rows);
   m.def("dropout", &dropout);
+  m.def("dropout_rows", &dropout_rows);
+  m.def("linear_pack", &linear_pack);
   m.def("kv_decode_attention", &kv_decode_attention);
   m.def("srw_rows_max", [](int64_t D) { return dsb_srw_rows_max(static_cast<int>(D)); });
   m.def("srw_fwd_gate_gather", &srw_fwd_gate_gather);

@@ -61,6 +61,22 @@ int dsb_route_bwd_rows(const float* dy, const float* y, const float* den, const 
 int dsb_dropout(const float* res, const float* x, float* y, long long n, unsigned long long seed,
                 float p, cudaStream_t stream);
 
+// Gradient operand of a linear layer: dst bf16 [T, n] = bf16(sum of the up to five fp32 sources that
+// cover a column: cols columns from col0, row stride ld), 0 where none does; colsum [n] (nullable,
+// zeroed) += its column sums.  With p > 0 the columns [0, n_drop) are the gradient of a dropped
+// [T, n_drop] tensor: the keep mask of (seed, p) is applied.  n % 8 == 0, n_drop % 4 == 0.
+struct DsbPackSrc {
+  const float* ptr;
+  long long ld;
+  int col0, cols;
+  int vec;          // set by the launcher: rows may be read as float4
+};
+int dsb_linear_pack(const struct DsbPackSrc* src, int n_src, int T, int n, void* dst_bf16, float* colsum,
+                    unsigned long long seed, float p, int n_drop, cudaStream_t stream);
+// y [T, n] = dropout(x [T, ldx]) with the mask of the contiguous tensor; n, ldx % 4 == 0.
+int dsb_dropout_rows(const float* x, long long ldx, float* y, int T, int n, unsigned long long seed, float p,
+                     cudaStream_t stream);
+
 // Per-token score statistics from hg = h . (E^T E) (fp32 [N, r]) and bf16 h [N, ldh]:
 //   mu = <h, esum> * inv_u,  var = <hg, h> * inv_u - mu^2,  sd = sqrt(max(var, 1e-12)) + 1e-8,
 //   tau = mu + off * sd,  isd = 1 / sd;  hsum[r] += column sums of h (hsum may be null).

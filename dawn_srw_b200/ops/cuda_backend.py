@@ -230,11 +230,66 @@ class _LinearFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         xb, w_bf = ctx.saved_tensors
-        dyb = _bf16_2d(dy)
+        if dy.dtype == torch.float32 and dy.stride(1) == 1 and dy.shape[1] % 8 == 0:
+            # the bf16 operand and the bias gradient in one pass
+            dyb, *db = ext().linear_pack([dy], [0], dy.shape[0], dy.shape[1], ctx.has_bias, 0, 0.0, 0)
+            db = db[0] if ctx.has_bias else None
+            count_launches(1)
+        else:
+            dyb = _bf16_2d(dy)
+            db = dy.float().sum(0) if ctx.has_bias else None
         dx = gemm(dyb, False, w_bf, True, out_dtype=ctx.x_dtype) if ctx.needs_input_grad[0] else None
         dw = gemm(dyb, True, xb, True, out_dtype=torch.float32)           # dy^T . x
-        db = dy.float().sum(0) if ctx.has_bias else None
         return dx, dw, db, None, None
+
+
+class _RouterFn(torch.autograd.Function):
+    """Router projection and threshold head on the same input as ONE GEMM over their concatenated
+    (8-padded) weights, dropout on the projection.  Returns the projection cut into ``h_cuts``
+    columns, the thresholds cut into ``tau_cuts`` (none if that is a single piece) and all
+    thresholds: views of one buffer, so that neither direction slices, pads or concatenates; the
+    backward pass packs all cotangents into one bf16 operand (one kernel, with the dropout mask
+    and the bias gradients)."""
+
+    @staticmethod
+    def forward(ctx, x, w1, b1, w2, b2, w_cat, b_cat, h_cuts, tau_cuts, p):
+        xb = _bf16_2d(x)
+        n1, n2 = w1.shape[0], w2.shape[0]
+        y = gemm(xb, False, w_cat, False, out_dtype=torch.float32, bias=b_cat)
+        h, seed = y[:, :n1], 0
+        if p > 0.0:
+            seed = int(torch.randint(0, 2 ** 62, (1,)).item())        # CPU generator: no device sync
+            h = ext().dropout_rows(h, seed, p)
+            count_launches(1)
+        ctx.save_for_backward(xb, w_cat)
+        ctx.args = (n1, n2, seed, float(p), x.dtype)
+        tau = y[:, n1:n1 + n2]
+        outs, ctx.cols = [], []
+        for t, cuts, base in ((h, h_cuts, 0), (tau, tau_cuts, n1)):
+            a = 0
+            for n in cuts:
+                outs.append(t[:, a:a + n])
+                ctx.cols.append(base + a)
+                a += n
+        outs.append(tau)
+        ctx.cols.append(n1)
+        ctx.set_materialize_grads(False)
+        return tuple(outs)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        xb, w_cat = ctx.saved_tensors
+        n1, n2, seed, p, x_dtype = ctx.args
+        T, n = xb.shape[0], w_cat.shape[0]
+        srcs = [(g.float(), c) for g, c in zip(grads, ctx.cols) if g is not None]
+        srcs = [(g if g.stride(1) == 1 else g.contiguous(), c) for g, c in srcs]
+        if not srcs:
+            return (None,) * 10
+        dyb, db = ext().linear_pack([g for g, _ in srcs], [c for _, c in srcs], T, n, True, seed, p, n1)
+        count_launches(1)
+        dx = gemm(dyb, False, w_cat, True, out_dtype=x_dtype) if ctx.needs_input_grad[0] else None
+        dw = gemm(dyb, True, xb, True, out_dtype=torch.float32)
+        return (dx, dw[:n1], db[:n1], dw[n1:n1 + n2], db[n1:n1 + n2], None, None, None, None, None)
 
 
 class _DropoutFn(torch.autograd.Function):
@@ -872,6 +927,12 @@ class CudaBackend:
         """Forward-only: several ``nn.Linear`` layers on the same input as ONE GEMM over
         their concatenated (and 8-padded) weights; the bf16 weight and the bias are cached
         until a parameter changes.  Returns one output view per layer."""
+        w, b, cuts = self._cat_weights(layers)
+        y = gemm(_bf16_2d(x), False, w, False, out_dtype=torch.float32, bias=b)
+        return [y[:, a:e] for a, e in cuts]
+
+    @torch.no_grad()
+    def _cat_weights(self, layers):
         key = tuple((l.weight.data_ptr(), l.weight._version,
                      0 if l.bias is None else l.bias._version) for l in layers)
         cache = self.__dict__.setdefault("_cat_cache", {})
@@ -890,9 +951,16 @@ class CudaBackend:
             b = F.pad(torch.cat(bs, 0), (0, pad)).contiguous()
             hit = (key, w, b, cuts)
             cache[id(layers[0])] = hit
-        _, w, b, cuts = hit
-        y = gemm(_bf16_2d(x), False, w, False, out_dtype=torch.float32, bias=b)
-        return [y[:, a:e] for a, e in cuts]
+        return hit[1:]
+
+    def router(self, x, proj, tau, p, training, h_cuts, tau_cuts):
+        """Router projection (cut into ``h_cuts`` columns, under dropout ``p`` in training) and
+        thresholds (cut into ``tau_cuts``) of x: (pieces of h, pieces of tau, all of tau)."""
+        w, b, _ = self._cat_weights((proj, tau))
+        outs = _RouterFn.apply(x, proj.weight, proj.bias, tau.weight, tau.bias, w, b, tuple(h_cuts),
+                               tuple(tau_cuts) if len(tau_cuts) > 1 else (), float(p) if training else 0.0)
+        k = len(h_cuts)
+        return outs[:k], (outs[k:-1] if len(tau_cuts) > 1 else outs[-1:]), outs[-1]
 
     @torch.no_grad()
     def decode_attention(self, q, k, v, cache_k, cache_v, pos, n_heads: int):

@@ -960,3 +960,39 @@ def test_plain_gemm_with_few_tiles_and_a_long_k(cb, M, N, K, a_mn):
     cb.gemm(A.t().contiguous() if a_mn else A, a_mn, B, False, out=buf[:, :N], alpha=0.3, row_scale=rs)
     cb.check_status()
     assert _rel(buf[:, :N], ref) < 1e-5 and bool(buf[:, N:].isnan().all())
+
+
+@pytest.mark.parametrize("T,D,n1,n2,p", [(1, 64, 8, 1, 0.0), (65, 136, 24, 3, 0.0), (300, 384, 384, 3, 0.1),
+                                         (257, 128, 128, 1, 0.1)])
+def test_router_projection_and_its_gradients(cb, T, D, n1, n2, p):
+    """One GEMM for projection and thresholds: pieces, ragged column cuts, dropout and the packed
+    backward operand (cotangents of overlapping thresholds add up) against the separate layers;
+    bf16 operands on both sides, so 1e-2 on gradients."""
+    dev = torch.device("cuda")
+    torch.manual_seed(T)
+    be = cb.CudaBackend()
+    proj, tau = torch.nn.Linear(D, n1).to(dev), torch.nn.Linear(D, n2).to(dev)
+    x0 = torch.randn(T, D, device=dev)
+    cuts, tcuts = ((n1 // 3 * 2, n1 - n1 // 3 * 2), (n2 - 1, 1)) if n2 > 1 else ((n1,), (1,))
+    wh, wt, wa = torch.randn(T, n1, device=dev), torch.randn(T, n2, device=dev), torch.randn(T, n2, device=dev)
+    got = []
+    for fused in (True, False):
+        for l in (proj, tau):
+            l.zero_grad()
+        x = x0.clone().requires_grad_(True)
+        torch.manual_seed(7)
+        if fused:
+            hs, ts, ta = be.router(x, proj, tau, p, True, cuts, tcuts)
+            h, t = torch.cat(hs, 1), torch.cat(ts, 1)
+        else:
+            h = be.dropout(be.linear(x, proj.weight, proj.bias).contiguous(), p, True)
+            t = ta = be.linear(x, tau.weight, tau.bias)
+        ((h * wh).sum() + (t * wt).sum() + (ta * wa).sum()).backward()
+        got.append([h.detach(), t.detach(), ta.detach(), x.grad] + [q.grad.clone() for l in (proj, tau)
+                                                                    for q in (l.weight, l.bias)])
+    cb.check_status()
+    for a, b in zip(*got):
+        assert _rel(a, b) < 1e-2
+    ref = torch.nn.functional.linear(x0.double(), proj.weight.double(), proj.bias.double())
+    kept = got[0][0] != 0
+    assert _rel(got[0][0][kept] * (1 - p), ref[kept]) < 1e-2
