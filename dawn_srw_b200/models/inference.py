@@ -182,10 +182,13 @@ def prefill(model, input_ids: torch.Tensor):
     for li, blk in enumerate(model.layers):
         n = be.layer_norm(x, blk.norm1.weight, blk.norm1.bias).reshape(B * S, D)
         q, k, v, _, _ = _layer_qkv(model, be, n, pools)
-        qh, kh, vh = heads(q), heads(k), heads(v)
-        cache_k[li, :, :, :S] = kh
-        cache_v[li, :, :, :S] = vh
-        o = be.attention(qh, kh, vh, 0.0, False).transpose(1, 2).reshape(B * S, D)
+        if hasattr(be, "prompt_attention"):
+            o = be.prompt_attention(q, k, v, cache_k[li], cache_v[li], B, S)
+        else:
+            qh, kh, vh = heads(q), heads(k), heads(v)
+            cache_k[li, :, :, :S] = kh
+            cache_v[li, :, :, :S] = vh
+            o = be.attention(qh, kh, vh, 0.0, False).transpose(1, 2).reshape(B * S, D)
         x = x + be.linear(o, blk.attn.expand_O.weight, None).reshape(B, S, D)
         n = be.layer_norm(x, blk.norm2.weight, blk.norm2.bias).reshape(B * S, D)
         ko, _ = _know(model, be, n, pools)

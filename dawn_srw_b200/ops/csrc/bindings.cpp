@@ -573,6 +573,34 @@ std::vector<Tensor> attention_bwd(const Tensor& q, const Tensor& k, const Tensor
   return {dq, dk, dv};
 }
 
+// Prompt attention of a cached generation: q, k, v fp32 [B*S, H*dh], caches fp32 [B, H, s_max, dh]
+// (written at positions 0..S-1) -> causal attention output, bf16 [B*S, H*dh].
+Tensor prompt_attention(const Tensor& q, const Tensor& k, const Tensor& v, Tensor& cache_k, Tensor& cache_v,
+                        int64_t B, int64_t S, Tensor& status) {
+  auto ok = [&](const Tensor& t) {
+    return t.is_cuda() && t.scalar_type() == torch::kFloat32 && t.is_contiguous() &&
+           (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  };
+  TORCH_CHECK(ok(q) && ok(k) && ok(v) && ok(cache_k) && ok(cache_v) && q.dim() == 2 && q.sizes() == k.sizes() &&
+              q.sizes() == v.sizes() && q.size(0) == B * S && cache_k.dim() == 4 && cache_k.size(0) == B &&
+              cache_k.sizes() == cache_v.sizes() && cache_k.size(1) * cache_k.size(3) == q.size(1) &&
+              S <= cache_k.size(2), "prompt_attention: bad operands");
+  const c10::cuda::CUDAGuard guard(q.device());
+  const int H = cache_k.size(1), dh = cache_k.size(3), s_max = cache_k.size(2);
+  auto o = q.options().dtype(torch::kBFloat16);
+  auto b16 = torch::empty({4, B * S, q.size(1)}, o);
+  auto lse = torch::empty({B, H, S}, q.options());
+  auto qb = b16[0], kb = b16[1], vb = b16[2], out = b16[3];
+  int rc = dsb_prompt_qkv(q.data_ptr<float>(), k.data_ptr<float>(), v.data_ptr<float>(), qb.data_ptr(),
+                          kb.data_ptr(), vb.data_ptr(), cache_k.data_ptr<float>(), cache_v.data_ptr<float>(), B,
+                          S, H, dh, s_max, cur_stream());
+  if (rc == 0)
+    rc = dsb_attention_fwd(qb.data_ptr(), kb.data_ptr(), vb.data_ptr(), out.data_ptr(), lse.data_ptr<float>(),
+                           B, H, S, dh, 0.0, 0, status.data_ptr<int>(), cur_stream());
+  TORCH_CHECK(rc == 0, "prompt_attention failed with code ", rc);
+  return out;
+}
+
 Tensor embed_fwd(const Tensor& ids, const Tensor& tok, const Tensor& pos) {
   TORCH_CHECK(ids.is_cuda() && ids.dim() == 2 && ids.scalar_type() == torch::kInt64 &&
               ids.is_contiguous() && tok.scalar_type() == torch::kFloat32 && tok.is_contiguous() &&
@@ -1076,6 +1104,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("route_bwd_prologue", &route_bwd_prologue);
   m.def("attention_fwd", &attention_fwd);
   m.def("attention_bwd", &attention_bwd);
+  m.def("prompt_attention", &prompt_attention);
   m.def("grad_sq_norm", &grad_sq_norm);
   m.def("score_stats_fwd", &score_stats_fwd);
   m.def("score_stats_bwd", &score_stats_bwd);

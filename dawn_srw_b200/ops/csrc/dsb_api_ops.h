@@ -77,6 +77,12 @@ int dsb_linear_pack(const struct DsbPackSrc* src, int n_src, int T, int n, void*
 int dsb_dropout_rows(const float* x, long long ldx, float* y, int T, int n, unsigned long long seed, float p,
                      cudaStream_t stream);
 
+// q, k, v fp32 [B*S, H*dh] -> bf16 copies; k, v also into the fp32 caches [B, H, s_max, dh] at
+// positions 0..S-1.  dh % 4 == 0, everything 16-byte aligned, S <= s_max.
+int dsb_prompt_qkv(const float* q, const float* k, const float* v, void* qb, void* kb, void* vb,
+                   float* cache_k, float* cache_v, int B, int S, int H, int dh, int s_max,
+                   cudaStream_t stream);
+
 // Per-token score statistics from hg = h . (E^T E) (fp32 [N, r]) and bf16 h [N, ldh]:
 //   mu = <h, esum> * inv_u,  var = <hg, h> * inv_u - mu^2,  sd = sqrt(max(var, 1e-12)) + 1e-8,
 //   tau = mu + off * sd,  isd = 1 / sd;  hsum[r] += column sums of h (hsum may be null).

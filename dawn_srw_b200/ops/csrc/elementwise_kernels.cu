@@ -739,6 +739,51 @@ extern "C" int dsb_dropout_rows(const float* x, long long ldx, float* y, int T, 
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
+// Prompt of a cached generation: q, k, v fp32 [B * S, H * dh] -> bf16 operands of the attention kernel
+// and, for k and v, their fp32 rows in the caches [B, H, s_max, dh] at positions 0..S-1.  Bound by its
+// bytes (12 read, 14 written per position and column) from a few thousand positions on, by being one
+// launch in place of five below.
+namespace {
+__global__ void __launch_bounds__(256) prompt_qkv_kernel(const float4* __restrict__ q,
+                                                         const float4* __restrict__ k,
+                                                         const float4* __restrict__ v,
+                                                         uint2* __restrict__ qb, uint2* __restrict__ kb,
+                                                         uint2* __restrict__ vb, float* __restrict__ ck,
+                                                         float* __restrict__ cv, int S, int H, int dh4,
+                                                         int s_max, long long n) {
+  auto bf = [](const float4& a) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+  };
+  const int d4 = H * dh4;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) {
+    const float4 a = q[i], b = k[i], c = v[i];
+    qb[i] = bf(a);
+    kb[i] = bf(b);
+    vb[i] = bf(c);
+    const long long row = i / d4;
+    const int col = static_cast<int>(i - row * d4), h = col / dh4, j = col - h * dh4;
+    const long long bi = row / S, s = row - bi * S;
+    const long long at = ((bi * H + h) * s_max + s) * dh4 + j;
+    reinterpret_cast<float4*>(ck)[at] = b;
+    reinterpret_cast<float4*>(cv)[at] = c;
+  }
+}
+}  // namespace
+
+extern "C" int dsb_prompt_qkv(const float* q, const float* k, const float* v, void* qb, void* kb, void* vb,
+                              float* cache_k, float* cache_v, int B, int S, int H, int dh, int s_max,
+                              cudaStream_t stream) {
+  if (B <= 0 || S <= 0 || H <= 0) return 0;
+  if (dh <= 0 || (dh & 3) || S > s_max) return 2;
+  const long long n = static_cast<long long>(B) * S * H * (dh >> 2);
+  prompt_qkv_kernel<<<grid_for(n, 256, 148 * 16), 256, 0, stream>>>(
+      reinterpret_cast<const float4*>(q), reinterpret_cast<const float4*>(k), reinterpret_cast<const float4*>(v),
+      static_cast<uint2*>(qb), static_cast<uint2*>(kb), static_cast<uint2*>(vb), cache_k, cache_v, S, H,
+      dh >> 2, s_max, n);
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+
 // ----------------------------------------------------- multi-tensor launches
 // AdamW and the squared gradient norm over a whole list of tensors in one launch
 // each: a block takes one 64 K-element chunk of one tensor; the chunk -> tensor

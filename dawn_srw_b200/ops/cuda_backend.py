@@ -972,6 +972,18 @@ class CudaBackend:
         count_launches(1)
         return ext().kv_decode_attention(f(q), f(k), f(v), cache_k, cache_v, pos, int(n_heads))
 
+    @torch.no_grad()
+    def prompt_attention(self, q, k, v, cache_k, cache_v, B: int, S: int):
+        """Causal attention over a prompt whose k and v also go into the fp32 caches
+        [B, H, S_max, dh]; q, k, v [B*S, D].  Returns [B*S, D] (bf16, as ``attention``)."""
+        H, dh = cache_k.shape[1], cache_k.shape[3]
+        if dh % 16 != 0 or dh > 128:
+            raise ValueError(f"head dimension {dh} is not supported by the attention kernels "
+                             "(multiple of 16, at most 128)")
+        f = lambda t: t.float().contiguous()
+        count_launches(2)
+        return ext().prompt_attention(f(q), f(k), f(v), cache_k, cache_v, B, S, status_word(q.device))
+
     def embed(self, ids, tok, pos):
         if tok.shape[1] % 4 != 0 or tok.dtype != torch.float32:
             return R.embed(ids, tok, pos)

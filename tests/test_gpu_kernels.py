@@ -996,3 +996,21 @@ def test_router_projection_and_its_gradients(cb, T, D, n1, n2, p):
     ref = torch.nn.functional.linear(x0.double(), proj.weight.double(), proj.bias.double())
     kept = got[0][0] != 0
     assert _rel(got[0][0][kept] * (1 - p), ref[kept]) < 1e-2
+
+
+@pytest.mark.parametrize("B,S,H,dh,s_max", [(1, 1, 1, 16, 1), (3, 109, 6, 64, 128), (2, 130, 2, 80, 131),
+                                            (1, 257, 3, 128, 300)])
+def test_prompt_attention_fills_the_caches(cb, B, S, H, dh, s_max):
+    """Caches exact at 0..S-1 and untouched beyond; output as the attention entry point gives it."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(S)
+    q, k, v = (torch.randn(B * S, H * dh, device=dev, generator=g) for _ in range(3))
+    ck, cv = torch.full((2, B, H, s_max, dh), 7.0, device=dev).unbind(0)
+    be = cb.CudaBackend()
+    o = be.prompt_attention(q, k, v, ck, cv, B, S)
+    heads = lambda t: t.view(B, S, H, dh).transpose(1, 2)
+    assert torch.equal(ck[:, :, :S], heads(k)) and torch.equal(cv[:, :, :S], heads(v))
+    assert bool((ck[:, :, S:] == 7.0).all()) and bool((cv[:, :, S:] == 7.0).all())
+    ref = be.attention(heads(q), heads(k), heads(v), 0.0, False).transpose(1, 2).reshape(B * S, H * dh)
+    cb.check_status()
+    assert torch.equal(o, ref)
