@@ -67,6 +67,152 @@ __global__ void ln_fwd_kernel(const float* __restrict__ x, const float* __restri
   }
 }
 
+__device__ __forceinline__ float4 bf16x4(const uint2& u) {
+  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
+  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
+// The same for rows that can be read as float4 (D % 4 == 0, D <= 128 * NV, 16-byte aligned): one
+// warp per row, the row in registers after NV loads in flight.  Bound by its bytes (6 per element) for
+// many rows, by one round trip to memory for few: 4.4 us for 512 x 1280 and 5.1 us for 8192 x 384
+// (3.7 TB/s); with scalar loads 14.5 and 8.2 us.
+template <int NV>
+__global__ void __launch_bounds__(128) ln_fwd_vec_kernel(const float* __restrict__ x,
+                                                         const float* __restrict__ w,
+                                                         const float* __restrict__ b,
+                                                         __nv_bfloat16* __restrict__ y,
+                                                         float* __restrict__ mean, float* __restrict__ rstd,
+                                                         int T, int D, float eps) {
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= T) return;
+  const int d4 = D >> 2;
+  const float4* xr = reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * D);
+  float4 v[NV];
+  float s = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = lane + 32 * k;
+    v[k] = i < d4 ? xr[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k) s += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+  const float mu = warp_sum(s) / D;
+  float q = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    if (lane + 32 * k < d4) {
+      const float a = v[k].x - mu, c = v[k].y - mu, d = v[k].z - mu, e = v[k].w - mu;
+      q += (a * a + c * c) + (d * d + e * e);
+    }
+  }
+  const float rs = rsqrtf(warp_sum(q) / D + eps);
+  uint2* yr = reinterpret_cast<uint2*>(y + static_cast<size_t>(row) * D);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = lane + 32 * k;
+    if (i < d4) {
+      const float4 g = reinterpret_cast<const float4*>(w)[i], c = reinterpret_cast<const float4*>(b)[i];
+      const __nv_bfloat162 lo = __floats2bfloat162_rn((v[k].x - mu) * rs * g.x + c.x, (v[k].y - mu) * rs * g.y + c.y);
+      const __nv_bfloat162 hi = __floats2bfloat162_rn((v[k].z - mu) * rs * g.z + c.z, (v[k].w - mu) * rs * g.w + c.w);
+      yr[i] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+  if (lane == 0) { mean[row] = mu; rstd[row] = rs; }
+}
+
+// dx of the backward pass under the same conditions: dy and x are read once (7.2 us for 8192 x 384, 8.6
+// with a second read).
+template <int NV>
+__global__ void __launch_bounds__(128) ln_bwd_dx_vec_kernel(const __nv_bfloat16* __restrict__ dy,
+                                                            const float* __restrict__ x,
+                                                            const float* __restrict__ w,
+                                                            const float* __restrict__ mean,
+                                                            const float* __restrict__ rstd,
+                                                            float* __restrict__ dx, int T, int D) {
+  const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= T) return;
+  const int d4 = D >> 2;
+  const float mu = mean[row], rs = rstd[row];
+  const float4* xr = reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * D);
+  const uint2* dyr = reinterpret_cast<const uint2*>(dy + static_cast<size_t>(row) * D);
+  float4 v[NV];
+  uint2 g2[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = lane + 32 * k;
+    v[k] = i < d4 ? xr[i] : make_float4(mu, mu, mu, mu);
+    g2[k] = i < d4 ? dyr[i] : make_uint2(0u, 0u);
+  }
+  float s1 = 0.f, s2 = 0.f;
+  auto scaled = [&](int k) {                       // dy * w of this lane's four columns
+    const int i = lane + 32 * k;
+    const float4 d = bf16x4(g2[k]);
+    const float4 c = i < d4 ? reinterpret_cast<const float4*>(w)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(d.x * c.x, d.y * c.y, d.z * c.z, d.w * c.w);
+  };
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const float4 g = scaled(k);
+    s1 += (g.x + g.y) + (g.z + g.w);
+    s2 += (g.x * ((v[k].x - mu) * rs) + g.y * ((v[k].y - mu) * rs)) +
+          (g.z * ((v[k].z - mu) * rs) + g.w * ((v[k].w - mu) * rs));
+  }
+  s1 = warp_sum(s1) / D;
+  s2 = warp_sum(s2) / D;
+  float4* dxr = reinterpret_cast<float4*>(dx + static_cast<size_t>(row) * D);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = lane + 32 * k;
+    if (i < d4) {
+      const float4 g = scaled(k);
+      dxr[i] = make_float4(rs * (g.x - s1 - (v[k].x - mu) * rs * s2), rs * (g.y - s1 - (v[k].y - mu) * rs * s2),
+                           rs * (g.z - s1 - (v[k].z - mu) * rs * s2), rs * (g.w - s1 - (v[k].w - mu) * rs * s2));
+    }
+  }
+}
+
+// dw, db under the same conditions: a block covers 128 columns (four per thread) of 64 rows (4.3 us for
+// 8192 x 384, 8.9 with 32 columns of 256 rows and scalar loads).
+__global__ void __launch_bounds__(256) ln_bwd_dwdb_vec_kernel(const __nv_bfloat16* __restrict__ dy,
+                                                              const float* __restrict__ x,
+                                                              const float* __restrict__ mean,
+                                                              const float* __restrict__ rstd,
+                                                              float* __restrict__ dw, float* __restrict__ db,
+                                                              int T, int D) {
+  __shared__ float s_w[8][128], s_b[8][128];
+  const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5, c = blockIdx.x * 128 + 4 * cx;
+  const int lo = blockIdx.y * 64, hi = min(T, lo + 64);
+  float aw[4] = {0.f, 0.f, 0.f, 0.f}, ab[4] = {0.f, 0.f, 0.f, 0.f};
+  if (c < D) {
+#pragma unroll 4
+    for (int row = lo + ry; row < hi; row += 8) {
+      const float4 d = bf16x4(*reinterpret_cast<const uint2*>(dy + static_cast<size_t>(row) * D + c));
+      const float4 v = *reinterpret_cast<const float4*>(x + static_cast<size_t>(row) * D + c);
+      const float mu = mean[row], rs = rstd[row];
+      aw[0] += d.x * ((v.x - mu) * rs); aw[1] += d.y * ((v.y - mu) * rs);
+      aw[2] += d.z * ((v.z - mu) * rs); aw[3] += d.w * ((v.w - mu) * rs);
+      ab[0] += d.x; ab[1] += d.y; ab[2] += d.z; ab[3] += d.w;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { s_w[ry][4 * cx + j] = aw[j]; s_b[ry][4 * cx + j] = ab[j]; }
+  __syncthreads();
+  const int col = threadIdx.x & 127, out = blockIdx.x * 128 + col;
+  if (out < D) {
+    const float (*src)[128] = threadIdx.x < 128 ? s_w : s_b;
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += src[k][col];
+    atomicAdd((threadIdx.x < 128 ? dw : db) + out, t);
+  }
+}
+
+bool aligned16(const void* a, const void* b, const void* c, const void* d) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) |
+           reinterpret_cast<uintptr_t>(d)) & 15) == 0;
+}
+
 // A few rows only (decoding): one block of 256 threads per row, the row in
 // registers (D <= 256 * 8), two block reductions.
 __global__ void __launch_bounds__(256) ln_fwd_block_kernel(
@@ -458,6 +604,14 @@ extern "C" int dsb_layernorm_fwd(const float* x, const float* w, const float* b,
     ln_fwd_block_kernel<<<T, 256, 0, stream>>>(x, w, b, y, mean, rstd, D, eps);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
   }
+  if (D % 4 == 0 && D <= 2048 && aligned16(x, w, b, y)) {
+    const int blocks = (T + 3) / 4;
+    if (D <= 512) ln_fwd_vec_kernel<4><<<blocks, 128, 0, stream>>>(x, w, b, y, mean, rstd, T, D, eps);
+    else if (D <= 1280) ln_fwd_vec_kernel<10><<<blocks, 128, 0, stream>>>(x, w, b, y, mean, rstd, T, D, eps);
+    else ln_fwd_vec_kernel<16><<<blocks, 128, 0, stream>>>(x, w, b, y, mean, rstd, T, D, eps);
+    return cudaGetLastError() == cudaSuccess ? 0 : 1;
+  }
+  // rows of other lengths or alignments
   const int warps = 8;
   const dim3 grid((T + warps - 1) / warps), block(warps * 32);
   if (D <= 32 * 16) ln_fwd_kernel<16><<<grid, block, 0, stream>>>(x, w, b, y, mean, rstd, T, D, eps);
@@ -472,6 +626,14 @@ extern "C" int dsb_layernorm_bwd(const void* dy_bf16, const float* x, const floa
                                  float* db, int T, int D, cudaStream_t stream) {
   if (T <= 0) return 0;
   const __nv_bfloat16* dy = reinterpret_cast<const __nv_bfloat16*>(dy_bf16);
+  if (D % 4 == 0 && D <= 2048 && aligned16(x, w, dy, dx)) {
+    const int blocks = (T + 3) / 4;
+    if (D <= 512) ln_bwd_dx_vec_kernel<4><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
+    else if (D <= 1280) ln_bwd_dx_vec_kernel<10><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
+    else ln_bwd_dx_vec_kernel<16><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
+    ln_bwd_dwdb_vec_kernel<<<dim3((D + 127) / 128, (T + 63) / 64), 256, 0, stream>>>(dy, x, mean, rstd, dw, db, T, D);
+    return cudaGetLastError() == cudaSuccess ? 0 : 1;
+  }
   ln_bwd_dx_kernel<<<(T + 7) / 8, 256, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
   const dim3 grid((D + 31) / 32, (T + kLnRowsPerBlock - 1) / kLnRowsPerBlock);
   ln_bwd_dwdb_kernel<<<grid, 256, 0, stream>>>(dy, x, mean, rstd, dw, db, T, D);

@@ -1014,3 +1014,23 @@ def test_prompt_attention_fills_the_caches(cb, B, S, H, dh, s_max):
     ref = be.attention(heads(q), heads(k), heads(v), 0.0, False).transpose(1, 2).reshape(B * S, H * dh)
     cb.check_status()
     assert torch.equal(o, ref)
+
+
+@pytest.mark.parametrize("T,D", [(297, 4), (300, 384), (513, 512), (1000, 516), (299, 1280), (320, 2048),
+                                 (301, 130), (300, 2052)])
+def test_layer_norm_over_row_lengths(cb, T, D):
+    """Vector rows at the edges of their register tiles, a row length that is no multiple of four,
+    one beyond the vector kernels; bf16 output and incoming gradient, so 8e-3 against fp64."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(D)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    x, w, b = (rn(T, D) * 2 + 1).requires_grad_(True), rn(D).requires_grad_(True), rn(D).requires_grad_(True)
+    y = cb.CudaBackend().layer_norm(x, w, b)
+    dy = rn(T, D).bfloat16()
+    y.backward(dy)
+    x6, w6, b6 = (t.detach().double().requires_grad_(True) for t in (x, w, b))
+    ref = torch.nn.functional.layer_norm(x6, (D,), w6, b6, 1e-6)
+    ref.backward(dy.double())
+    assert _rel(y, ref) < 8e-3
+    for a, r in ((x.grad, x6.grad), (w.grad, w6.grad), (b.grad, b6.grad)):
+        assert _rel(a, r) < 1e-4
