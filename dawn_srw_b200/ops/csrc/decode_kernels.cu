@@ -366,9 +366,11 @@ struct KvParams {
 constexpr int kKvThreads = 128, kKvGroups = kKvThreads / 4;
 constexpr int kKvMaxDh = 128;
 
-__device__ __forceinline__ float merge_weight(float m, float m_all) {
-  return m > -INFINITY ? __expf(m - m_all) : 0.f;
-}
+// A running maximum starts at the lowest finite value, not at -inf: a score of -inf then weighs
+// nothing (exp(-inf - finite)) instead of turning into exp(-inf + inf), and a group without a
+// position has nothing to weigh.
+constexpr float kLowest = -3.402823466e38f;
+__device__ __forceinline__ float merge_weight(float m, float m_all) { return __expf(m - m_all); }
 
 // NV: 16-byte chunks of a head row per lane (dh <= 16 * NV, dh % 4 == 0).
 template <int NV>
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(kKvThreads) kv_decode_split_kernel(const KvPar
     qv[i] = c < nv4 ? q4[c] : make_float4(0.f, 0.f, 0.f, 0.f);
     qv[i].x *= p.scale; qv[i].y *= p.scale; qv[i].z *= p.scale; qv[i].w *= p.scale;
   }
-  float m = -INFINITY, l = 0.f;
+  float m = kLowest, l = 0.f;
   float4 o[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -489,7 +491,7 @@ __global__ void __launch_bounds__(kKvThreads) kv_decode_split_kernel(const KvPar
   if (tid == 0) { c_ml[0] = mc; c_ml[1] = lc; }
   cluster_sync_all();
   if (rank == 0) {
-    float ms[8], ls[8], ma = -INFINITY;
+    float ms[8], ls[8], ma = kLowest;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       if (r < splits) {

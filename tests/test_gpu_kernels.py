@@ -1034,3 +1034,19 @@ def test_layer_norm_over_row_lengths(cb, T, D):
     assert _rel(y, ref) < 8e-3
     for a, r in ((x.grad, x6.grad), (w.grad, w6.grad), (b.grad, b6.grad)):
         assert _rel(a, r) < 1e-4
+
+
+def test_decode_attention_with_scores_of_minus_infinity(cb):
+    """A cached key whose score is -inf gets no weight wherever it falls: first of its group, alone
+    in its group, or after others."""
+    from dawn_srw_b200.ops import reference as R
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(3)
+    B, H, dh, S, n = 2, 3, 64, 300, 200
+    ck, cv = (torch.randn(B, H, S, dh, device=dev, generator=g) for _ in range(2))
+    ck[:, :, [0, 1, 33, 64, 190], 5] = float("-inf")
+    q = torch.rand(B, H * dh, device=dev, generator=g) + 0.1
+    k, v = (torch.randn(B, H * dh, device=dev, generator=g) for _ in range(2))
+    out = cb.CudaBackend().decode_attention(q, k, v, ck, cv, torch.tensor([n], device=dev), H)
+    ref = R.cached_attention(q.view(B, H, 1, dh), ck, cv, n + 1).reshape(B, H * dh)
+    assert bool(ref.isfinite().all()) and _rel(out, ref) < 1e-5
