@@ -42,6 +42,8 @@ DsbGate to_gate(const std::vector<double>& g) {
   return d;
 }
 
+bool f32(const Tensor& t) { return t.is_cuda() && t.scalar_type() == torch::kFloat32; }
+
 // C (=|+=) alpha * row_scale * op(A) . op(B)^T + bias.
 //   a_mn == false: A is [M,K];  a_mn == true: A is stored [K,M]
 //   b_mn == false: B is [N,K];  b_mn == true: B is stored [K,N]
@@ -678,8 +680,6 @@ std::vector<Tensor> score_stats_fwd(const Tensor& hg, const Tensor& h, const Ten
   return {tau, isd, mu, sd, hsum};
 }
 
-bool f32(const Tensor& t) { return t.is_cuda() && t.scalar_type() == torch::kFloat32; }
-
 // Statistics of a pool call, routes stacked (row ri * T + t): h fp32 [T, R, r], off [T, R],
 // gcat bf16 [2r, r] = the two bf16 terms of G.  -> hb bf16 [R*T, r], hg fp32 [R*T, 2r] (its halves
 // add up to h . G), tau, isd, mu, sd [R*T], den [R, T] (zeros), hsum [r].
@@ -763,6 +763,79 @@ void srw_route_fwd(const Tensor& h, const Tensor& x, const Tensor& emb, const Te
                      den.data_ptr<float>(), scale, sp, y.data_ptr<float>(), y.stride(0), accumulate,
                      status.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_srw_write failed with code ", rc);
+}
+
+// Gate step and GEMMs of one route's backward in one call (the host side of a small step is its
+// Python and binding time: seven launches, some 12 us each from Python).  With the read scalars xr
+// kept by the forward pass, p overwrites them; otherwise S and XR are recomputed.  dtau [T] is added
+// into, dh32 [T, r] filled, the pool's gradients accumulated; dx: bf16, or fp32 added into dx32.
+c10::optional<Tensor> srw_route_bwd(const Tensor& x, const Tensor& h, const Tensor& tau, const Tensor& isd,
+                                    const Tensor& dy, const Tensor& d_den, Tensor& dtau, const Tensor& emb,
+                                    const Tensor& read, const Tensor& write, Tensor& g_emb, Tensor& g_read,
+                                    Tensor& g_write, c10::optional<Tensor> xr, Tensor& dh32, bool want_dx,
+                                    c10::optional<Tensor> dx32, std::vector<double> gate, Tensor& status) {
+  check_bf16_2d(x, "x"); check_bf16_2d(h, "h"); check_bf16_2d(dy, "dy"); check_bf16_2d(emb, "emb");
+  check_bf16_2d(read, "read"); check_bf16_2d(write, "write");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int T = x.size(0), D = x.size(1), U = emb.size(0), r = emb.size(1);
+  TORCH_CHECK(h.size(0) == T && h.size(1) == r && dy.size(0) == T && dy.size(1) == D && read.size(0) == U &&
+              read.size(1) == D && write.size(0) == U && write.size(1) == D, "srw_route_bwd: bad shapes");
+  auto vec = [&](const Tensor& t) { return f32(t) && t.is_contiguous() && t.numel() == T; };
+  auto mat = [&](const Tensor& t, int rows, int cols) {
+    return f32(t) && t.dim() == 2 && t.size(0) == rows && t.size(1) == cols && t.stride(1) == 1;
+  };
+  TORCH_CHECK(vec(tau) && vec(isd) && vec(d_den) && vec(dtau) && mat(g_emb, U, r) && mat(g_read, U, D) &&
+              mat(g_write, U, D) && mat(dh32, T, r), "srw_route_bwd: bad buffers");
+  auto o16 = x.options();
+  const int64_t Up = (U + 7) / 8 * 8;
+  const bool saved = xr.has_value() && xr->defined();
+  if (saved) {
+    check_bf16_2d(*xr, "xr");
+    TORCH_CHECK(xr->size(0) == T && xr->size(1) == Up && xr->is_contiguous());
+  }
+  auto p = saved ? *xr : torch::empty({T, Up}, o16);
+  auto dxr = torch::empty({T, Up}, o16), ds = torch::empty({T, Up}, o16);
+  DsbGate g = to_gate(gate);
+  const cudaStream_t st = cur_stream();
+  int* status_p = status.data_ptr<int>();
+  int rc;
+  if (saved) {
+    rc = dsb_srw_bwd_gate_xr(h.data_ptr(), h.stride(0), emb.data_ptr(), emb.stride(0), dy.data_ptr(),
+                             dy.stride(0), write.data_ptr(), write.stride(0), p.data_ptr(), Up, T, U, r, D,
+                             p.data_ptr(), dxr.data_ptr(), ds.data_ptr(), Up, tau.data_ptr<float>(),
+                             isd.data_ptr<float>(), d_den.data_ptr<float>(), nullptr, dtau.data_ptr<float>(),
+                             &g, nullptr, status_p, st);
+  } else {
+    // the sigma sum is derived from dh32 and dtau: the kernel's own output for it is unused
+    auto dsz = torch::empty({T}, tau.options());
+    rc = dsb_srw_bwd_gate(h.data_ptr(), h.stride(0), emb.data_ptr(), emb.stride(0), x.data_ptr(), x.stride(0),
+                          read.data_ptr(), read.stride(0), dy.data_ptr(), dy.stride(0), write.data_ptr(),
+                          write.stride(0), T, U, r, D, p.data_ptr(), dxr.data_ptr(), ds.data_ptr(), Up,
+                          tau.data_ptr<float>(), isd.data_ptr<float>(), d_den.data_ptr<float>(),
+                          dtau.data_ptr<float>(), dsz.data_ptr<float>(), &g, status_p, st);
+  }
+  TORCH_CHECK(rc == 0, "srw_route_bwd: gate step failed with code ", rc);
+  // out [M, N] (=|+=) op(A) . op(B)^T, block width as in the other products of these shapes
+  auto mm = [&](const Tensor& A, bool a_mn, long long lda, const Tensor& B, long long ldb, int M, int N, int K,
+                Tensor& C, bool accumulate) {
+    const int e = dsb_gemm_bf16(A.data_ptr(), a_mn, lda, B.data_ptr(), 1, ldb, M, N, K, C.data_ptr(),
+                                C.stride(0), C.scalar_type() == torch::kBFloat16, accumulate, 1.f, nullptr,
+                                nullptr, N <= 128 ? 128 : 256, status_p, st);
+    TORCH_CHECK(e == 0, "srw_route_bwd: GEMM failed with code ", e);
+  };
+  mm(p, true, Up, dy, dy.stride(0), U, D, T, g_write, true);           // p^T dy
+  mm(dxr, true, Up, x, x.stride(0), U, D, T, g_read, true);            // dxr^T x
+  mm(ds, true, Up, h, h.stride(0), U, r, T, g_emb, true);              // ds^T h
+  mm(ds, false, Up, emb, emb.stride(0), T, r, U, dh32, false);         // ds . emb
+  if (!want_dx) return c10::nullopt;
+  if (dx32.has_value() && dx32->defined()) {
+    TORCH_CHECK(mat(*dx32, T, D));
+    mm(dxr, false, Up, read, read.stride(0), T, D, U, *dx32, true);    // dxr . read
+    return dx32;
+  }
+  auto dx = torch::empty({T, D}, o16);
+  mm(dxr, false, Up, read, read.stride(0), T, D, U, dx, false);
+  return dx;
 }
 
 // -> dy bf16 [T, D], d_den [T]; dtau [T] is zeroed, d_scale (optional) accumulated
@@ -1116,6 +1189,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("srw_route_fwd", &srw_route_fwd);
   m.def("route_bwd_rows", &route_bwd_rows);
   m.def("srw_stats_bwd", &srw_stats_bwd);
+  m.def("srw_route_bwd", &srw_route_bwd);
   m.def("srw_rows", &srw_rows);
   m.def("gemv_rows", &gemv_rows);
   m.def("dropout", &dropout);

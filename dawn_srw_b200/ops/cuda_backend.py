@@ -523,36 +523,10 @@ def _route_backward_gemms(x_bf, h_bf, tau, inv_sd, dy, d_den, dtau, hd, spec, U,
     """Gate step and GEMMs of one route's backward: adds into the zeroed ``dtau`` [T] and the
     pool's gradient buffers, fills ``dh32`` [T, r] = ds . emb; returns dx (bf16, or fp32 added
     into ``dx32``)."""
-    e = ext()
-    dev = x_bf.device
-    T = x_bf.shape[0]
-    Up = _round_up(U, 8)
-    emb, read, write = hd.emb[:U], hd.read[:U], hd.write[:U]
-    if xr is not None:
-        p = xr
-        dxr = torch.empty_like(p)
-        ds = torch.empty_like(p)
-        count_launches(1)
-        e.srw_bwd_gate_xr(h_bf, emb, dy, write, xr, p, dxr, ds, tau, inv_sd, d_den, None, dtau,
-                          _gate_list(spec), status_word(dev), *NO_GATHER)
-    else:
-        p = torch.empty(T, Up, dtype=torch.bfloat16, device=dev)
-        dxr = torch.empty_like(p)
-        ds = torch.empty_like(p)
-        count_launches(2)
-        # the sigma sum is derived from dh32 and dtau: the kernel's own output for it is unused
-        e.srw_bwd_gate(h_bf, emb, x_bf, read, dy, write, p, dxr, ds, tau, inv_sd, d_den, dtau,
-                       torch.empty_like(dtau), _gate_list(spec), status_word(dev))
-    pv, dxrv, dsv = p[:, :U], dxr[:, :U], ds[:, :U]
-    gemm(pv, True, dy, True, out=hd.g_write[:U], accumulate=True)       # p^T dy
-    gemm(dxrv, True, x_bf, True, out=hd.g_read[:U], accumulate=True)    # dxr^T x
-    gemm(dsv, True, h_bf, True, out=hd.g_emb[:U], accumulate=True)      # ds^T h
-    gemm(dsv, False, emb, True, out=dh32)                               # ds . emb
-    if not want_dx:
-        return None
-    if dx32 is not None:
-        return gemm(dxrv, False, read, True, out=dx32, accumulate=True)  # dxr . read
-    return gemm(dxrv, False, read, True, out_dtype=torch.bfloat16)
+    count_launches(6 if xr is not None else 7)
+    return ext().srw_route_bwd(x_bf, h_bf, tau, inv_sd, dy, d_den, dtau, hd.emb[:U], hd.read[:U],
+                               hd.write[:U], hd.g_emb[:U], hd.g_read[:U], hd.g_write[:U], xr, dh32,
+                               want_dx, dx32, _gate_list(spec), status_word(x_bf.device))
 
 
 class _SRWRouteFn(torch.autograd.Function):
@@ -933,11 +907,13 @@ class CudaBackend:
 
     @torch.no_grad()
     def _cat_weights(self, layers):
-        key = tuple((l.weight.data_ptr(), l.weight._version,
-                     0 if l.bias is None else l.bias._version) for l in layers)
+        # the parameters themselves (weakly), their storage and versions: an id alone may be reused
+        ps = [q for l in layers for q in (l.weight, l.bias) if q is not None]
+        key = tuple((q.data_ptr(), q._version) for q in ps)
         cache = self.__dict__.setdefault("_cat_cache", {})
         hit = cache.get(id(layers[0]))
-        if hit is None or hit[0] != key:
+        if hit is None or hit[0] != key or any(r() is not q for r, q in zip(hit[4], ps)):
+            import weakref
             ws, bs, cuts, n0 = [], [], [], 0
             for l in layers:
                 n = l.weight.shape[0]
@@ -949,9 +925,9 @@ class CudaBackend:
             pad = _round_up(n0, 8) - n0
             w = F.pad(torch.cat(ws, 0), (0, 0, 0, pad)).to(torch.bfloat16).contiguous()
             b = F.pad(torch.cat(bs, 0), (0, pad)).contiguous()
-            hit = (key, w, b, cuts)
+            hit = (key, w, b, cuts, [weakref.ref(q) for q in ps])
             cache[id(layers[0])] = hit
-        return hit[1:]
+        return hit[1:4]
 
     def router(self, x, proj, tau, p, training, h_cuts, tau_cuts):
         """Router projection (cut into ``h_cuts`` columns, under dropout ``p`` in training) and
