@@ -987,16 +987,50 @@ __global__ void __launch_bounds__(256) adamw_multi_kernel(const __grid_constant_
   float* __restrict__ m = t.m[ti] + off;
   float* __restrict__ v = t.v[ti] + off;
   const float cs = *clip_scale;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
-    const float gi = g[i] * cs;
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float pi = p[i];
+  auto update = [&](float& pi, float gi, float& mi, float& vi) {
+    gi *= cs;
+    mi = b1 * mi + (1.f - b1) * gi;
+    vi = b2 * vi + (1.f - b2) * gi * gi;
     const float upd = (mi / bc1) / (sqrtf(vi / bc2) + eps) + wd * pi;
-    p[i] = pi - lr * upd;
+    pi = pi - lr * upd;
+  };
+  // Seven fp32 streams and nothing else to wait for: float4, two in flight per stream.  A step of the
+  // 40M model's parameters takes 0.19 ms (0.64 with one float at a time), of the 400M model's 1.80 (2.79).
+  long long i0 = 0;
+  if (((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(m) |
+        reinterpret_cast<uintptr_t>(v)) & 15) == 0) {
+    const long long n4 = n >> 2;
+    float4* p4 = reinterpret_cast<float4*>(p);
+    const float4* g4 = reinterpret_cast<const float4*>(g);
+    float4* m4 = reinterpret_cast<float4*>(m);
+    float4* v4 = reinterpret_cast<float4*>(v);
+    for (long long i = threadIdx.x; i < n4; i += 512) {
+      float4 pq[2], gq[2], mq[2], vq[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (i + 256 * k < n4) {
+          pq[k] = p4[i + 256 * k];
+          gq[k] = __ldcs(g4 + i + 256 * k);
+          mq[k] = m4[i + 256 * k];
+          vq[k] = v4[i + 256 * k];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (i + 256 * k < n4) {
+          update(pq[k].x, gq[k].x, mq[k].x, vq[k].x);
+          update(pq[k].y, gq[k].y, mq[k].y, vq[k].y);
+          update(pq[k].z, gq[k].z, mq[k].z, vq[k].z);
+          update(pq[k].w, gq[k].w, mq[k].w, vq[k].w);
+          p4[i + 256 * k] = pq[k];
+          m4[i + 256 * k] = mq[k];
+          v4[i + 256 * k] = vq[k];
+        }
+      }
+    }
+    i0 = n4 << 2;
   }
+  for (long long i = i0 + threadIdx.x; i < n; i += blockDim.x) update(p[i], g[i], m[i], v[i]);
 }
 
 __global__ void __launch_bounds__(256) sqnorm_multi_kernel(const __grid_constant__ MultiTable t,
@@ -1006,7 +1040,18 @@ __global__ void __launch_bounds__(256) sqnorm_multi_kernel(const __grid_constant
   const long long n = min(kMultiChunk, t.n[ti] - off);
   const float* __restrict__ g = t.g[ti] + off;
   float s = 0.f;
-  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
+  long long i0 = 0;
+  if ((reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+    const long long n4 = n >> 2;
+    const float4* g4 = reinterpret_cast<const float4*>(g);
+#pragma unroll 4
+    for (long long i = threadIdx.x; i < n4; i += 256) {
+      const float4 x = g4[i];
+      s = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, s))));
+    }
+    i0 = n4 << 2;
+  }
+  for (long long i = i0 + threadIdx.x; i < n; i += blockDim.x) {
     const float x = g[i];
     s = fmaf(x, x, s);
   }

@@ -1050,3 +1050,27 @@ def test_decode_attention_with_scores_of_minus_infinity(cb):
     out = cb.CudaBackend().decode_attention(q, k, v, ck, cv, torch.tensor([n], device=dev), H)
     ref = R.cached_attention(q.view(B, H, 1, dh), ck, cv, n + 1).reshape(B, H * dh)
     assert bool(ref.isfinite().all()) and _rel(out, ref) < 1e-5
+
+
+@pytest.mark.parametrize("sizes", [(1, 3, 4, 7), (1023, 1024, 1030), (65536, 65537, 200003)])
+def test_multi_tensor_optimizer_over_sizes_and_alignments(cb, sizes):
+    """Remainders of four, chunk edges, and tensors that start 4 bytes off a 16-byte boundary (the
+    scalar form); one fp32 update, so 1e-6, and an fp32 sum of squares, so 1e-5."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(len(sizes))
+    mk = lambda n, off: torch.randn(n + off, device=dev, generator=g)[off:]
+    ts = [[mk(n, k % 2) for k, n in enumerate(sizes)] for _ in range(4)]
+    p, gr, m, v = ts[0], ts[1], ts[2], [t.abs() for t in ts[3]]
+    v = [mk(t.numel(), k % 2).abs_() for k, t in enumerate(v)]
+    old = [[t.double().clone() for t in lst] for lst in (p, gr, m, v)]
+    cs = torch.full((1,), 0.37, device=dev)
+    total = cb.ext().grad_sq_norm(gr)
+    cb.ext().adamw_multi(p, gr, m, v, cs, 1e-2, 0.9, 0.95, 1e-8, 0.1, 0.5, 0.3)
+    assert _rel(total.reshape(()), sum((t * t).sum() for t in old[1])) < 1e-5
+    for k in range(len(sizes)):
+        po, go, mo, vo = (o[k] for o in old)
+        go = go * 0.37
+        mo, vo = 0.9 * mo + 0.1 * go, 0.95 * vo + 0.05 * go * go
+        po = po - 1e-2 * ((mo / 0.5) / ((vo / 0.3).sqrt() + 1e-8) + 0.1 * po)
+        for a, b in ((p[k], po), (m[k], mo), (v[k], vo)):
+            assert _rel(a, b) < 1e-6
