@@ -15,8 +15,9 @@
 // blocks write partial outputs, and a second kernel adds those and applies scale / max(sum den, 1);
 // adding them up with global reductions would save that launch, but a decoded token would no longer
 // repeat bit by bit.  One row, 28 % of the units
-// active: 100 000 units of 256 + 2 x 1280 and 10 400 of them in 35.5 us on average, 43.6 before (with
-// the kernel that added the blocks' partials); 25 200 and 2 600 units of 128 + 2 x 384 in 11.3, 15.9.
+// active: 100 000 units of 256 + 2 x 1280 and 10 400 of them in 31.2 us on average (39.2 for a warp per
+// unit), 25 200 and 2 600 units of 128 + 2 x 384 in 8.8 (11.6); about half of the issue slots are used,
+// a third of them for the loads' latency.
 // The reference runs the generic chunked kernels for decoding
 // (models/dawn_spatial_v41_exp.py:1713-1739, 1913-1957).
 #include <cuda_bf16.h>
@@ -86,8 +87,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
   constexpr int kScoreUnroll = NR * EC == 1 ? 8 : 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* s_acc = reinterpret_cast<float*>(smem_raw);                                // [warps][NR][D]
-  __nv_bfloat16* s_x = reinterpret_cast<__nv_bfloat16*>(s_acc + kRowWarps * NR * p.D);   // [NR][D]
-  __nv_bfloat16* s_h = s_x + NR * p.D;                                              // [NR][r]
+  float* s_x = s_acc + kRowWarps * NR * p.D;                                        // [NR][D]
+  __nv_bfloat16* s_h = reinterpret_cast<__nv_bfloat16*>(s_x + NR * p.D);                                            // [NR][r]
   float* s_g = reinterpret_cast<float*>(s_h + NR * p.r);                            // [kListUnits][NR]
   int* s_u = reinterpret_cast<int*>(s_g + kListUnits * NR);                         // [kListUnits] active units
   __shared__ float s_den[kRowWarps][NR];
@@ -99,8 +100,13 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
   for (int t = 0; t < NR; ++t) {
     const uint4* xs = reinterpret_cast<const uint4*>(p.x) + static_cast<size_t>(t % p.x_rows) * d_chunks;
     const uint4* hs = reinterpret_cast<const uint4*>(p.h) + static_cast<size_t>(t) * r_chunks;
-    for (int c = tid; c < d_chunks; c += kRowWarps * 32)
-      reinterpret_cast<uint4*>(s_x)[t * d_chunks + c] = t < p.N ? xs[c] : none;
+    for (int c = tid; c < d_chunks; c += kRowWarps * 32) {
+      float f[8];                                        // fp32: the row is used once per active unit
+      unpack8(t < p.N ? xs[c] : none, f);
+      float4* dst = reinterpret_cast<float4*>(s_x + t * p.D + 8 * c);
+      dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+      dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+    }
     for (int c = tid; c < r_chunks; c += kRowWarps * 32)
       reinterpret_cast<uint4*>(s_h)[t * r_chunks + c] = t < p.N ? hs[c] : none;
   }
@@ -160,17 +166,27 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
         }
       }
 #pragma unroll
-      for (int i = 0; i < kScoreUnroll; ++i) {
-        const int u = u0 + i * groups + grp;
+      for (int i = 0; i < kScoreUnroll; ++i)
 #pragma unroll
         for (int t = 0; t < NR; ++t)
           for (int o = lpu >> 1; o > 0; o >>= 1) s[i][t] += __shfl_xor_sync(0xffffffffu, s[i][t], o);
-        if (sub == 0 && u < end) {
+      // every lane of a group holds the group's sums: lane `sub` evaluates the gate of unit `sub`
+      // (of units sub, sub + lpu, .. in groups of fewer lanes), not the first lane that of all
+      for (int i0 = 0; i0 < kScoreUnroll; i0 += lpu) {
+        const int i = i0 + sub, u = u0 + i * groups + grp;
+        float st[NR];
+#pragma unroll
+        for (int t = 0; t < NR; ++t) {
+          st[t] = s[0][t];
+#pragma unroll
+          for (int k = 1; k < kScoreUnroll; ++k) st[t] = i == k ? s[k][t] : st[t];
+        }
+        if (i < kScoreUnroll && u < end) {
           const float um = p.unit_mask != nullptr ? p.unit_mask[u] : 1.f;
 #pragma unroll
           for (int t = 0; t < NR; ++t) {
             float g, dt;
-            gate_fwd_shifted<KIND>(p.gc, fmaf(s[i][t], rg[t].a, rg[t].b), g, dt);
+            gate_fwd_shifted<KIND>(p.gc, fmaf(st[t], rg[t].a, rg[t].b), g, dt);
             if (t < p.N) den[t] = fmaf(dt, um, den[t]);
             s_g[(u - base) * NR + t] = t < p.N ? g * um : 0.f;
           }
@@ -236,8 +252,9 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
           unpack8(rq[k], rv);
 #pragma unroll
           for (int t = 0; t < NR; ++t) {
-            float xv[8];
-            unpack8(*reinterpret_cast<const uint4*>(s_x + t * p.D + 8 * c), xv);
+            const float4 a = *reinterpret_cast<const float4*>(s_x + t * p.D + 8 * c);
+            const float4 b = *reinterpret_cast<const float4*>(s_x + t * p.D + 8 * c + 4);
+            const float xv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int j = 0; j < 8; ++j) xr[t] = fmaf(rv[j], xv[j], xr[t]);
           }
@@ -649,7 +666,7 @@ int launch_kv(const KvParams& p, int B, cudaStream_t stream) {
 
 template <int KIND, int NR, int KC, int EC>
 int launch_rows(const RowsParams& p, int blocks, cudaStream_t stream) {
-  const size_t smem = static_cast<size_t>(NR) * (p.D + p.r) * 2 +
+  const size_t smem = static_cast<size_t>(NR) * (p.D * 4 + p.r * 2) +
                       static_cast<size_t>(kRowWarps) * NR * p.D * 4 + static_cast<size_t>(kListUnits) * (NR + 1) * 4;
   static bool attr_set = false;
   if (!attr_set) {
