@@ -155,12 +155,12 @@ def load_full_state_dict(model: nn.Module, sd: Dict[str, torch.Tensor], strict: 
         src = sd[name]
         rows = getattr(dst, "_fsdp_rows", None)
         if rows is None:
-            dst.data.copy_(src)
+            dst.copy_(src)                # not through .data: the kept bf16 copies follow the version
             continue
         group = dst._fsdp_group
         per, rank = dst.shape[0], group_rank(group)
         lo, hi = rank * per, min(rows, (rank + 1) * per)
-        dst.data.zero_()
+        dst.zero_()
         if hi > lo:
-            dst.data[: hi - lo].copy_(src[lo:hi])
+            dst[: hi - lo].copy_(src[lo:hi])
     return missing, unexpected

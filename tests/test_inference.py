@@ -138,3 +138,19 @@ def test_prepared_pools_are_cached_until_a_parameter_changes():
     with torch.no_grad():
         ref = m(ids, want_diag=False)["logits"]
     assert torch.allclose(c, ref, atol=1e-4)
+
+
+def test_loading_a_state_dict_moves_the_version_of_every_parameter(monkeypatch):
+    """bf16 copies of weights are refreshed when the version counter of a parameter has moved."""
+    from dawn_srw_b200.ops import cuda_backend as cb
+    from dawn_srw_b200.parallel.fsdp import load_full_state_dict
+    monkeypatch.setattr(cb, "ext", lambda: None)
+    be, lin, other = cb.CudaBackend(), torch.nn.Linear(16, 8), torch.nn.Linear(16, 8)
+    be._w(lin.weight)
+    load_full_state_dict(lin, other.state_dict())
+    assert torch.equal(be._w(lin.weight), other.weight.detach().bfloat16())
+    lin.weight._fsdp_rows, lin.weight._fsdp_group = 5, None
+    short = {"weight": torch.randn(5, 16), "bias": other.bias.detach()}
+    load_full_state_dict(lin, short)
+    assert torch.equal(be._w(lin.weight)[:5], short["weight"].bfloat16())
+    assert float(be._w(lin.weight)[5:].abs().max()) == 0.0
