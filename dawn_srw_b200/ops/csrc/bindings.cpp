@@ -953,6 +953,20 @@ Tensor dropout_rows(const Tensor& x, int64_t seed, double p) {
   return y;
 }
 
+// -> bf16 [n, D] of w1's and w2's rows and fp32 [n] of both biases, n = n1 + n2 rounded up to 8
+std::vector<Tensor> router_operand(const Tensor& w1, const Tensor& b1, const Tensor& w2, const Tensor& b2) {
+  auto ok = [](const Tensor& t, int dim) { return f32(t) && t.is_contiguous() && t.dim() == dim; };
+  TORCH_CHECK(ok(w1, 2) && ok(w2, 2) && ok(b1, 1) && ok(b2, 1) && w1.size(1) == w2.size(1) &&
+              b1.size(0) == w1.size(0) && b2.size(0) == w2.size(0), "router_operand: bad parameters");
+  const c10::cuda::CUDAGuard guard(w1.device());
+  const int64_t n1 = w1.size(0), n2 = w2.size(0), n = (n1 + n2 + 7) / 8 * 8, D = w1.size(1);
+  auto w = torch::empty({n, D}, w1.options().dtype(torch::kBFloat16)), b = torch::empty({n}, w1.options());
+  int rc = dsb_router_operand(w1.data_ptr<float>(), b1.data_ptr<float>(), w2.data_ptr<float>(),
+                              b2.data_ptr<float>(), n1, n2, n, D, w.data_ptr(), b.data_ptr<float>(), cur_stream());
+  TORCH_CHECK(rc == 0, "dsb_router_operand failed with code ", rc);
+  return {w, b};
+}
+
 // sources fp32 [T, cols_i] at columns cols0[i] -> bf16 [T, n] and, if wanted, its column sums [n]
 std::vector<Tensor> linear_pack(std::vector<Tensor> srcs, std::vector<int64_t> cols0, int64_t T, int64_t n,
                                 bool want_sum, int64_t seed, double p, int64_t n_drop) {
@@ -1195,6 +1209,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("dropout", &dropout);
   m.def("dropout_rows", &dropout_rows);
   m.def("linear_pack", &linear_pack);
+  m.def("router_operand", &router_operand);
   m.def("kv_decode_attention", &kv_decode_attention);
   m.def("srw_rows_max", [](int64_t D) { return dsb_srw_rows_max(static_cast<int>(D)); });
   m.def("srw_fwd_gate_gather", &srw_fwd_gate_gather);

@@ -73,6 +73,10 @@ struct DsbPackSrc {
 };
 int dsb_linear_pack(const struct DsbPackSrc* src, int n_src, int T, int n, void* dst_bf16, float* colsum,
                     unsigned long long seed, float p, int n_drop, cudaStream_t stream);
+// Operand of a router GEMM: w bf16 [n, D] = rows of w1 [n1, D], of w2 [n2, D], zeros; b [n] likewise
+// (all fp32 contiguous, n >= n1 + n2).
+int dsb_router_operand(const float* w1, const float* b1, const float* w2, const float* b2, int n1, int n2,
+                       int n, int D, void* w_bf16, float* b, cudaStream_t stream);
 // y [T, n] = dropout(x [T, ldx]) with the mask of the contiguous tensor; n, ldx % 4 == 0.
 int dsb_dropout_rows(const float* x, long long ldx, float* y, int T, int n, unsigned long long seed, float p,
                      cudaStream_t stream);

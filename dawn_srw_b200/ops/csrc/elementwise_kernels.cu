@@ -901,6 +901,52 @@ extern "C" int dsb_dropout_rows(const float* x, long long ldx, float* y, int T, 
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
+// ------------------------------------------------------- operand of a router GEMM
+// w [n, D] bf16 = bf16 of w1's n1 rows, then w2's n2, then zeros; b [n] = b1, b2, zeros.  Bound by its
+// bytes (6 per element: 5.1 us for the 1152 + 3 rows of 2048 of the largest model, 1.6 for 384 + 3 of 384): made anew in
+// every call, so that a kept copy need not be told of every way to write to a parameter.
+namespace {
+template <bool kVec>
+__global__ void __launch_bounds__(256) router_operand_kernel(const float* __restrict__ w1,
+                                                             const float* __restrict__ b1,
+                                                             const float* __restrict__ w2,
+                                                             const float* __restrict__ b2, int n1, int n2,
+                                                             int n, int D, __nv_bfloat16* __restrict__ w,
+                                                             float* __restrict__ b) {
+  const long long first = static_cast<long long>(blockIdx.x) * 256 + threadIdx.x;
+  const long long stride = static_cast<long long>(gridDim.x) * 256;
+  const long long l1 = static_cast<long long>(n1) * D, l2 = l1 + static_cast<long long>(n2) * D;
+  const long long total = static_cast<long long>(n) * D;
+  for (long long i = first; i < n; i += stride) b[i] = i < n1 ? b1[i] : i < n1 + n2 ? b2[i - n1] : 0.f;
+  if constexpr (kVec) {                                  // D % 4 == 0: a chunk lies in one row
+    for (long long i = 4 * first; i < total; i += 4 * stride) {
+      const float4 v = i < l1   ? *reinterpret_cast<const float4*>(w1 + i)
+                       : i < l2 ? *reinterpret_cast<const float4*>(w2 + (i - l1))
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+      *reinterpret_cast<uint2*>(w + i) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  } else {
+    for (long long i = first; i < total; i += stride)
+      w[i] = __float2bfloat16(i < l1 ? w1[i] : i < l2 ? w2[i - l1] : 0.f);
+  }
+}
+}  // namespace
+
+extern "C" int dsb_router_operand(const float* w1, const float* b1, const float* w2, const float* b2, int n1,
+                                  int n2, int n, int D, void* w_bf16, float* b, cudaStream_t stream) {
+  if (n1 < 0 || n2 < 0 || n < n1 + n2 || D < 0) return 2;
+  if (n == 0) return 0;
+  __nv_bfloat16* w = static_cast<__nv_bfloat16*>(w_bf16);
+  const long long total = static_cast<long long>(n) * D;
+  if ((D & 3) == 0 && aligned16(w1, w2, w_bf16, nullptr))
+    router_operand_kernel<true><<<grid_for(total / 4 + n, 256, 148 * 8), 256, 0, stream>>>(w1, b1, w2, b2, n1, n2, n, D, w, b);
+  else
+    router_operand_kernel<false><<<grid_for(total + n, 256, 148 * 8), 256, 0, stream>>>(w1, b1, w2, b2, n1, n2, n, D, w, b);
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+
 // Prompt of a cached generation: q, k, v fp32 [B * S, H * dh] -> bf16 operands of the attention kernel
 // and, for k and v, their fp32 rows in the caches [B, H, s_max, dh] at positions 0..S-1.  Bound by its
 // bytes (12 read, 14 written per position and column) from a few thousand positions on, by being one

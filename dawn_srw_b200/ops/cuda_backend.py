@@ -245,16 +245,20 @@ class _LinearFn(torch.autograd.Function):
 
 class _RouterFn(torch.autograd.Function):
     """Router projection and threshold head on the same input as ONE GEMM over their concatenated
-    (8-padded) weights, dropout on the projection.  Returns the projection cut into ``h_cuts``
+    (8-padded) weights, dropout on the projection.  The bf16 operand and the bias are made from the
+    parameters in every call (one launch): nothing is kept, so no write to a parameter can be missed.
+    Returns the projection cut into ``h_cuts``
     columns, the thresholds cut into ``tau_cuts`` (none if that is a single piece) and all
     thresholds: views of one buffer, so that neither direction slices, pads or concatenates; the
     backward pass packs all cotangents into one bf16 operand (one kernel, with the dropout mask
     and the bias gradients)."""
 
     @staticmethod
-    def forward(ctx, x, w1, b1, w2, b2, w_cat, b_cat, h_cuts, tau_cuts, p):
+    def forward(ctx, x, w1, b1, w2, b2, h_cuts, tau_cuts, p):
         xb = _bf16_2d(x)
         n1, n2 = w1.shape[0], w2.shape[0]
+        w_cat, b_cat = ext().router_operand(*(t.detach().float().contiguous() for t in (w1, b1, w2, b2)))
+        count_launches(1)
         y = gemm(xb, False, w_cat, False, out_dtype=torch.float32, bias=b_cat)
         h, seed = y[:, :n1], 0
         if p > 0.0:
@@ -284,12 +288,12 @@ class _RouterFn(torch.autograd.Function):
         srcs = [(g.float(), c) for g, c in zip(grads, ctx.cols) if g is not None]
         srcs = [(g if g.stride(1) == 1 else g.contiguous(), c) for g, c in srcs]
         if not srcs:
-            return (None,) * 10
+            return (None,) * 8
         dyb, db = ext().linear_pack([g for g, _ in srcs], [c for _, c in srcs], T, n, True, seed, p, n1)
         count_launches(1)
         dx = gemm(dyb, False, w_cat, True, out_dtype=x_dtype) if ctx.needs_input_grad[0] else None
         dw = gemm(dyb, True, xb, True, out_dtype=torch.float32)
-        return (dx, dw[:n1], db[:n1], dw[n1:n1 + n2], db[n1:n1 + n2], None, None, None, None, None)
+        return (dx, dw[:n1], db[:n1], dw[n1:n1 + n2], db[n1:n1 + n2], None, None, None)
 
 
 class _DropoutFn(torch.autograd.Function):
@@ -932,8 +936,7 @@ class CudaBackend:
     def router(self, x, proj, tau, p, training, h_cuts, tau_cuts):
         """Router projection (cut into ``h_cuts`` columns, under dropout ``p`` in training) and
         thresholds (cut into ``tau_cuts``) of x: (pieces of h, pieces of tau, all of tau)."""
-        w, b, _ = self._cat_weights((proj, tau))
-        outs = _RouterFn.apply(x, proj.weight, proj.bias, tau.weight, tau.bias, w, b, tuple(h_cuts),
+        outs = _RouterFn.apply(x, proj.weight, proj.bias, tau.weight, tau.bias, tuple(h_cuts),
                                tuple(tau_cuts) if len(tau_cuts) > 1 else (), float(p) if training else 0.0)
         k = len(h_cuts)
         return outs[:k], (outs[k:-1] if len(tau_cuts) > 1 else outs[-1:]), outs[-1]

@@ -1074,3 +1074,35 @@ def test_multi_tensor_optimizer_over_sizes_and_alignments(cb, sizes):
         po = po - 1e-2 * ((mo / 0.5) / ((vo / 0.3).sqrt() + 1e-8) + 0.1 * po)
         for a, b in ((p[k], po), (m[k], mo), (v[k], vo)):
             assert _rel(a, b) < 1e-6
+
+
+@pytest.mark.parametrize("D,n1,n2", [(64, 24, 3), (128, 128, 1), (2048, 1152, 3)])
+def test_router_sees_every_write_to_its_parameters(cb, D, n1, n2):
+    """Writes through .data move no version counter; the next call has to use them all the same.
+    Against fp64 of the parameters as they are: bf16 operands, 1e-2."""
+    dev = torch.device("cuda")
+    torch.manual_seed(D)
+    be, x = cb.CudaBackend(), torch.randn(70, D, device=dev)
+    proj, tau = torch.nn.Linear(D, n1).to(dev), torch.nn.Linear(D, n2).to(dev)
+    for q in (None, tau.bias, proj.bias, tau.weight, proj.weight):
+        if q is not None:
+            q.data.copy_(torch.randn_like(q))
+        (h,), _, t = be.router(x, proj, tau, 0.0, False, (n1,), (n2,))
+        for got, l in ((h, proj), (t, tau)):
+            want = torch.nn.functional.linear(x.double(), l.weight.double(), l.bias.double())
+            assert _rel(got, want) < 1e-2
+    cb.check_status()
+
+
+@pytest.mark.parametrize("n1,n2,D", [(8, 1, 4), (24, 3, 130), (768, 3, 1280), (5, 3, 64)])
+def test_router_operand_rows(cb, n1, n2, D):
+    dev = torch.device("cuda")
+    w1, w2 = torch.randn(n1, D, device=dev), torch.randn(n2 * D + 1, device=dev)[1:].view(n2, D)   # 4 bytes off
+    b1, b2 = torch.randn(n1, device=dev), torch.randn(n2, device=dev)
+    for second in (w2, w2.clone()):
+        w, b = cb.ext().router_operand(w1, b1, second, b2)
+        n = (n1 + n2 + 7) // 8 * 8
+        want = torch.zeros(n, D, device=dev)
+        want[:n1], want[n1:n1 + n2] = w1, w2
+        assert torch.equal(w, want.bfloat16())
+        assert torch.equal(b, torch.nn.functional.pad(torch.cat([b1, b2]), (0, n - n1 - n2)))
