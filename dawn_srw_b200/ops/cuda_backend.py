@@ -875,6 +875,13 @@ class CudaBackend:
         self.fused_comm = fused_comm     # in-kernel all-gather / reduce-scatter when sharded
         self._comm = {}
 
+    def __getstate__(self):
+        """Settings only: kept weight copies (keyed by object identity and held by weak references)
+        and communication buffers belong to this process, a copy makes its own."""
+        state = dict(self.__dict__, _wcache={}, _comm={})
+        state.pop("_cat_cache", None)
+        return state
+
     # ---- dense ops -----------------------------------------------------
     def _w(self, w):
         """bf16 compute copy of a master weight, refreshed when the weight changes."""

@@ -154,3 +154,22 @@ def test_loading_a_state_dict_moves_the_version_of_every_parameter(monkeypatch):
     load_full_state_dict(lin, short)
     assert torch.equal(be._w(lin.weight)[:5], short["weight"].bfloat16())
     assert float(be._w(lin.weight)[5:].abs().max()) == 0.0
+
+
+def test_a_backend_that_has_run_can_be_copied_and_pickled(monkeypatch):
+    """The weight copies a backend keeps (here: of two concatenated layers) do not travel with it, and
+    the copy makes its own from the layers that it is given."""
+    import copy
+    import pickle
+
+    from dawn_srw_b200.ops import cuda_backend as cb
+    monkeypatch.setattr(cb, "ext", lambda: None)
+    be = cb.CudaBackend(diag_chunk=77, keep_xr=False)
+    layers = (torch.nn.Linear(16, 24), torch.nn.Linear(16, 3))
+    w, b, cuts = be._cat_weights(layers)
+    be._w(layers[0].weight)
+    assert w.shape == (32, 16) and be._cat_weights(layers)[0] is w
+    for other in (pickle.loads(pickle.dumps(be)), copy.deepcopy(be)):
+        assert (other.diag_chunk, other.keep_xr) == (77, False) and not other._wcache
+        assert torch.equal(other._cat_weights(layers)[0], w) and other._cat_weights(layers)[0] is not w
+    assert be._cat_weights(layers)[0] is w
