@@ -974,8 +974,9 @@ std::vector<Tensor> linear_pack(std::vector<Tensor> srcs, std::vector<int64_t> c
   DsbPackSrc s[5];
   for (size_t i = 0; i < srcs.size(); ++i) {
     const Tensor& t = srcs[i];
-    TORCH_CHECK(f32(t) && t.dim() == 2 && t.stride(1) == 1 && t.size(0) == T && cols0[i] >= 0 &&
-                cols0[i] + t.size(1) <= n, "linear_pack: bad source");
+    // (a single column may have any inner stride: [T, 1] with strides (1, T) counts as contiguous)
+    TORCH_CHECK(f32(t) && t.dim() == 2 && (t.stride(1) == 1 || t.size(1) == 1) && t.size(0) == T &&
+                cols0[i] >= 0 && cols0[i] + t.size(1) <= n, "linear_pack: bad source");
     s[i] = {t.data_ptr<float>(), t.stride(0), static_cast<int>(cols0[i]), static_cast<int>(t.size(1)), 0};
   }
   const c10::cuda::CUDAGuard guard(srcs[0].device());

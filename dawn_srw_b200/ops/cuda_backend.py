@@ -257,6 +257,8 @@ class _RouterFn(torch.autograd.Function):
     def forward(ctx, x, w1, b1, w2, b2, h_cuts, tau_cuts, p):
         xb = _bf16_2d(x)
         n1, n2 = w1.shape[0], w2.shape[0]
+        ctx.biases = (b1 is not None, b2 is not None)
+        b1, b2 = (w.new_zeros(w.shape[0]) if b is None else b for w, b in ((w1, b1), (w2, b2)))
         w_cat, b_cat = ext().router_operand(*(t.detach().float().contiguous() for t in (w1, b1, w2, b2)))
         count_launches(1)
         y = gemm(xb, False, w_cat, False, out_dtype=torch.float32, bias=b_cat)
@@ -293,7 +295,8 @@ class _RouterFn(torch.autograd.Function):
         count_launches(1)
         dx = gemm(dyb, False, w_cat, True, out_dtype=x_dtype) if ctx.needs_input_grad[0] else None
         dw = gemm(dyb, True, xb, True, out_dtype=torch.float32)
-        return (dx, dw[:n1], db[:n1], dw[n1:n1 + n2], db[n1:n1 + n2], None, None, None)
+        db1, db2 = (d if has else None for d, has in zip((db[:n1], db[n1:n1 + n2]), ctx.biases))
+        return dx, dw[:n1], db1, dw[n1:n1 + n2], db2, None, None, None
 
 
 class _DropoutFn(torch.autograd.Function):

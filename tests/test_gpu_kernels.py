@@ -1106,3 +1106,26 @@ def test_router_operand_rows(cb, n1, n2, D):
         want[:n1], want[n1:n1 + n2] = w1, w2
         assert torch.equal(w, want.bfloat16())
         assert torch.equal(b, torch.nn.functional.pad(torch.cat([b1, b2]), (0, n - n1 - n2)))
+
+
+@pytest.mark.parametrize("n2", [1, 3])
+@pytest.mark.parametrize("bias", [True, False])
+def test_router_takes_transposed_uses_and_layers_without_bias(cb, n2, bias):
+    """A loss on the transposed thresholds gives a [T, 1] cotangent of strides (1, T), which counts as
+    contiguous; bf16 operands on both sides, so 1e-2 against the separate layers in fp64."""
+    dev = torch.device("cuda")
+    torch.manual_seed(n2)
+    be, T, D, n1 = cb.CudaBackend(), 69, 64, 24
+    proj, tau = (torch.nn.Linear(D, n, bias=bias).to(dev) for n in (n1, n2))
+    x = torch.randn(T, D, device=dev)
+    wt, wh = torch.randn(n2, T, device=dev), torch.randn(n1, T, device=dev)
+    xs = x.clone().requires_grad_(True)
+    (h,), _, t = be.router(xs, proj, tau, 0.0, True, (n1,), (n2,))
+    ((t.t() * wt).sum() + (h.t() * wh).sum()).backward()
+    cb.check_status()
+    want = [wt.t().double() @ tau.weight.double() + wh.t().double() @ proj.weight.double(),
+            wt.double() @ x.double(), wh.double() @ x.double()]
+    for a, b in zip((xs.grad, tau.weight.grad, proj.weight.grad), want):
+        assert _rel(a, b) < 1e-2
+    if bias:
+        assert _rel(tau.bias.grad, wt.sum(1)) < 1e-2 and _rel(proj.bias.grad, wh.sum(1)) < 1e-2
