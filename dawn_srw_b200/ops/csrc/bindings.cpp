@@ -44,6 +44,15 @@ DsbGate to_gate(const std::vector<double>& g) {
 
 bool f32(const Tensor& t) { return t.is_cuda() && t.scalar_type() == torch::kFloat32; }
 
+int block_width(int n) { return n <= 128 ? 128 : 256; }
+
+// Workspace of a split product of M x N from K (undefined where it is not cut).
+Tensor gemm_workspace(int64_t M, int64_t N, int64_t K, int64_t block_n, const Tensor& like) {
+  const int64_t n = dsb_gemm_workspace(M, N, K, block_n);
+  return n > 0 ? torch::empty({n}, like.options().dtype(torch::kFloat32)) : Tensor();
+}
+float* ptr(const Tensor& t) { return t.defined() ? t.data_ptr<float>() : nullptr; }
+
 // C (=|+=) alpha * row_scale * op(A) . op(B)^T + bias.
 //   a_mn == false: A is [M,K];  a_mn == true: A is stored [K,M]
 //   b_mn == false: B is [N,K];  b_mn == true: B is stored [K,N]
@@ -62,9 +71,12 @@ void gemm(const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, Tensor& C, boo
   const bool c_bf16 = C.scalar_type() == torch::kBFloat16;
   TORCH_CHECK(c_bf16 || C.scalar_type() == torch::kFloat32, "gemm: C must be bf16 or fp32");
   TORCH_CHECK(!(accumulate && c_bf16), "gemm: accumulate needs an fp32 C");
+  // a caller that accumulates gets reduce-adds in any order, any other a result that repeats
+  const bool ordered = !accumulate && !c_bf16 && opt_f32(bias) == nullptr;
+  auto ws = ordered ? gemm_workspace(M, N, K, block_n, A) : Tensor();
   int rc = dsb_gemm_bf16(A.data_ptr(), a_mn, A.stride(0), B.data_ptr(), b_mn, B.stride(0), M, N, K,
                          C.data_ptr(), C.stride(0), c_bf16, accumulate, alpha, opt_f32(row_scale),
-                         opt_f32(bias), block_n, status.data_ptr<int>(), cur_stream());
+                         opt_f32(bias), block_n, ptr(ws), status.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_gemm_bf16 failed with code ", rc);
 }
 
@@ -701,7 +713,7 @@ std::vector<Tensor> srw_stats(const Tensor& h, const Tensor& off, const Tensor& 
                           den.data_ptr<float>(), N, hsum.data_ptr<float>(), r, cur_stream());
   if (rc == 0)
     rc = dsb_gemm_bf16(hb.data_ptr(), 0, r, gcat.data_ptr(), 0, gcat.stride(0), N, 2 * r, r, hg.data_ptr(),
-                       2 * r, 0, 0, 1.f, nullptr, nullptr, 2 * r <= 128 ? 128 : 256,
+                       2 * r, 0, 0, 1.f, nullptr, nullptr, block_width(2 * r), nullptr,
                        status.data_ptr<int>(), cur_stream());
   if (rc == 0)
     rc = dsb_score_stats_fwd(hg.data_ptr<float>(), hg.data_ptr<float>() + r, 2 * r, hb.data_ptr(), r,
@@ -759,9 +771,10 @@ void srw_route_fwd(const Tensor& h, const Tensor& x, const Tensor& emb, const Te
                                nullptr, den.data_ptr<float>(), nullptr, diag_p, alive_p,
                                opt_f32(unit_mask), &g, nullptr, status.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_srw_fwd_gate_xr failed with code ", rc);
+  auto ws = accumulate ? Tensor() : gemm_workspace(T, D, U, block_width(D), y);
   rc = dsb_srw_write(p.data_ptr(), p.stride(0), write.data_ptr(), write.stride(0), T, U, D,
                      den.data_ptr<float>(), scale, sp, y.data_ptr<float>(), y.stride(0), accumulate,
-                     status.data_ptr<int>(), cur_stream());
+                     ptr(ws), status.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_srw_write failed with code ", rc);
 }
 
@@ -815,26 +828,28 @@ c10::optional<Tensor> srw_route_bwd(const Tensor& x, const Tensor& h, const Tens
                           dtau.data_ptr<float>(), dsz.data_ptr<float>(), &g, status_p, st);
   }
   TORCH_CHECK(rc == 0, "srw_route_bwd: gate step failed with code ", rc);
-  // out [M, N] (=|+=) op(A) . op(B)^T, block width as in the other products of these shapes
+  // out [M, N] (=|+=) op(A) . op(B)^T, block width as in the other products of these shapes; the pool's
+  // gradients are shared by all layers and may take their parts in any order, the rest repeats
   auto mm = [&](const Tensor& A, bool a_mn, long long lda, const Tensor& B, long long ldb, int M, int N, int K,
-                Tensor& C, bool accumulate) {
+                Tensor& C, bool accumulate, bool ordered) {
+    auto ws = ordered && C.scalar_type() == torch::kFloat32 ? gemm_workspace(M, N, K, block_width(N), C) : Tensor();
     const int e = dsb_gemm_bf16(A.data_ptr(), a_mn, lda, B.data_ptr(), 1, ldb, M, N, K, C.data_ptr(),
                                 C.stride(0), C.scalar_type() == torch::kBFloat16, accumulate, 1.f, nullptr,
-                                nullptr, N <= 128 ? 128 : 256, status_p, st);
+                                nullptr, block_width(N), ptr(ws), status_p, st);
     TORCH_CHECK(e == 0, "srw_route_bwd: GEMM failed with code ", e);
   };
-  mm(p, true, Up, dy, dy.stride(0), U, D, T, g_write, true);           // p^T dy
-  mm(dxr, true, Up, x, x.stride(0), U, D, T, g_read, true);            // dxr^T x
-  mm(ds, true, Up, h, h.stride(0), U, r, T, g_emb, true);              // ds^T h
-  mm(ds, false, Up, emb, emb.stride(0), T, r, U, dh32, false);         // ds . emb
+  mm(p, true, Up, dy, dy.stride(0), U, D, T, g_write, true, false);           // p^T dy
+  mm(dxr, true, Up, x, x.stride(0), U, D, T, g_read, true, false);            // dxr^T x
+  mm(ds, true, Up, h, h.stride(0), U, r, T, g_emb, true, false);              // ds^T h
+  mm(ds, false, Up, emb, emb.stride(0), T, r, U, dh32, false, true);         // ds . emb
   if (!want_dx) return c10::nullopt;
   if (dx32.has_value() && dx32->defined()) {
     TORCH_CHECK(mat(*dx32, T, D));
-    mm(dxr, false, Up, read, read.stride(0), T, D, U, *dx32, true);    // dxr . read
+    mm(dxr, false, Up, read, read.stride(0), T, D, U, *dx32, true, true);    // dxr . read
     return dx32;
   }
   auto dx = torch::empty({T, D}, o16);
-  mm(dxr, false, Up, read, read.stride(0), T, D, U, dx, false);
+  mm(dxr, false, Up, read, read.stride(0), T, D, U, dx, false, true);
   return dx;
 }
 
@@ -886,7 +901,7 @@ std::vector<Tensor> srw_stats_bwd(const Tensor& dtau, const Tensor& dh32, c10::o
   if (rc == 0 && g_gram.has_value() && g_gram->defined()) {
     TORCH_CHECK(ok(*g_gram, static_cast<int64_t>(r) * r));
     rc = dsb_gemm_bf16(w.data_ptr(), 1, r, hb.data_ptr(), 1, r, r, r, N, g_gram->data_ptr(), r, 0, 1, inv_u,
-                       nullptr, nullptr, r <= 128 ? 128 : 256, status.data_ptr<int>(), cur_stream());
+                       nullptr, nullptr, block_width(r), nullptr, status.data_ptr<int>(), cur_stream());
   }
   TORCH_CHECK(rc == 0, "srw_stats_bwd failed with code ", rc);
   return {dh, d_off};

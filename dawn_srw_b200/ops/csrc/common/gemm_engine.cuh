@@ -187,6 +187,7 @@ struct AccCtl {
   int lane;
   volatile int* abort_flag;
   bool ok;
+  int split;            // which of the K splits this tile is
 
   __device__ __forceinline__ static constexpr int col_off(int a) {
     int c = 0;
@@ -647,7 +648,7 @@ gemm_engine_kernel(const __grid_constant__ GemmParams<typename Epi::Params> p) {
       int mt, nt;
       tile_coords(p, t2, mt, nt);
       Ctl ctl{acc_full, acc_empty, tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16), it,
-              lane, abort_flag, true};
+              lane, abort_flag, true, tile / mn_tiles};
       Epi::template run<BN>(p.epi, p.tma_out, stager, ctl,
                             mt * kTileM + static_cast<int>(rank) * kBlockM, nt * BN, p.M, p.N, warp,
                             lane);

@@ -42,16 +42,21 @@ typedef struct DsbGather {
 //   B: b_mn == 0 -> stored [N][K];             b_mn == 1 -> stored [K][N]
 //   bf16 operands, fp32 accumulation; C is bf16 (c_is_bf16) or fp32.
 //   Leading dimensions must be multiples of 8 elements, bases 16-byte aligned.
+//   workspace: dsb_gemm_workspace floats, 16-byte aligned, or null.  With it a product of few output
+//   tiles and a long K (fp32, no bias) is cut in K and its parts are added up in order; without it
+//   it is cut only if it accumulates, and the parts arrive in any order.
+long long dsb_gemm_workspace(int M, int N, int K, int block_n);
 int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn, long long ldb,
                   int M, int N, int K, void* C, long long ldc, int c_is_bf16, int accumulate,
                   float alpha, const float* row_scale, const float* bias, int block_n,
-                  int* status, cudaStream_t stream);
+                  float* workspace, int* status, cudaStream_t stream);
 
 // Write GEMM of a route, normalised in its epilogue: y[T, D] (=|+=) (p[T, U] . write[U, D]) *
-// norm / max(den[t], 1), y fp32; norm_ptr (device scalar) overrides norm when not null.
+// norm / max(den[t], 1), y fp32; norm_ptr (device scalar) overrides norm when not null.  workspace:
+// as above, for (T, D, U).
 int dsb_srw_write(const void* p, long long ldp, const void* write, long long ldw, int T, int U, int D,
                   const float* den, float norm, const float* norm_ptr, float* y, long long ldy,
-                  int accumulate, int* status, cudaStream_t stream);
+                  int accumulate, float* workspace, int* status, cudaStream_t stream);
 
 // SRW forward gate kernel: p[T,U] = gate(h.emb^T; tau, 1/sigma) * (x.read^T),
 // den_sum[T] += sum_U den_term.  gate_sum / alive / unit_mask may be null.

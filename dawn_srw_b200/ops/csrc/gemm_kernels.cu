@@ -107,6 +107,8 @@ struct PlainEpi {
     const float* den;
     const float* norm_ptr;
     float norm;
+    // K splits that are added up later, in order: rows of a split's partial output (else 0).
+    int split_rows;
   };
   template <int BN, class Ctl>
   __device__ static void run(const Params& p, const CUtensorMap* maps, WarpStager& st, Ctl& ctl,
@@ -185,7 +187,7 @@ struct PlainEpi {
           st.flush(&maps[owner], buf, col0,
                    p.scatter_rank * p.scatter_rows + (r0 - owner * p.scatter_rows), false, true);
         } else {
-          st.flush(&maps[0], buf, col0, r0, p.accumulate != 0, true);
+          st.flush(&maps[0], buf, col0, r0 + ctl.split * p.split_rows, p.accumulate != 0, true);
         }
       }
     }
@@ -1621,10 +1623,71 @@ static int few_rows_gemm(const void* x, long long ldx, const void* w, int w_mn, 
 }
 }  // namespace dsb
 
+// out[m, n] (=|+=) f(m) * (ws[0][m][n] + ws[1][m][n] + ...) with f = alpha * row_scale[m] * norm /
+// max(den[m], 1), each factor where given: the parts of a split product, in order.  Bound by its bytes
+// (4 per part and element, mostly from L2) and by being a launch of its own.  With it, 384 x 384 from K = 8192 takes
+// 16.7 us (52.7 uncut), 512 x 384 from 25 200 22.2 (146.8).
+template <bool kVec>
+__global__ void __launch_bounds__(256) split_sum_kernel(const float* __restrict__ ws, long long part,
+                                                        int splits, int ldw, int M, int N,
+                                                        float* __restrict__ out, long long ldc, int accumulate,
+                                                        float alpha, const float* __restrict__ row_scale,
+                                                        const float* __restrict__ den,
+                                                        const float* __restrict__ norm_ptr, float norm) {
+  const int n4 = ldw >> 2;                                 // ldw: N rounded up to four
+  const long long total = static_cast<long long>(M) * n4;
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < total; i += gridDim.x * 256LL) {
+    const int m = static_cast<int>(i / n4), c = 4 * static_cast<int>(i - static_cast<long long>(m) * n4);
+    const float* src = ws + static_cast<long long>(m) * ldw + c;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = 0; s < splits; s += 8) {
+      float4 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        v[k] = s + k < splits ? *reinterpret_cast<const float4*>(src + (s + k) * part) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { a.x += v[k].x; a.y += v[k].y; a.z += v[k].z; a.w += v[k].w; }
+    }
+    float f = alpha * (row_scale != nullptr ? row_scale[m] : 1.f);
+    if (den != nullptr) {
+      const float d = den[m];
+      f *= (norm_ptr != nullptr ? *norm_ptr : norm) / (d < 1.f ? 1.f : d);             // a NaN stays one
+    }
+    a.x *= f; a.y *= f; a.z *= f; a.w *= f;
+    float* dst = out + static_cast<long long>(m) * ldc + c;
+    if (kVec && c + 4 <= N) {
+      float4* d4 = reinterpret_cast<float4*>(dst);
+      if (accumulate) { const float4 o = *d4; a.x += o.x; a.y += o.y; a.z += o.z; a.w += o.w; }
+      *d4 = a;
+    } else {
+      const float e[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c + k < N) dst[k] = accumulate ? dst[k] + e[k] : e[k];
+    }
+  }
+}
+
+// How an fp32 product without a bias is cut in K.  Few output tiles but a long K (weight gradients, the
+// write GEMM of a small batch) leave SM pairs idle, so K is cut until every pair has work.  Every
+// part writes or reduce-adds a whole output tile, so parts are long (32 K tiles; 16 where the tiles
+// would leave most of the chip idle, 8 for a few rows).  384 x 384 from K = 8192 is 4 tiles.
+struct SplitPlan { int splits, tile_m, m_tiles; };
+static SplitPlan plan_splits(int M, int N, int K, int block_n) {
+  const bool pairs = use_cta_pairs() && M > kBlockM;
+  const int BN = block_n == 128 ? 128 : 256, tm = pairs ? 2 * kBlockM : kBlockM;
+  const int m_tiles = (M + tm - 1) / tm, k_tiles = (K + kBlockK - 1) / kBlockK;
+  const long long tiles = static_cast<long long>(m_tiles) * ((N + BN - 1) / BN);
+  const int units = sm_count() / (pairs ? 2 : 1);
+  if (tiles >= 2 * units || k_tiles < 64) return {1, tm, m_tiles};
+  const int min_len = M <= tm ? 8 : 4 * tiles <= units ? 16 : 32;
+  return {choose_k_splits(tiles, units, k_tiles, k_tiles / min_len), tm, m_tiles};
+}
 static int gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn, long long ldb,
                      int M, int N, int K, void* C, long long ldc, int c_is_bf16, int accumulate,
                      float alpha, const float* row_scale, const float* bias, const float* den,
-                     const float* norm_ptr, float norm, int block_n, int* status, cudaStream_t stream) {
+                     const float* norm_ptr, float norm, int block_n, float* ws, int* status,
+                     cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   GemmParams<PlainEpi::Params> gp;
   memset(&gp, 0, sizeof(gp));
@@ -1642,57 +1705,66 @@ static int gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int 
   gp.status = status;
   rc = make_out_tmap(&gp.tma_out[0], C, M, N, ldc, c_is_bf16 ? 2 : 4);
   if (rc) return 300 + rc;
-  gp.epi = {alpha, row_scale, bias, c_is_bf16, accumulate, 0, 0, nullptr, {}, den, norm_ptr, norm};
-  if (!c_is_bf16 && bias == nullptr) {
-    // few output tiles but a long K (weight gradients, the write GEMM of a small batch): cut K so
-    // that every SM pair has work; the splits meet in the fp32 reduce-add epilogue, in an output
-    // that is cleared first where the caller did not ask to add to it.  Every split reduce-adds a
-    // whole output tile, so splits are long (32 K tiles; 16 where the tiles would leave most of
-    // the chip idle, 8 for a few rows).  384 x 384 from K = 8192 is 4 tiles.
-    const int tm = pairs ? 2 * kBlockM : kBlockM;
-    const long long tiles = static_cast<long long>((M + tm - 1) / tm) * ((N + BN - 1) / BN);
-    const int units = sm_count() / (pairs ? 2 : 1);
-    const int k_tiles = gp.seg[0].k_tiles;
-    if (tiles < 2 * units && k_tiles >= 64) {
-      const int min_len = M <= tm ? 8 : 4 * tiles <= units ? 16 : 32;
-      const int want = choose_k_splits(tiles, units, k_tiles, k_tiles / min_len);
-      if (want > 1) {
-        gp.k_splits = want;
-        if (!accumulate) {
-          if (cudaMemset2DAsync(C, ldc * sizeof(float), 0, N * sizeof(float), M, stream) != cudaSuccess) return 12;
-          gp.epi.accumulate = 1;
-        }
-      }
-    }
+  gp.epi = {alpha, row_scale, bias, c_is_bf16, accumulate, 0, 0, nullptr, {}, den, norm_ptr, norm, 0};
+  // With a workspace the parts of a split product are added up in order by a second kernel, and the
+  // result repeats bit by bit; without one they meet in the reduce-add of the epilogue, in the order
+  // in which they arrive, which only a caller that accumulates asks for.
+  const bool may_split = !c_is_bf16 && bias == nullptr && (accumulate || ws != nullptr);
+  const SplitPlan plan = may_split ? plan_splits(M, N, K, BN) : SplitPlan{1, 0, 0};
+  const bool ordered = plan.splits > 1 && ws != nullptr;
+  const int ldw = (N + 3) / 4 * 4;
+  if (plan.splits > 1) gp.k_splits = plan.splits;
+  if (ordered) {
+    if ((reinterpret_cast<uintptr_t>(ws) & 15) != 0) return 12;
+    const int rows = plan.m_tiles * plan.tile_m;
+    rc = make_out_tmap(&gp.tma_out[0], ws, static_cast<uint64_t>(plan.splits) * rows, N, ldw, 4);
+    if (rc) return 400 + rc;
+    gp.epi = {1.f, nullptr, nullptr, 0, 0, 0, 0, nullptr, {}, nullptr, nullptr, 1.f, rows};
   }
-  if (!pairs)
-    return BN == 128 ? launch_engine_impl<128, PlainEpi, 1>(gp, stream)
-                     : launch_engine_impl<256, PlainEpi, 1>(gp, stream);
-  return BN == 128 ? launch_engine_impl<128, PlainEpi, 2>(gp, stream)
-                   : launch_engine_impl<256, PlainEpi, 2>(gp, stream);
+  rc = !pairs ? (BN == 128 ? launch_engine_impl<128, PlainEpi, 1>(gp, stream)
+                           : launch_engine_impl<256, PlainEpi, 1>(gp, stream))
+              : (BN == 128 ? launch_engine_impl<128, PlainEpi, 2>(gp, stream)
+                           : launch_engine_impl<256, PlainEpi, 2>(gp, stream));
+  if (rc != 0 || !ordered) return rc;
+  float* out = static_cast<float*>(C);
+  const long long chunks = static_cast<long long>(M) * (ldw >> 2);
+  const int blocks = static_cast<int>(chunks / 256 + 1 < 148 * 8 ? chunks / 256 + 1 : 148 * 8);
+  const long long part = static_cast<long long>(plan.m_tiles) * plan.tile_m * ldw;
+  auto sum = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 ? split_sum_kernel<true>
+                                                                          : split_sum_kernel<false>;
+  sum<<<blocks, 256, 0, stream>>>(ws, part, plan.splits, ldw, M, N, out, ldc, accumulate, alpha, row_scale,
+                                  den, norm_ptr, norm);
+  return cudaGetLastError() == cudaSuccess ? 0 : 13;
+}
+
+extern "C" long long dsb_gemm_workspace(int M, int N, int K, int block_n) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const SplitPlan plan = plan_splits(M, N, K, block_n);
+  return plan.splits > 1 ? static_cast<long long>(plan.splits) * plan.m_tiles * plan.tile_m * ((N + 3) / 4 * 4) : 0;
 }
 
 extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn,
                              long long ldb, int M, int N, int K, void* C, long long ldc,
                              int c_is_bf16, int accumulate, float alpha, const float* row_scale,
-                             const float* bias, int block_n, int* status, cudaStream_t stream) {
+                             const float* bias, int block_n, float* ws, int* status,
+                             cudaStream_t stream) {
   if (M > 0 && M <= kFewRows && N > 0 && K > 0 && !a_mn && !b_mn && !c_is_bf16 && !accumulate &&
       row_scale == nullptr)
     return few_rows_gemm(A, lda, B, 0, ldb, M, N, K,
                          {static_cast<float*>(C), ldc, bias, nullptr, nullptr, alpha, 0}, status, stream);
   return gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, C, ldc, c_is_bf16, accumulate, alpha, row_scale,
-                   bias, nullptr, nullptr, 1.f, block_n, status, stream);
+                   bias, nullptr, nullptr, 1.f, block_n, ws, status, stream);
 }
 
 extern "C" int dsb_srw_write(const void* p, long long ldp, const void* write, long long ldw, int T, int U,
                              int D, const float* den, float norm, const float* norm_ptr, float* y,
-                             long long ldy, int accumulate, int* status, cudaStream_t stream) {
+                             long long ldy, int accumulate, float* ws, int* status, cudaStream_t stream) {
   if (T <= 0 || U <= 0 || D <= 0) return 0;
   if (T <= kFewRows && accumulate)
     return few_rows_gemm(p, ldp, write, 1, ldw, T, D, U, {y, ldy, nullptr, den, norm_ptr, norm, 1}, status,
                          stream);
   return gemm_bf16(p, 0, ldp, write, 1, ldw, T, D, U, y, ldy, 0, accumulate, 1.f, nullptr, nullptr, den,
-                   norm_ptr, norm, D <= 128 ? 128 : 256, status, stream);
+                   norm_ptr, norm, D <= 128 ? 128 : 256, ws, status, stream);
 }
 
 static GateConsts make_gc(const DsbGate* g) {
@@ -1963,7 +2035,7 @@ extern "C" int dsb_srw_forward(const void* h, long long ldh, const void* emb, lo
   if (rc) return rc;
   // raw_out[T,D] = p[T,U] . write[U,D]   (write is the MN-major B operand)
   return dsb_gemm_bf16(p_scratch, 0, ldp, write, 1, ldw, T, D, U, raw_out, ldo, 0, 0, 1.0f,
-                       nullptr, nullptr, 256, status, stream);
+                       nullptr, nullptr, 256, nullptr, status, stream);
 }
 
 // GEMM whose output rows are scattered to their owner ranks (first half of a

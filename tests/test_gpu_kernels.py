@@ -499,7 +499,8 @@ def test_lm_head_cross_entropy(cb):
 def test_kernels_are_run_to_run_deterministic(cb):
     """Every tile-produced output must be bit-identical between two runs (a
     missing barrier or a racing tile shows up here); only the per-token sums
-    that are accumulated with atomics may differ in the last bits."""
+    that are accumulated with atomics may differ in the last bits.  Products with
+    few tiles and a long K, which are cut: the next test."""
     from dawn_srw_b200.ops.gates import GateSpec
     dev = torch.device("cuda")
     g = torch.Generator(device=dev).manual_seed(9)
@@ -1129,3 +1130,48 @@ def test_router_takes_transposed_uses_and_layers_without_bias(cb, n2, bias):
         assert _rel(a, b) < 1e-2
     if bias:
         assert _rel(tau.bias.grad, wt.sum(1)) < 1e-2 and _rel(proj.bias.grad, wh.sum(1)) < 1e-2
+
+
+@pytest.mark.parametrize("M,N,K,a_mn", [(512, 384, 25200, False), (384, 384, 8192, True), (300, 131, 10400, False),
+                                        (8, 384, 8200, True), (129, 1280, 100000, False)])
+def test_split_products_repeat_bit_by_bit(cb, M, N, K, a_mn):
+    """A product that does not accumulate has the same bits in every run, also where K is cut: between
+    the runs another product of other sizes moves the splits to other SMs and stale accumulators."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(M)
+    A, B = torch.randn(M, K, device=dev, generator=g).bfloat16(), torch.randn(K, (N + 7) // 8 * 8, device=dev,
+                                                                             generator=g).bfloat16()[:, :N]
+    As = A.t().contiguous() if a_mn and M % 8 == 0 else A
+    big = torch.randn(777, 1024, device=dev, generator=g).bfloat16()
+    outs = []
+    for k in range(6):
+        cb.gemm(big[:100 * k + 1], False, big, False)
+        outs.append(cb.gemm(As, As is not A, B, True, out_dtype=torch.float32))
+    cb.check_status()
+    assert _rel(outs[0], A.double() @ B.double()) < 1e-5
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+
+
+def test_route_backward_of_few_tokens_repeats_bit_by_bit(cb):
+    """dx (in fp32, both routes added) and dh of a route against 25 200 units."""
+    from dawn_srw_b200.ops.gates import GateSpec
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(1)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    nz = lambda *s: torch.nn.functional.normalize(rn(*s), dim=-1).bfloat16()
+    T, U, r, D = 200, 25200, 128, 384
+    h, x, dy, emb, read, write = rn(T, r).bfloat16(), rn(T, D).bfloat16(), rn(T, D).bfloat16(), nz(U, r), nz(U, D), nz(U, D)
+    tau, isd, dden = torch.full((T,), 0.3, device=dev), torch.ones(T, device=dev), rn(T) * 0.01
+    runs = []
+    for _ in range(4):
+        gr = [torch.zeros(U, d, device=dev) for d in (r, D, D)]
+        dh, dx = torch.empty(T, r, device=dev), rn(T, D) * 0
+        for _ in range(2):
+            dtau = torch.zeros(T, device=dev)
+            cb.ext().srw_route_bwd(x, h, tau, isd, dy, dden, dtau, emb, read, write, *gr, None, dh, True, dx,
+                                   cb._gate_list(GateSpec(kind=1)), cb.status_word(dev))
+        runs.append((dh, dx))
+    cb.check_status()
+    assert float(runs[0][1].abs().max()) > 0
+    for dh, dx in runs[1:]:
+        assert torch.equal(dh, runs[0][0]) and torch.equal(dx, runs[0][1])
