@@ -997,9 +997,12 @@ std::vector<Tensor> linear_pack(std::vector<Tensor> srcs, std::vector<int64_t> c
   const c10::cuda::CUDAGuard guard(srcs[0].device());
   auto o = srcs[0].options();
   auto dst = torch::empty({T, n}, o.dtype(torch::kBFloat16));
-  auto sum = want_sum ? torch::zeros({n}, o) : Tensor();
-  int rc = dsb_linear_pack(s, static_cast<int>(srcs.size()), T, n, dst.data_ptr(),
-                           want_sum ? sum.data_ptr<float>() : nullptr, static_cast<unsigned long long>(seed),
+  Tensor sum, part;
+  if (want_sum) {
+    sum = T > 0 ? torch::empty({n}, o) : torch::zeros({n}, o);
+    part = torch::empty({dsb_linear_pack_blocks(T) * n}, o);
+  }
+  int rc = dsb_linear_pack(s, static_cast<int>(srcs.size()), T, n, dst.data_ptr(), ptr(sum), ptr(part), static_cast<unsigned long long>(seed),
                            static_cast<float>(p), n_drop, cur_stream());
   TORCH_CHECK(rc == 0, "dsb_linear_pack failed with code ", rc);
   if (want_sum) return {dst, sum};

@@ -61,9 +61,12 @@ int dsb_route_bwd_rows(const float* dy, const float* y, const float* den, const 
 int dsb_dropout(const float* res, const float* x, float* y, long long n, unsigned long long seed,
                 float p, cudaStream_t stream);
 
+// out[j] = sum over the rows of part [rows, n], in a fixed order; n % 4 == 0, part 16-byte aligned.
+int dsb_column_sum(const float* part, int rows, int n, float* out, cudaStream_t stream);
+
 // Gradient operand of a linear layer: dst bf16 [T, n] = bf16(sum of the up to five fp32 sources that
-// cover a column: cols columns from col0, row stride ld), 0 where none does; colsum [n] (nullable,
-// zeroed) += its column sums.  With p > 0 the columns [0, n_drop) are the gradient of a dropped
+// cover a column: cols columns from col0, row stride ld), 0 where none does; colsum [n] (nullable) = its
+// column sums, with part as scratch (dsb_linear_pack_blocks(T) * n floats, 16-byte aligned).  With p > 0 the columns [0, n_drop) are the gradient of a dropped
 // [T, n_drop] tensor: the keep mask of (seed, p) is applied.  n % 8 == 0, n_drop % 4 == 0.
 struct DsbPackSrc {
   const float* ptr;
@@ -71,8 +74,9 @@ struct DsbPackSrc {
   int col0, cols;
   int vec;          // set by the launcher: rows may be read as float4
 };
+int dsb_linear_pack_blocks(int T);
 int dsb_linear_pack(const struct DsbPackSrc* src, int n_src, int T, int n, void* dst_bf16, float* colsum,
-                    unsigned long long seed, float p, int n_drop, cudaStream_t stream);
+                    float* part, unsigned long long seed, float p, int n_drop, cudaStream_t stream);
 // Operand of a router GEMM: w bf16 [n, D] = rows of w1 [n1, D], of w2 [n2, D], zeros; b [n] likewise
 // (all fp32 contiguous, n >= n1 + n2).
 int dsb_router_operand(const float* w1, const float* b1, const float* w2, const float* b2, int n1, int n2,

@@ -782,24 +782,52 @@ extern "C" int dsb_dropout(const float* res, const float* x, float* y, long long
 // ------------------------------------------------- operand of a linear layer's backward
 // dst bf16 [T, n] = bf16(sum of the sources that cover a column), 0 where none does, and the column
 // sums of the same values (the bias gradient) in one pass: a source is an fp32 [T, cols] block at
-// column col0, source 0 optionally under the keep mask of a [T, n_drop]-shaped dropout.  Bound by
-// its bytes (6 per element): separate cast, sum, slice and pad ops read a gradient three times,
-// and a column sum of 8192 x 384 alone took 18.6 us.  A thread owns four columns, a block 128 columns
-// of 64 rows.
+// column col0; the columns of the sum below n_drop are optionally under the keep mask of a
+// [T, n_drop]-shaped dropout.  Bound by its bytes (6 per element): separate cast, sum, slice and pad ops
+// read a gradient three times, and a column sum of 8192 x 384 alone took 18.6 us.  A thread owns four
+// columns, a block 128 columns of 64 rows (more where the grid could not hold them); the blocks' sums
+// are added up in their order by column_sum_kernel, so that a bias gradient repeats bit by bit.
 namespace {
-constexpr int kPackRows = 64;
+constexpr int kPackRows = 64, kMaxGridY = 65535;
+int pack_rows(int T) { return T <= kPackRows * kMaxGridY ? kPackRows : (T / kMaxGridY / 8 + 1) * 8; }
+
+// out[j] = part[0][j] + part[1][j] + ... in a fixed order (n % 4 == 0, part 16-byte aligned): a block takes 32
+// columns, its 32 groups of eight threads every 32nd row.
+__global__ void __launch_bounds__(256) column_sum_kernel(const float* __restrict__ part, int rows, int n,
+                                                         float* __restrict__ out) {
+  __shared__ __align__(16) float s_sum[32][36];
+  const int q = threadIdx.x & 7, ry = threadIdx.x >> 3, c = blockIdx.x * 32 + 4 * q;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < n) {
+#pragma unroll 4
+    for (int y = ry; y < rows; y += 32) {
+      const float4 v = *reinterpret_cast<const float4*>(part + static_cast<size_t>(y) * n + c);
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+  }
+  *reinterpret_cast<float4*>(&s_sum[ry][4 * q]) = a;
+  __syncthreads();
+  const int j = blockIdx.x * 32 + threadIdx.x;
+  if (threadIdx.x < 32 && j < n) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) t += s_sum[k][threadIdx.x];
+    out[j] = t;
+  }
+}
+
 template <int kSrc>
 __global__ void __launch_bounds__(256) linear_pack_kernel(const DsbPackSrc s0, const DsbPackSrc s1,
                                                           const DsbPackSrc s2, const DsbPackSrc s3,
-                                                          const DsbPackSrc s4, int T, int n,
+                                                          const DsbPackSrc s4, int T, int n, int rows,
                                                           __nv_bfloat16* __restrict__ dst,
-                                                          float* __restrict__ colsum, uint64_t seed,
+                                                          float* __restrict__ part, uint64_t seed,
                                                           uint32_t thresh, float keep_scale, int n_drop) {
   __shared__ float s_sum[8][128];
   const DsbPackSrc src[5] = {s0, s1, s2, s3, s4};
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 128 + 4 * cx;
-  const int lo = blockIdx.y * kPackRows, hi = min(T, lo + kPackRows);
+  const int lo = blockIdx.y * rows, hi = T - lo < rows ? T : lo + rows;
   float sum[4] = {0.f, 0.f, 0.f, 0.f};
   if (c < n) {                                            // n % 8 == 0
 #pragma unroll 2
@@ -837,7 +865,7 @@ __global__ void __launch_bounds__(256) linear_pack_kernel(const DsbPackSrc s0, c
       for (int j = 0; j < 4; ++j) sum[j] += v[j];
     }
   }
-  if (colsum == nullptr) return;
+  if (part == nullptr) return;
 #pragma unroll
   for (int j = 0; j < 4; ++j) s_sum[ry][4 * cx + j] = sum[j];
   __syncthreads();
@@ -845,7 +873,7 @@ __global__ void __launch_bounds__(256) linear_pack_kernel(const DsbPackSrc s0, c
     float a = 0.f;
 #pragma unroll
     for (int r = 0; r < 8; ++r) a += s_sum[r][threadIdx.x];
-    atomicAdd(colsum + blockIdx.x * 128 + threadIdx.x, a);
+    part[static_cast<size_t>(blockIdx.y) * n + blockIdx.x * 128 + threadIdx.x] = a;
   }
 }
 
@@ -866,10 +894,23 @@ __global__ void __launch_bounds__(256) dropout_rows_kernel(const float* __restri
 }
 }  // namespace
 
+extern "C" int dsb_column_sum(const float* part, int rows, int n, float* out, cudaStream_t stream) {
+  if (rows < 0 || n < 0 || (n & 3) || (reinterpret_cast<uintptr_t>(part) & 15) != 0) return 2;
+  if (n == 0) return 0;
+  column_sum_kernel<<<(n + 31) / 32, 256, 0, stream>>>(part, rows, n, out);
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
+}
+
+extern "C" int dsb_linear_pack_blocks(int T) {
+  const int rows = pack_rows(T);
+  return T / rows + (T % rows != 0);
+}
+
 extern "C" int dsb_linear_pack(const DsbPackSrc* src, int n_src, int T, int n, void* dst_bf16,
-                               float* colsum, unsigned long long seed, float p, int n_drop,
+                               float* colsum, float* part, unsigned long long seed, float p, int n_drop,
                                cudaStream_t stream) {
   if (T <= 0 || n <= 0) return 0;
+  if (colsum != nullptr && (part == nullptr || (reinterpret_cast<uintptr_t>(part) & 15) != 0)) return 2;
   if (n_src < 1 || n_src > 5 || (n & 7) || (n_drop & 3) || !(p >= 0.f && p < 1.f)) return 2;
   DsbPackSrc s[5];
   for (int i = 0; i < 5; ++i) {
@@ -877,17 +918,20 @@ extern "C" int dsb_linear_pack(const DsbPackSrc* src, int n_src, int T, int n, v
     s[i].vec = (reinterpret_cast<uintptr_t>(s[i].ptr) & 15) == 0 && (s[i].ld & 3) == 0 && (s[i].col0 & 3) == 0;
   }
   const uint32_t thresh = static_cast<uint32_t>(static_cast<double>(p) * 4294967296.0);
-  const dim3 grid((n + 127) / 128, (T + kPackRows - 1) / kPackRows);
+  const int rows = pack_rows(T), row_blocks = dsb_linear_pack_blocks(T);
+  const dim3 grid((n + 127) / 128, row_blocks);
+  float* sums = colsum == nullptr ? nullptr : row_blocks == 1 ? colsum : part;
   __nv_bfloat16* d = static_cast<__nv_bfloat16*>(dst_bf16);
   const float sc = 1.f / (1.f - p);
   if (n_src == 1)
-    linear_pack_kernel<1><<<grid, 256, 0, stream>>>(s[0], s[1], s[2], s[3], s[4], T, n, d, colsum, seed, thresh, sc, n_drop);
+    linear_pack_kernel<1><<<grid, 256, 0, stream>>>(s[0], s[1], s[2], s[3], s[4], T, n, rows, d, sums, seed, thresh, sc, n_drop);
   else if (n_src == 2)
-    linear_pack_kernel<2><<<grid, 256, 0, stream>>>(s[0], s[1], s[2], s[3], s[4], T, n, d, colsum, seed, thresh, sc, n_drop);
+    linear_pack_kernel<2><<<grid, 256, 0, stream>>>(s[0], s[1], s[2], s[3], s[4], T, n, rows, d, sums, seed, thresh, sc, n_drop);
   else {
     for (int i = n_src; i < 5; ++i) s[i].cols = 0;         // covers nothing
-    linear_pack_kernel<5><<<grid, 256, 0, stream>>>(s[0], s[1], s[2], s[3], s[4], T, n, d, colsum, seed, thresh, sc, n_drop);
+    linear_pack_kernel<5><<<grid, 256, 0, stream>>>(s[0], s[1], s[2], s[3], s[4], T, n, rows, d, sums, seed, thresh, sc, n_drop);
   }
+  if (sums != colsum) column_sum_kernel<<<(n + 31) / 32, 256, 0, stream>>>(part, row_blocks, n, colsum);
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

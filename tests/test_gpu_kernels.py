@@ -1175,3 +1175,30 @@ def test_route_backward_of_few_tokens_repeats_bit_by_bit(cb):
     assert float(runs[0][1].abs().max()) > 0
     for dh, dx in runs[1:]:
         assert torch.equal(dh, runs[0][0]) and torch.equal(dx, runs[0][1])
+
+
+@pytest.mark.parametrize("T,n,cols", [(1, 8, [(0, 8)]), (64, 128, [(0, 128)]), (65, 136, [(3, 130), (0, 136)]),
+                                      (8192, 384, [(0, 384)]), (20011, 1160, [(0, 768), (768, 3), (768, 1)])])
+def test_packed_gradient_and_its_column_sums_repeat(cb, T, n, cols):
+    """One row block to many, ragged columns and rows: the bf16 operand exact, fp32 sums of T terms against
+    fp64 (1e-5 of the terms' norm) and the same bits in every run."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(T)
+    srcs = [torch.randn(T, w, device=dev, generator=g) for _, w in cols]
+    total = torch.zeros(T, n, device=dev)
+    for (c, w), s in zip(cols, srcs):
+        total[:, c:c + w] += s
+    first = None
+    for _ in range(4):
+        dst, db = cb.ext().linear_pack(srcs, [c for c, _ in cols], T, n, True, 0, 0.0, 0)
+        first = db if first is None else first
+        assert torch.equal(dst, total.bfloat16()) and torch.equal(db, first)
+    assert float((db.double() - total.double().sum(0)).norm()) < 1e-5 * float(total.double().norm()) + 1e-6
+
+
+def test_packed_gradient_of_more_rows_than_a_grid_has_blocks_of_64(cb):
+    T, dev = 65535 * 64 + 77, torch.device("cuda")
+    src = torch.randn(T, 8, device=dev)
+    dst, db = cb.ext().linear_pack([src], [0], T, 8, True, 0, 0.0, 0)
+    assert torch.equal(dst, src.bfloat16())
+    assert float((db.double() - src.double().sum(0)).norm()) < 1e-5 * float(src.double().norm())
