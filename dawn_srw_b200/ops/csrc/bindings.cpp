@@ -867,10 +867,11 @@ std::vector<Tensor> route_bwd_rows(const Tensor& dy, const Tensor& y, const Tens
               "route_bwd_rows: dy and y must be 16-byte aligned");
   const c10::cuda::CUDAGuard guard(dy.device());
   auto dyb = torch::empty({T, D}, dy.options().dtype(torch::kBFloat16)), d_den = torch::empty({T}, dy.options());
+  auto dots = opt_f32_mut(d_scale) != nullptr ? torch::empty({(T + 7) / 8}, dy.options()) : Tensor();
   int rc = dsb_route_bwd_rows(dy.data_ptr<float>(), y.data_ptr<float>(), den.data_ptr<float>(),
                               opt_f32(scale_t), scale, opt_f32(ext_dden), dyb.data_ptr(),
-                              d_den.data_ptr<float>(), dtau.data_ptr<float>(), opt_f32_mut(d_scale), T, D,
-                              cur_stream());
+                              d_den.data_ptr<float>(), dtau.data_ptr<float>(), opt_f32_mut(d_scale), ptr(dots),
+                              T, D, cur_stream());
   TORCH_CHECK(rc == 0, "dsb_route_bwd_rows failed with code ", rc);
   return {dyb, d_den};
 }

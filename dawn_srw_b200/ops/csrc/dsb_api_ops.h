@@ -50,10 +50,10 @@ int dsb_route_bwd_prologue(const float* dy, const float* y, const float* row_sca
 
 // With rs = s / max(den, 1), s = *scale_ptr or scale: dy_bf = bf16(dy * rs); with rowdot = <dy, y>:
 // d_den = -rowdot / den where den > 1, else 0 (+ ext_dden, nullable); dtau = 0;
-// d_scale[0] += sum_t rowdot / s (nullable).  dy, y fp32 [T, D], D % 4 == 0, 16-byte aligned.
+// d_scale[0] += sum_t rowdot / s (nullable; dots: T / 8 rounded up floats of scratch for it).  dy, y fp32 [T, D], D % 4 == 0, 16-byte aligned.
 int dsb_route_bwd_rows(const float* dy, const float* y, const float* den, const float* scale_ptr,
                        float scale, const float* ext_dden, void* dy_bf16, float* d_den, float* dtau,
-                       float* d_scale, int T, int D, cudaStream_t stream);
+                       float* d_scale, float* dots, int T, int D, cudaStream_t stream);
 
 // y = res + dropout(x) (res may be null: y = dropout(x)); fp32, n % 4 == 0.  An element is kept
 // (and scaled by 1 / (1 - p)) iff a hash of (seed, its index) is >= p * 2^32, so the gradient

@@ -541,13 +541,13 @@ __global__ void route_bwd_prologue_kernel(const float* __restrict__ dy, const fl
 
 // The same for a route whose denominator and scale are still separate, with all that follows per
 // row: row_scale = s / max(den, 1);  d_den = -rowdot / den where den > 1 (+ ext_dden);
-// d_scale += sum_t rowdot / s;  dtau = 0 (the gate kernel adds into it).  One pass over dy and y
+// dots[block] = its rows' sum of rowdot (scale_grad_kernel);  dtau = 0 (the gate kernel adds into it).  One pass over dy and y
 // instead of that plus nine tensor ops on [T].
 __global__ void __launch_bounds__(256) route_bwd_rows_kernel(
     const float* __restrict__ dy, const float* __restrict__ y, const float* __restrict__ den,
     const float* __restrict__ scale_ptr, float scale, const float* __restrict__ ext_dden,
     __nv_bfloat16* __restrict__ dy_bf, float* __restrict__ d_den, float* __restrict__ dtau,
-    float* __restrict__ d_scale, int T, int D) {
+    float* __restrict__ dots, int T, int D) {
   __shared__ float s_dot[8];
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -576,15 +576,34 @@ __global__ void __launch_bounds__(256) route_bwd_rows_kernel(
       dtau[t] = 0.f;
     }
   }
-  if (d_scale != nullptr) {
+  if (dots != nullptr) {
     if (lane == 0) s_dot[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
       float tot = 0.f;
 #pragma unroll
       for (int k = 0; k < 8; ++k) tot += s_dot[k];
-      atomicAdd(d_scale, tot / sc);
+      dots[blockIdx.x] = tot;
     }
+  }
+}
+
+// d_scale += (dots[0] + dots[1] + ...) / s, in a fixed order: the gradient of a scale repeats bit by bit.
+__global__ void __launch_bounds__(256) scale_grad_kernel(const float* __restrict__ dots, int n,
+                                                         const float* __restrict__ scale_ptr, float scale,
+                                                         float* __restrict__ d_scale) {
+  __shared__ float s_sum[8];
+  float a = 0.f;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += 256) a += dots[i];
+  a = warp_sum(a);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a += s_sum[k];
+    d_scale[0] += a / (scale_ptr != nullptr ? scale_ptr[0] : scale);
   }
 }
 
@@ -711,13 +730,15 @@ extern "C" int dsb_route_bwd_prologue(const float* dy, const float* y, const flo
 
 extern "C" int dsb_route_bwd_rows(const float* dy, const float* y, const float* den,
                                   const float* scale_ptr, float scale, const float* ext_dden,
-                                  void* dy_bf16, float* d_den, float* dtau, float* d_scale, int T, int D,
-                                  cudaStream_t stream) {
+                                  void* dy_bf16, float* d_den, float* dtau, float* d_scale, float* dots,
+                                  int T, int D, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if (D & 3) return 2;
+  if ((D & 3) || (d_scale != nullptr && dots == nullptr)) return 2;
   route_bwd_rows_kernel<<<(T + 7) / 8, 256, 0, stream>>>(
       dy, y, den, scale_ptr, scale, ext_dden, reinterpret_cast<__nv_bfloat16*>(dy_bf16), d_den, dtau,
-      d_scale, T, D);
+      d_scale != nullptr ? dots : nullptr, T, D);
+  if (d_scale != nullptr)
+    scale_grad_kernel<<<1, 256, 0, stream>>>(dots, (T + 7) / 8, scale_ptr, scale, d_scale);
   return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 

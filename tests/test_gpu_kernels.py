@@ -1202,3 +1202,20 @@ def test_packed_gradient_of_more_rows_than_a_grid_has_blocks_of_64(cb):
     dst, db = cb.ext().linear_pack([src], [0], T, 8, True, 0, 0.0, 0)
     assert torch.equal(dst, src.bfloat16())
     assert float((db.double() - src.double().sum(0)).norm()) < 1e-5 * float(src.double().norm())
+
+
+@pytest.mark.parametrize("T,D", [(1, 8), (9, 128), (8195, 136)])
+def test_scale_gradient_of_a_route_repeats_bit_by_bit(cb, T, D):
+    """Added to what is there; fp32 sums of T * D products against fp64: 1e-5 of their norm, sqrt(T)-fold for
+    the sum over rows; the same bits in every run."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(T)
+    dy, y, den = (torch.randn(*s, device=dev, generator=g) for s in ((T, D), (T, D), (T,)))
+    scale, outs = torch.full((), 1.7, device=dev), []
+    for _ in range(5):
+        d_scale = torch.full((), 0.5, device=dev)
+        cb.ext().route_bwd_rows(dy, y, den, 1.0, scale, None, torch.empty(T, device=dev), d_scale)
+        outs.append(d_scale)
+    dots = (dy.double() * y.double()).sum(-1) / 1.7
+    assert abs(float(outs[0]) - 0.5 - float(dots.sum())) < 1e-5 * float(dots.norm()) * T ** 0.5 + 1e-5
+    assert all(torch.equal(o, outs[0]) for o in outs)
