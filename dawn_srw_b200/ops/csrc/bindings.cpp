@@ -1121,10 +1121,11 @@ std::vector<Tensor> load_balance_bwd(const Tensor& emb, const Tensor& m_u, const
   const int U = emb.size(0), r = emb.size(1);
   TORCH_CHECK(g_lb.is_cuda() && g_lb.scalar_type() == torch::kFloat32 && g_lb.numel() == 1 &&
               m_u.numel() == U && m_u.is_contiguous() && stat.numel() == 2);
-  auto dmn = torch::empty({U}, m_u.options()), d_hsum = torch::zeros({r}, m_u.options());
+  auto dmn = torch::empty({U}, m_u.options()), d_hsum = torch::empty({r}, m_u.options()),
+       part = torch::empty({static_cast<int64_t>(dsb_load_balance_blocks(U, r)) * r}, m_u.options());
   int rc = dsb_load_balance_bwd(emb.data_ptr(), emb.stride(0), m_u.data_ptr<float>(), stat.data_ptr<float>(),
                                 g_lb.data_ptr<float>(), inv_n, units, U, r, dmn.data_ptr<float>(),
-                                d_hsum.data_ptr<float>(), cur_stream());
+                                d_hsum.data_ptr<float>(), part.data_ptr<float>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_load_balance_bwd failed with code ", rc);
   return {dmn, d_hsum};
 }

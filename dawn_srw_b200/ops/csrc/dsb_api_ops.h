@@ -134,14 +134,15 @@ int dsb_score_stats_bwd(const float* d_tau, const float* d_isd, const float* d_h
 //   lb = var / (mean^2 + var + 0.01) with mean = sum m_u / units, var = sum m_u^2 / units - mean^2.
 // emb bf16 [U, lde], r and lde multiples of 8, r <= 512.  part: 2 * dsb_load_balance_blocks floats of
 // scratch; m_u and stat [2] are kept for the backward call, which writes dmn [U] (= d m_u * inv_n)
-// and accumulates d_hsum [r] (zero it first); the embedding gradient is dmn[u] * hsum.
+// and d_hsum [r], with dsb_load_balance_blocks * r floats of scratch (16-byte aligned) as its part; the
+// embedding gradient is dmn[u] * hsum.
 int dsb_load_balance_blocks(int U, int r);
 int dsb_load_balance_fwd(const void* emb_bf16, long long lde, const float* hsum, float inv_n,
                          float units, int U, int r, float* m_u, float* part, float* lb, float* stat,
                          cudaStream_t stream);
 int dsb_load_balance_bwd(const void* emb_bf16, long long lde, const float* m_u, const float* stat,
                          const float* g_lb, float inv_n, float units, int U, int r, float* dmn,
-                         float* d_hsum, cudaStream_t stream);
+                         float* d_hsum, float* part, cudaStream_t stream);
 // g[u, :] += sum_l dm[l, u] * hs[l, :]  (g fp32 [U, ldg], dm [L, U], hs [L, r], r % 4 == 0).
 int dsb_rank1_add(float* g, long long ldg, const float* dm, const float* hs, int L, int U, int r,
                   cudaStream_t stream);

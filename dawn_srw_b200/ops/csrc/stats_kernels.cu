@@ -437,7 +437,8 @@ __global__ void __launch_bounds__(256) lb_finish_kernel(const float* __restrict_
 
 // With q = mean^2 + var + eps:  d mean = -2 mean / q,  d (sum m^2 / U) = (mean^2 + eps) / q^2, so
 //   dm_u = g / U * (d mean + 2 m_u d(sum m^2 / U)),   dmn[u] = dm_u * inv_n,
-//   d_hsum += sum_u dmn[u] e_u.   The embedding gradient dmn[u] * hsum is left to
+//   d_hsum = sum_u dmn[u] e_u: a slab of shared memory per warp, a row of part per block, and a launch
+// that adds the rows up in order, so that it repeats bit by bit.  The embedding gradient dmn[u] * hsum is left to
 // rank1_add_kernel, which takes the calls of all layers in one pass over the gradient buffer.
 template <int KC>
 __global__ void __launch_bounds__(kLbThreads) lb_bwd_kernel(const __nv_bfloat16* __restrict__ emb,
@@ -446,10 +447,8 @@ __global__ void __launch_bounds__(kLbThreads) lb_bwd_kernel(const __nv_bfloat16*
                                                             const float* __restrict__ g_lb, float units,
                                                             float inv_n, int U, int r, int lpu,
                                                             float* __restrict__ dmn,
-                                                            float* __restrict__ d_hsum) {
-  __shared__ float s_sum[kMaxR];
-  for (int j = threadIdx.x; j < r; j += kLbThreads) s_sum[j] = 0.f;
-  __syncthreads();
+                                                            float* __restrict__ part) {
+  __shared__ float s_sum[kLbThreads / 32][kMaxR];
   const int lane = threadIdx.x & 31, sub = lane & (lpu - 1), chunks = r >> 3;
   const int per_warp = 32 / lpu;
   const float mean = stat[0], q = stat[1], g = g_lb[0] * inv_n / units;
@@ -492,13 +491,19 @@ __global__ void __launch_bounds__(kLbThreads) lb_bwd_kernel(const __nv_bfloat16*
 #pragma unroll
   for (int k = 0; k < KC; ++k) {
     const int c = sub + lpu * k;
-    if (c < chunks) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) atomicAdd(&s_sum[8 * c + j], acc[k][j]);
+    for (int j = 0; j < 8; ++j) {
+      for (int o = lpu; o < 32; o <<= 1) acc[k][j] += __shfl_xor_sync(0xffffffffu, acc[k][j], o);
+      if (lane < lpu && c < chunks) s_sum[threadIdx.x >> 5][8 * c + j] = acc[k][j];
     }
   }
   __syncthreads();
-  for (int j = threadIdx.x; j < r; j += kLbThreads) atomicAdd(d_hsum + j, s_sum[j]);
+  for (int j = threadIdx.x; j < r; j += kLbThreads) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < kLbThreads / 32; ++w) t += s_sum[w][j];
+    part[static_cast<size_t>(blockIdx.x) * r + j] = t;
+  }
 }
 
 // g[u, :] += sum_l dm[l, u] * hs[l, :] (fp32 [U, r], row stride ldg): one read and write of the
@@ -638,15 +643,17 @@ extern "C" int dsb_load_balance_fwd(const void* emb_bf16, long long lde, const f
 
 extern "C" int dsb_load_balance_bwd(const void* emb_bf16, long long lde, const float* m_u,
                                     const float* stat, const float* g_lb, float inv_n, float units,
-                                    int U, int r, float* dmn, float* d_hsum, cudaStream_t stream) {
+                                    int U, int r, float* dmn, float* d_hsum, float* part,
+                                    cudaStream_t stream) {
   if (U <= 0 || r <= 0 || r > kMaxR || r % 8 != 0 || lde % 8 != 0) return 803;
   const int lpu = lb_lanes(r), blocks = dsb_load_balance_blocks(U, r);
   const __nv_bfloat16* e = static_cast<const __nv_bfloat16*>(emb_bf16);
   if (r <= 8 * lpu)
-    lb_bwd_kernel<1><<<blocks, kLbThreads, 0, stream>>>(e, lde, m_u, stat, g_lb, units, inv_n, U, r, lpu, dmn, d_hsum);
+    lb_bwd_kernel<1><<<blocks, kLbThreads, 0, stream>>>(e, lde, m_u, stat, g_lb, units, inv_n, U, r, lpu, dmn, part);
   else
-    lb_bwd_kernel<2><<<blocks, kLbThreads, 0, stream>>>(e, lde, m_u, stat, g_lb, units, inv_n, U, r, lpu, dmn, d_hsum);
-  return cudaGetLastError() == cudaSuccess ? 0 : 802;
+    lb_bwd_kernel<2><<<blocks, kLbThreads, 0, stream>>>(e, lde, m_u, stat, g_lb, units, inv_n, U, r, lpu, dmn, part);
+  if (cudaGetLastError() != cudaSuccess) return 802;
+  return dsb_column_sum(part, blocks, r, d_hsum, stream);
 }
 
 extern "C" int dsb_rank1_add(float* g, long long ldg, const float* dm, const float* hs, int L, int U,

@@ -1219,3 +1219,17 @@ def test_scale_gradient_of_a_route_repeats_bit_by_bit(cb, T, D):
     dots = (dy.double() * y.double()).sum(-1) / 1.7
     assert abs(float(outs[0]) - 0.5 - float(dots.sum())) < 1e-5 * float(dots.norm()) * T ** 0.5 + 1e-5
     assert all(torch.equal(o, outs[0]) for o in outs)
+
+
+@pytest.mark.parametrize("U,r", [(1, 8), (77, 512), (2600, 128), (100000, 256)])
+def test_load_balance_gradient_repeats_bit_by_bit(cb, U, r):
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(U)
+    emb = torch.randn(U, r, device=dev, generator=g).bfloat16()
+    m_u = torch.randn(U, device=dev, generator=g)
+    stat, one = torch.tensor([0.1, 1.2], device=dev), torch.ones((), device=dev)
+    runs = [cb.ext().load_balance_bwd(emb, m_u, stat, one, 0.01, float(U)) for _ in range(4)]
+    dmn, d_hsum = runs[0]
+    want = dmn.double() @ emb.double()
+    assert float((d_hsum.double() - want).norm()) < 1e-5 * float(dmn.norm()) * float(emb.double().norm()) / r ** 0.5
+    assert all(torch.equal(a, dmn) and torch.equal(b, d_hsum) for a, b in runs[1:])
