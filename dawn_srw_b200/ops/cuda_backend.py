@@ -1077,10 +1077,10 @@ class CudaBackend:
         x_bf = _bf16_2d(x)
         Up = _round_up(U, 8)
         D = x.shape[1]
-        if out_scale is None:
-            scale = 1.0
-        else:
-            scale = out_scale.detach().float() if isinstance(out_scale, torch.Tensor) else float(out_scale)
+        if isinstance(out_scale, torch.Tensor) and out_scale.is_cuda:
+            scale = out_scale.detach().float()
+        else:                                        # a number, on the host
+            scale = 1.0 if out_scale is None else float(out_scale)
         gl = _gate_list(spec)
         # Routes of one pool are independent token rows as far as the kernels care: with few
         # tokens (decoding) they are stacked into one call, so the pool is streamed once.

@@ -1233,3 +1233,20 @@ def test_load_balance_gradient_repeats_bit_by_bit(cb, U, r):
     want = dmn.double() @ emb.double()
     assert float((d_hsum.double() - want).norm()) < 1e-5 * float(dmn.norm()) * float(emb.double().norm()) / r ** 0.5
     assert all(torch.equal(a, dmn) and torch.equal(b, d_hsum) for a, b in runs[1:])
+
+
+@pytest.mark.parametrize("T", [1, 40, 150])
+def test_inference_call_takes_a_scale_on_the_host(cb, T):
+    """The three regimes of row counts; a 0-dim tensor in host memory is a number like any other."""
+    from dawn_srw_b200.ops.gates import GateSpec
+    dev = torch.device("cuda")
+    torch.manual_seed(T)
+    U, r, D, be, spec = 600, 64, 128, cb.CudaBackend(), GateSpec(kind=1)
+    pool = be.prepare_pool(*(torch.nn.functional.normalize(torch.randn(U, d, device=dev), dim=-1) for d in (r, D, D)),
+                           spec)
+    x, h, off = torch.randn(T, D, device=dev), torch.randn(T, 2, r, device=dev), torch.randn(T, 2, device=dev) * 0.1
+    outs = [torch.stack(be.srw_infer(x, h, off, pool, spec, out_scale=s))
+            for s in (0.75, torch.tensor(0.75), torch.tensor(0.75, device=dev), torch.tensor([0.75]))]
+    cb.check_status()
+    for o in outs[1:]:
+        assert _rel(o, outs[0]) < 1e-5
