@@ -593,7 +593,7 @@ class _SRWCallFn(torch.autograd.Function):
         ys, xrs = [], []
         for i in range(R):
             rows = slice(i * T, (i + 1) * T)
-            xr = _alloc_saved_xr(dev, T, Up, U, keep)
+            xr = _alloc_saved_xr(dev, T, Up, U, keep and any(ctx.needs_input_grad))
             y = torch.empty(T, D, dtype=torch.float32, device=dev)
             e.srw_route_fwd(hb[rows], x_bf, emb, read, write, p, xr, tau[rows], isd[rows], den[i],
                             None if diag is None else diag[i], alive, unit_mask, gl, sc_f, sc_t, y, False, st)

@@ -1250,3 +1250,17 @@ def test_inference_call_takes_a_scale_on_the_host(cb, T):
     cb.check_status()
     for o in outs[1:]:
         assert _rel(o, outs[0]) < 1e-5
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_read_scalars_are_kept_only_for_a_backward_pass(cb, monkeypatch, grad):
+    """With gradients enabled but nothing that requires one (a frozen model), no buffer is taken."""
+    from dawn_srw_b200.ops.gates import GateSpec
+    dev, kept = torch.device("cuda"), []
+    U, r, D, T, be, spec = 2600, 64, 128, 300, cb.CudaBackend(), GateSpec(kind=1)
+    alloc = cb._alloc_saved_xr
+    monkeypatch.setattr(cb, "_alloc_saved_xr", lambda *a: kept.append(alloc(*a)) or kept[-1])
+    pool = be.prepare_pool(*(torch.randn(U, d, device=dev) for d in (r, D, D)), spec)
+    h = torch.randn(T, 1, r, device=dev, requires_grad=grad)
+    be.srw(torch.randn(T, D, device=dev), h, torch.zeros(T, 1, device=dev), pool, spec, want_diag=False)
+    assert len(kept) == 1 and (kept[0] is not None) == grad
