@@ -707,7 +707,7 @@ std::vector<Tensor> srw_stats(const Tensor& h, const Tensor& off, const Tensor& 
   auto o = h.options();
   auto hb = torch::empty({N, r}, o.dtype(torch::kBFloat16)), hg = torch::empty({N, 2 * r}, o);
   auto rows = torch::empty({4 * static_cast<int64_t>(N)}, o), den = torch::empty({R, T}, o),
-       hsum = torch::empty({r}, o);
+       hsum = N > 0 ? torch::empty({r}, o) : torch::zeros({r}, o);
   float *tau = rows.data_ptr<float>(), *isd = tau + N, *mu = isd + N, *sd = mu + N;
   int rc = dsb_score_pack(h.data_ptr<float>(), h.stride(0), h.stride(1), T, R, r, hb.data_ptr(),
                           den.data_ptr<float>(), N, hsum.data_ptr<float>(), r, cur_stream());

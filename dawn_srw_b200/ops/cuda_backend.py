@@ -1284,7 +1284,8 @@ class CudaBackend:
             var_score = ns_sq / U_tot - mean_score ** 2
             lb = var_score / (mean_score ** 2 + var_score + 1e-2)
         else:
-            lb = _LoadBalanceFn.apply(hsum, anchor, pool.tensors, U, 1.0 / (T * Rr), float(U_tot))
+            inv_n = 1.0 / (T * Rr) if T > 0 else math.nan               # the mean over no token
+            lb = _LoadBalanceFn.apply(hsum, anchor, pool.tensors, U, inv_n, float(U_tot))
         den = den.t().clamp(min=1.0)
         dead_pen = x.new_zeros(())
         if spec.has_dead_penalty:

@@ -1264,3 +1264,18 @@ def test_read_scalars_are_kept_only_for_a_backward_pass(cb, monkeypatch, grad):
     h = torch.randn(T, 1, r, device=dev, requires_grad=grad)
     be.srw(torch.randn(T, D, device=dev), h, torch.zeros(T, 1, device=dev), pool, spec, want_diag=False)
     assert len(kept) == 1 and (kept[0] is not None) == grad
+
+
+def test_pool_call_without_tokens(cb):
+    """Empty outputs, no gradient, and a load-balance term that is the mean over nothing."""
+    from dawn_srw_b200.ops.gates import GateSpec
+    dev = torch.device("cuda")
+    U, r, D, be, spec = 600, 64, 128, cb.CudaBackend(), GateSpec(kind=1)
+    ps = [torch.randn(U, d, device=dev, requires_grad=True) for d in (r, D, D)]
+    x, h, off = (torch.empty(*s, device=dev, requires_grad=True) for s in ((0, D), (0, 2, r), (0, 2)))
+    scale = torch.tensor(1.5, device=dev, requires_grad=True)
+    res = be.srw(x, h, off, be.prepare_pool(*ps, spec), spec, want_diag=False, out_scale=scale)
+    assert res.route(0).shape == (0, D) and bool(res.lb.isnan())
+    (res.route(0).sum() + res.route(1).sum()).backward()
+    cb.check_status()
+    assert float(scale.grad) == 0.0 and all(float(p.grad.abs().max()) == 0.0 for p in ps)
