@@ -1232,6 +1232,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear_pack", &linear_pack);
   m.def("router_operand", &router_operand);
   m.def("kv_decode_attention", &kv_decode_attention);
+  m.def("gemm_few_tiles", [](int64_t M, int64_t N) { return dsb_gemm_few_tiles(M, N, block_width(N)) != 0; });
   m.def("srw_rows_max", [](int64_t D) { return dsb_srw_rows_max(static_cast<int>(D)); });
   m.def("srw_fwd_gate_gather", &srw_fwd_gate_gather);
   m.def("srw_bwd_gate_gather", &srw_bwd_gate_gather);

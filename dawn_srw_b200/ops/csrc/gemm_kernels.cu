@@ -1737,6 +1737,13 @@ static int gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int 
   return cudaGetLastError() == cudaSuccess ? 0 : 13;
 }
 
+extern "C" int dsb_gemm_few_tiles(int M, int N, int block_n) {
+  const bool pairs = use_cta_pairs() && M > kBlockM;
+  const int BN = block_n == 128 ? 128 : 256, tm = pairs ? 2 * kBlockM : kBlockM;
+  const long long tiles = static_cast<long long>((M + tm - 1) / tm) * ((N + BN - 1) / BN);
+  return 2 * tiles <= sm_count() / (pairs ? 2 : 1);
+}
+
 extern "C" long long dsb_gemm_workspace(int M, int N, int K, int block_n) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const SplitPlan plan = plan_splits(M, N, K, block_n);

@@ -624,9 +624,10 @@ class _SRWCallFn(torch.autograd.Function):
         d_scale = torch.zeros_like(sc_t) if sc_t is not None and ctx.needs_input_grad[3] else None
         xrs, ctx.xrs = ctx.xrs, [None] * R
         # few tokens: dx is a handful of tiles with K = U, which only an fp32 output lets the SM
-        # pairs share; the routes then add up there too
+        # pairs share (the launcher's own count of tiles); the routes then add up there too, in fp32.
+        # With many tokens every route's dx is rounded to bf16 by its GEMM before they are added.
         D = x_bf.shape[1]
-        few = ctx.needs_input_grad[0] and 2 * (-(-T // 256)) * (-(-D // 256)) <= 74
+        few = ctx.needs_input_grad[0] and e.gemm_few_tiles(T, D)
         dx = torch.zeros(T, D, dtype=torch.float32, device=dev) if few else None
         for i in range(R):
             rows = slice(i * T, (i + 1) * T)

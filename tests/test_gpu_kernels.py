@@ -1279,3 +1279,25 @@ def test_pool_call_without_tokens(cb):
     (res.route(0).sum() + res.route(1).sum()).backward()
     cb.check_status()
     assert float(scale.grad) == 0.0 and all(float(p.grad.abs().max()) == 0.0 for p in ps)
+
+
+def test_input_gradient_of_a_call_on_both_sides_of_its_summation_rule(cb):
+    """dx of a two-route call just below and above the token count from which the routes' gradients are
+    rounded to bf16 before they are added: rows of the same token agree to that rounding (2^-8 of the
+    largest route, 8e-3 of the norm), and with fp64 of the formula to 2e-2 (bf16 operands)."""
+    from dawn_srw_b200.ops.gates import GateSpec
+    dev = torch.device("cuda")
+    torch.manual_seed(5)
+    D, r, U, be, spec = 256, 64, 600, cb.CudaBackend(), GateSpec(kind=1)
+    T = next(t for t in range(256, 148 * 256, 256) if not cb.ext().gemm_few_tiles(t + 1, D))
+    assert cb.ext().gemm_few_tiles(T, D) and not cb.ext().gemm_few_tiles(T + 1, D)
+    ps = [torch.nn.functional.normalize(torch.randn(U, d, device=dev), dim=-1).requires_grad_(True) for d in (r, D, D)]
+    x0, h, off = torch.randn(T + 1, D, device=dev), torch.randn(T + 1, 2, r, device=dev), torch.zeros(T + 1, 2, device=dev)
+    dy, grads = torch.randn(2, T + 1, D, device=dev), []
+    for t in (T, T + 1):
+        x = x0[:t].clone().requires_grad_(True)
+        res = be.srw(x, h[:t], off[:t], be.prepare_pool(*ps, spec), spec, want_diag=False, out_scale=1.0)
+        sum((res.route(i) * dy[i, :t]).sum() for i in range(2)).backward()
+        grads.append(x.grad)
+    cb.check_status()
+    assert float(grads[0].abs().max()) > 0 and _rel(grads[1][:T], grads[0]) < 8e-3
