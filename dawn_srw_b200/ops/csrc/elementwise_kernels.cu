@@ -172,17 +172,19 @@ __global__ void __launch_bounds__(128) ln_bwd_dx_vec_kernel(const __nv_bfloat16*
   }
 }
 
-// dw, db under the same conditions: a block covers 128 columns (four per thread) of 64 rows (4.3 us for
-// 8192 x 384, 8.9 with 32 columns of 256 rows and scalar loads).
+// dw, db under the same conditions: a block covers 128 columns (four per thread) of 64 rows, or of more
+// where the grid could not hold them (4.3 us for 8192 x 384, 8.9 with 32 columns of 256 rows and scalar loads).
+constexpr int kRowsPerBlock = 64, kMaxGridY = 65535;
+int rows_per_block(int T) { return T <= kRowsPerBlock * kMaxGridY ? kRowsPerBlock : (T / kMaxGridY / 8 + 1) * 8; }
 __global__ void __launch_bounds__(256) ln_bwd_dwdb_vec_kernel(const __nv_bfloat16* __restrict__ dy,
                                                               const float* __restrict__ x,
                                                               const float* __restrict__ mean,
                                                               const float* __restrict__ rstd,
                                                               float* __restrict__ dw, float* __restrict__ db,
-                                                              int T, int D) {
+                                                              int T, int D, int rows) {
   __shared__ float s_w[8][128], s_b[8][128];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5, c = blockIdx.x * 128 + 4 * cx;
-  const int lo = blockIdx.y * 64, hi = min(T, lo + 64);
+  const int lo = blockIdx.y * rows, hi = T - lo < rows ? T : lo + rows;
   float aw[4] = {0.f, 0.f, 0.f, 0.f}, ab[4] = {0.f, 0.f, 0.f, 0.f};
   if (c < D) {
 #pragma unroll 4
@@ -650,7 +652,9 @@ extern "C" int dsb_layernorm_bwd(const void* dy_bf16, const float* x, const floa
     if (D <= 512) ln_bwd_dx_vec_kernel<4><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
     else if (D <= 1280) ln_bwd_dx_vec_kernel<10><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
     else ln_bwd_dx_vec_kernel<16><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
-    ln_bwd_dwdb_vec_kernel<<<dim3((D + 127) / 128, (T + 63) / 64), 256, 0, stream>>>(dy, x, mean, rstd, dw, db, T, D);
+    const int rows = rows_per_block(T);
+    ln_bwd_dwdb_vec_kernel<<<dim3((D + 127) / 128, T / rows + (T % rows != 0)), 256, 0, stream>>>(
+        dy, x, mean, rstd, dw, db, T, D, rows);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
   }
   ln_bwd_dx_kernel<<<(T + 7) / 8, 256, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
@@ -809,8 +813,6 @@ extern "C" int dsb_dropout(const float* res, const float* x, float* y, long long
 // columns, a block 128 columns of 64 rows (more where the grid could not hold them); the blocks' sums
 // are added up in their order by column_sum_kernel, so that a bias gradient repeats bit by bit.
 namespace {
-constexpr int kPackRows = 64, kMaxGridY = 65535;
-int pack_rows(int T) { return T <= kPackRows * kMaxGridY ? kPackRows : (T / kMaxGridY / 8 + 1) * 8; }
 
 // out[j] = part[0][j] + part[1][j] + ... in a fixed order (n % 4 == 0, part 16-byte aligned): a block takes 32
 // columns, its 32 groups of eight threads every 32nd row.
@@ -923,7 +925,7 @@ extern "C" int dsb_column_sum(const float* part, int rows, int n, float* out, cu
 }
 
 extern "C" int dsb_linear_pack_blocks(int T) {
-  const int rows = pack_rows(T);
+  const int rows = rows_per_block(T);
   return T / rows + (T % rows != 0);
 }
 
@@ -939,7 +941,7 @@ extern "C" int dsb_linear_pack(const DsbPackSrc* src, int n_src, int T, int n, v
     s[i].vec = (reinterpret_cast<uintptr_t>(s[i].ptr) & 15) == 0 && (s[i].ld & 3) == 0 && (s[i].col0 & 3) == 0;
   }
   const uint32_t thresh = static_cast<uint32_t>(static_cast<double>(p) * 4294967296.0);
-  const int rows = pack_rows(T), row_blocks = dsb_linear_pack_blocks(T);
+  const int rows = rows_per_block(T), row_blocks = dsb_linear_pack_blocks(T);
   const dim3 grid((n + 127) / 128, row_blocks);
   float* sums = colsum == nullptr ? nullptr : row_blocks == 1 ? colsum : part;
   __nv_bfloat16* d = static_cast<__nv_bfloat16*>(dst_bf16);

@@ -1301,3 +1301,16 @@ def test_input_gradient_of_a_call_on_both_sides_of_its_summation_rule(cb):
         grads.append(x.grad)
     cb.check_status()
     assert float(grads[0].abs().max()) > 0 and _rel(grads[1][:T], grads[0]) < 8e-3
+
+
+def test_layer_norm_gradients_of_more_rows_than_a_grid_has_blocks_of_64(cb):
+    """fp32 sums of four million terms, added up by atomics of 64 and more rows: 1e-4 of the terms' norm."""
+    T, D, dev = 65535 * 64 + 77, 4, torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(1)
+    x, dy = torch.randn(T, D, device=dev, generator=g), torch.randn(T, D, device=dev, generator=g).bfloat16()
+    w, b = torch.ones(D, device=dev, requires_grad=True), torch.zeros(D, device=dev, requires_grad=True)
+    cb.CudaBackend().layer_norm(x, w, b).backward(dy)
+    cb.check_status()
+    xn = torch.nn.functional.layer_norm(x.double(), (D,), eps=1e-6)
+    for got, terms in ((w.grad, dy.double() * xn), (b.grad, dy.double())):
+        assert float((got.double() - terms.sum(0)).norm()) < 1e-4 * float(terms.norm())
