@@ -29,6 +29,7 @@ terms is likewise ``emb . mean_t(h)``.
 from __future__ import annotations
 
 import math
+import weakref
 from typing import Any, List, Optional
 
 import torch
@@ -171,7 +172,6 @@ def _alloc_saved_xr(dev, T: int, Up: int, U: int, wanted: bool):
         return None
     xr = torch.empty(T, Up, dtype=torch.bfloat16, device=dev)
     key = dev.index if dev.index is not None else torch.cuda.current_device()
-    import weakref
     weakref.finalize(xr, XR_BUDGET.release, key, nbytes)
     return xr
 
@@ -888,11 +888,12 @@ class CudaBackend:
 
     # ---- dense ops -----------------------------------------------------
     def _w(self, w):
-        """bf16 compute copy of a master weight, refreshed when the weight changes."""
+        """bf16 compute copy of a master weight, refreshed when the weight changes.  The entry knows its
+        weight (weakly): a new tensor may get the id, and the version, of one that is gone."""
         key = id(w)
         hit = self._wcache.get(key)
-        if hit is None or hit[0] != w._version or hit[1].device != w.device:
-            hit = (w._version, w.detach().to(torch.bfloat16))
+        if hit is None or hit[0] != w._version or hit[1].device != w.device or hit[2]() is not w:
+            hit = (w._version, w.detach().to(torch.bfloat16), weakref.ref(w))
             self._wcache[key] = hit
         return hit[1]
 
@@ -928,7 +929,6 @@ class CudaBackend:
         cache = self.__dict__.setdefault("_cat_cache", {})
         hit = cache.get(id(layers[0]))
         if hit is None or hit[0] != key or any(r() is not q for r, q in zip(hit[4], ps)):
-            import weakref
             ws, bs, cuts, n0 = [], [], [], 0
             for l in layers:
                 n = l.weight.shape[0]

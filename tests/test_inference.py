@@ -173,3 +173,15 @@ def test_a_backend_that_has_run_can_be_copied_and_pickled(monkeypatch):
         assert (other.diag_chunk, other.keep_xr) == (77, False) and not other._wcache
         assert torch.equal(other._cat_weights(layers)[0], w) and other._cat_weights(layers)[0] is not w
     assert be._cat_weights(layers)[0] is w
+
+
+def test_a_kept_weight_copy_belongs_to_its_weight(monkeypatch):
+    """A new weight may get the id and the version of one that is gone; its copy is its own."""
+    from dawn_srw_b200.ops import cuda_backend as cb
+    monkeypatch.setattr(cb, "ext", lambda: None)
+    be = cb.CudaBackend()
+    old, new = (torch.nn.Parameter(torch.full((8, 16), v)) for v in (1.0, 2.0))
+    be._w(old)
+    be._wcache[id(new)] = be._wcache.pop(id(old))            # as if new had got the id of old
+    del old
+    assert torch.equal(be._w(new), new.detach().bfloat16())
