@@ -488,9 +488,10 @@ struct FwdGateEpi {
 // tile) and the 16 to 64 tokens the N side, so a stage is 16 KB of pool and 2 to 8 KB of tokens, eight of
 // them in flight per SM, and a tile is half the work of a 256-wide one, which evens out the last wave.
 // Lanes of an epilogue warp own consecutive units: stores of one token are consecutive addresses.
-// The 1B model's gate kernels, averaged over its pools: 52 us for 75 at 6 sequences; its write GEMMs
-// and projections 27 for 33; a decoded token 6.78 ms for 8.58, with 32 sequences (64 stacked rows of
-// Q and K) 7.90 for 8.73.  Above 64 rows the zeros are the smaller part and the wide tile stays.
+// Its epilogue costs more per token than that of a token tile (a tile has as many gates or columns
+// as before, in half the threads), so where the line lies follows from the K of a tile and from the
+// waves (few_rows_route, few_rows_plain).  The 1B model's gate kernels, averaged over its pools: 52 us for 75
+// at 6 sequences; its write GEMMs and projections 27 for 33.
 constexpr int kFewRows = 64;
 
 // Column sums over the 32 lanes of 16 values each; lane l gets the sum of value l & 15.
@@ -1591,6 +1592,33 @@ static int choose_k_splits(long long tiles, int units, int k_tiles, int max_by_k
   return (k_tiles + per_split - 1) / per_split;
 }
 
+// Whether a route (gate kernel and write GEMM) of T token rows runs swapped.  us a route, swapped / token
+// tiles, for d_model x units: up to 32 rows always (32 rows: 384 x 25 200 25 / 28, 1280 x 6400 25 / 29,
+// 1280 x 100 000 108 / 126, 2048 x 158 800 233 / 255).  Beyond that, with a short K only in one wave of unit
+// tiles (64 rows: 384 x 1580 29 / 31, 512 x 15 563 28 / 28, but 384 x 25 200 35 / 28); with a longer one up to
+// 48 rows (48: 1280 x 6400 28 / 29; 64: 31 / 29), and to 64 where the stream of the pool outweighs it (64:
+// 1280 x 100 000 118 / 127, 1024 x 40 000 61 / 79, 2048 x 9900 40 / 45, 2048 x 158 800 242 / 251).
+static bool few_rows_route(int T, int U, int D) {
+  if (T <= 32 || T > kFewRows) return T <= 32;
+  const int tiles = (U + kBlockM - 1) / kBlockM;
+  if (D < 768) return tiles <= sm_count();
+  return T <= 48 || D >= 1536 || tiles >= 2 * sm_count();
+}
+
+// The same for a plain product of M rows (N x K weights), us, swapped / token tiles.  With a bias (which a
+// token tile reads per column and row): always (64 rows: 128 x 384 9 / 10, 1160 x 2048 17 / 26, 30 522 x 1280
+// 23 / 31).  Without: by K (32 rows: 384 x 384 6.8 / 7.5; 48: 7.9 / 7.5, 1280 x 1280 12.9 / 13.9; 64: 13.8 / 14.0,
+// 1024 x 1024 12.6 / 11.7, 2048 x 2048 17.5 / 18.6); for a single tile half as many rows (16: 64 x 384 5.8 / 6.0;
+// 24: 6.6 / 6.0; 32: 8 x 2048 14.3 / 14.7; 48: 15.9 / 14.6); in more than one wave of tiles up to 24
+// rows (24: 30 522 x 1280 20.6 / 21.3; 32: 30 522 x 2048 30.2 / 28.9).
+static bool few_rows_plain(int M, int N, int K, bool bias) {
+  if (M > kFewRows) return false;
+  if (bias && N >= kBlockM) return true;
+  if (N > kBlockM * sm_count()) return M <= 24;
+  const int limit = K < 1024 ? 32 : K < 2048 ? 48 : 64;
+  return M <= (N <= kBlockM ? limit / 2 : limit);
+}
+
 template <class Epi>
 static int launch_few_rows(GemmParams<typename Epi::Params>& gp, int T, cudaStream_t stream) {
   if (T <= 16) return launch_engine_impl<16, Epi, 1>(gp, stream);
@@ -1755,8 +1783,10 @@ extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void*
                              int c_is_bf16, int accumulate, float alpha, const float* row_scale,
                              const float* bias, int block_n, float* ws, int* status,
                              cudaStream_t stream) {
-  if (M > 0 && M <= kFewRows && N > 0 && K > 0 && !a_mn && !b_mn && !c_is_bf16 && !accumulate &&
-      row_scale == nullptr)
+  // (a long K that a workspace allows to cut is better off with token tiles: 24 rows, 384 x 8192: 42 / 13)
+  if (M > 0 && N > 0 && K > 0 && !a_mn && !b_mn && !c_is_bf16 && !accumulate && row_scale == nullptr &&
+      few_rows_plain(M, N, K, bias != nullptr) &&
+      (bias != nullptr || ws == nullptr || plan_splits(M, N, K, block_n).splits == 1))
     return few_rows_gemm(A, lda, B, 0, ldb, M, N, K,
                          {static_cast<float*>(C), ldc, bias, nullptr, nullptr, alpha, 0}, status, stream);
   return gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, C, ldc, c_is_bf16, accumulate, alpha, row_scale,
@@ -1767,7 +1797,7 @@ extern "C" int dsb_srw_write(const void* p, long long ldp, const void* write, lo
                              int D, const float* den, float norm, const float* norm_ptr, float* y,
                              long long ldy, int accumulate, float* ws, int* status, cudaStream_t stream) {
   if (T <= 0 || U <= 0 || D <= 0) return 0;
-  if (T <= kFewRows && accumulate)
+  if (accumulate && few_rows_route(T, U, D))
     return few_rows_gemm(p, ldp, write, 1, ldw, T, D, U, {y, ldy, nullptr, den, norm_ptr, norm, 1}, status,
                          stream);
   return gemm_bf16(p, 0, ldp, write, 1, ldw, T, D, U, y, ldy, 0, accumulate, 1.f, nullptr, nullptr, den,
@@ -1847,7 +1877,7 @@ extern "C" int dsb_srw_fwd_gate_xr(const void* h, long long ldh, const void* emb
   // single CTAs take 128 x 256 tiles and twice as many of them stream the pool.
   const bool solo = wide && T <= kBlockM && xr_out == nullptr && diag == nullptr &&
                     !(gather != nullptr && gather->n_ranks > 1);
-  if (solo && T <= kFewRows && stats == nullptr && alive == nullptr && gate_sum == nullptr) {
+  if (solo && few_rows_route(T, U, D) && stats == nullptr && alive == nullptr && gate_sum == nullptr) {
     GemmParams<FewRowsGateParams> fp;
     memset(&fp, 0, sizeof(fp));
     const int bn = few_rows_tile(T);

@@ -1314,3 +1314,23 @@ def test_layer_norm_gradients_of_more_rows_than_a_grid_has_blocks_of_64(cb):
     xn = torch.nn.functional.layer_norm(x.double(), (D,), eps=1e-6)
     for got, terms in ((w.grad, dy.double() * xn), (b.grad, dy.double())):
         assert float((got.double() - terms.sum(0)).norm()) < 1e-4 * float(terms.norm())
+
+
+@pytest.mark.parametrize("T,U,D,r", [(32, 19200, 384, 64), (33, 19200, 384, 64), (33, 1580, 384, 64), (64, 1580, 384, 64),
+                                     (48, 6400, 1280, 64), (49, 6400, 1280, 64), (64, 6400, 2048, 64)])
+def test_routes_on_both_sides_of_the_swapped_form(cb, T, U, D, r):
+    """Where the rule by rows, units and width changes the form; the same bounds as between the forms."""
+    test_route_of_a_few_rows_on_the_tensor_engine(cb, 1, T, U, D, r)
+
+
+@pytest.mark.parametrize("M", [5, 16, 17, 24, 25, 32, 33, 48, 49, 64, 65])
+def test_gemms_on_both_sides_of_the_swapped_form(cb, M):
+    """One tile, one wave and more of them, short and long K, with and without a bias; fp32 sums, 1e-5."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(M)
+    for N, K in ((8, 384), (128, 2048), (384, 384), (1280, 1280), (2048, 2048), (19200, 128), (384, 8192)):
+        x, w = (torch.randn(n, K, device=dev, generator=g).bfloat16() for n in (M, N))
+        for bias in (None, torch.randn(N, device=dev, generator=g)):
+            ref = x.double() @ w.double().t() + (0.0 if bias is None else bias)
+            assert _rel(cb.gemm(x, False, w, False, out_dtype=torch.float32, bias=bias), ref) < 1e-5
+    cb.check_status()
