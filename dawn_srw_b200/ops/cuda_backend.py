@@ -230,10 +230,10 @@ class _LinearFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         xb, w_bf = ctx.saved_tensors
-        if dy.dtype == torch.float32 and dy.stride(1) == 1 and dy.shape[1] % 8 == 0:
-            # the bf16 operand and the bias gradient in one pass
-            dyb, *db = ext().linear_pack([dy], [0], dy.shape[0], dy.shape[1], ctx.has_bias, 0, 0.0, 0)
-            db = db[0] if ctx.has_bias else None
+        if ctx.has_bias and dy.dtype == torch.float32 and dy.stride(1) == 1 and dy.shape[1] % 8 == 0:
+            # the bf16 operand and the bias gradient in one pass (a cast alone is faster as a cast: forward
+            # and backward of 8192 x 2048 x 2048 without a bias took 243 us with this for 229)
+            dyb, db = ext().linear_pack([dy], [0], dy.shape[0], dy.shape[1], True, 0, 0.0, 0)
             count_launches(1)
         else:
             dyb = _bf16_2d(dy)
