@@ -382,6 +382,11 @@ struct KvParams {
 };
 constexpr int kKvThreads = 128, kKvGroups = kKvThreads / 4;
 constexpr int kKvMaxDh = 128;
+// Up to here the first CTA of a cluster takes all positions and the others leave: three rounds of its groups
+// cost less than two cluster barriers.  6 x 16 heads of 128: 4.5 us for 9.7 at 3 positions, 7.2 for 9.9 at
+// 96, 8.3 for 10.2 at 128; 6 heads of 64: 3.2 for 4.5, 4.4 for 4.7, and 5.0 for 4.8.  (A warp per position,
+// the form for unaligned rows, takes 2.6 us at 3 positions and 16 to 20 at 96.)
+constexpr int kSoloPositions = 96;
 
 // A running maximum starts at the lowest finite value, not at -inf: a score of -inf then weighs
 // nothing (exp(-inf - finite)) instead of turning into exp(-inf + inf), and a group without a
@@ -396,12 +401,14 @@ __global__ void __launch_bounds__(kKvThreads) kv_decode_split_kernel(const KvPar
   __shared__ __align__(16) float s_o[kKvThreads / 32][kKvMaxDh];
   __shared__ float c_ml[2];
   __shared__ float c_o[kKvMaxDh];
-  const int splits = gridDim.x, rank = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int rank = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, sub = lane & 3, grp = tid >> 2;
   const int nv4 = p.dh >> 2;
   long long pos = p.pos[0];
   pos = pos < 0 ? 0 : (pos >= p.s_max ? p.s_max - 1 : pos);
   const int n_old = static_cast<int>(pos);
+  const int splits = n_old <= kSoloPositions ? 1 : gridDim.x;       // the same in every CTA of a cluster
+  if (rank >= splits) return;
   const size_t row = (static_cast<size_t>(b) * p.H + h) * p.dh;
   float* ck = p.cache_k + row * p.s_max;
   float* cv = p.cache_v + row * p.s_max;

@@ -1334,3 +1334,18 @@ def test_gemms_on_both_sides_of_the_swapped_form(cb, M):
             ref = x.double() @ w.double().t() + (0.0 if bias is None else bias)
             assert _rel(cb.gemm(x, False, w, False, out_dtype=torch.float32, bias=bias), ref) < 1e-5
     cb.check_status()
+
+
+@pytest.mark.parametrize("B,H,dh,S", [(1, 6, 64, 512), (6, 16, 128, 512), (2, 3, 36, 200)])
+def test_decode_attention_around_the_positions_of_one_block(cb, B, H, dh, S):
+    """Up to 96 cached positions the first CTA of a cluster works alone; fp32 sums in another order."""
+    from dawn_srw_b200.ops import reference as R
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(dh)
+    rn = lambda *s: torch.randn(*s, device=dev, generator=g)
+    ck, cv, be = rn(B, H, S, dh), rn(B, H, S, dh), cb.CudaBackend()
+    for pos in (2, 95, 96, 97, 128):
+        q, k, v = rn(B, H * dh), rn(B, H * dh), rn(B, H * dh)
+        out = be.decode_attention(q, k, v, ck, cv, torch.tensor([pos], device=dev), H)
+        ref = R.cached_attention(q.view(B, H, 1, dh), ck, cv, pos + 1).reshape(B, H * dh)
+        assert torch.equal(ck[:, :, pos].reshape(B, -1), k) and _rel(out, ref) < 1e-5
