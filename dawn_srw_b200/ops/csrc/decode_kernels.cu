@@ -85,9 +85,12 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
   // registers allow the next read row to be in flight beside the accumulators
   constexpr bool kAhead = NR * KC <= 10;
   constexpr int kScoreUnroll = NR * EC == 1 ? 8 : 4;
+  // One x row is kept in fp32 (used once per active unit, 31.2 us for 33.1); of several, reading twice the
+  // shared memory costs more than unpacking: 100 000 units of 1280, all active, 2 rows 174 us in bf16, 196
+  // in fp32; 4 rows 229 and 263; 28 % active 112 and 124, 186 and 217.
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* s_acc = reinterpret_cast<float*>(smem_raw);                                // [warps][NR][D]
-  float* s_x = s_acc + kRowWarps * NR * p.D;                                        // [NR][D]
+  float* s_x = s_acc + kRowWarps * NR * p.D;                                        // [NR][D], fp32 or bf16
   __nv_bfloat16* s_h = reinterpret_cast<__nv_bfloat16*>(s_x + NR * p.D);                                            // [NR][r]
   float* s_g = reinterpret_cast<float*>(s_h + NR * p.r);                            // [kListUnits][NR]
   int* s_u = reinterpret_cast<int*>(s_g + kListUnits * NR);                         // [kListUnits] active units
@@ -101,11 +104,15 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
     const uint4* xs = reinterpret_cast<const uint4*>(p.x) + static_cast<size_t>(t % p.x_rows) * d_chunks;
     const uint4* hs = reinterpret_cast<const uint4*>(p.h) + static_cast<size_t>(t) * r_chunks;
     for (int c = tid; c < d_chunks; c += kRowWarps * 32) {
-      float f[8];                                        // fp32: the row is used once per active unit
-      unpack8(t < p.N ? xs[c] : none, f);
-      float4* dst = reinterpret_cast<float4*>(s_x + t * p.D + 8 * c);
-      dst[0] = make_float4(f[0], f[1], f[2], f[3]);
-      dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+      if constexpr (NR >= 2) {
+        reinterpret_cast<uint4*>(s_x)[t * d_chunks + c] = t < p.N ? xs[c] : none;
+      } else {
+        float f[8];
+        unpack8(t < p.N ? xs[c] : none, f);
+        float4* dst = reinterpret_cast<float4*>(s_x + t * p.D + 8 * c);
+        dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+        dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+      }
     }
     for (int c = tid; c < r_chunks; c += kRowWarps * 32)
       reinterpret_cast<uint4*>(s_h)[t * r_chunks + c] = t < p.N ? hs[c] : none;
@@ -252,9 +259,15 @@ __global__ void __launch_bounds__(kRowWarps * 32, (NR == 1 && KC == 5) ? 2 : 1) 
           unpack8(rq[k], rv);
 #pragma unroll
           for (int t = 0; t < NR; ++t) {
-            const float4 a = *reinterpret_cast<const float4*>(s_x + t * p.D + 8 * c);
-            const float4 b = *reinterpret_cast<const float4*>(s_x + t * p.D + 8 * c + 4);
-            const float xv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            float xv[8];
+            if constexpr (NR >= 2) {
+              unpack8(reinterpret_cast<const uint4*>(s_x)[t * d_chunks + c], xv);
+            } else {
+              const float4 a = *reinterpret_cast<const float4*>(s_x + t * p.D + 8 * c);
+              const float4 b = *reinterpret_cast<const float4*>(s_x + t * p.D + 8 * c + 4);
+              xv[0] = a.x; xv[1] = a.y; xv[2] = a.z; xv[3] = a.w;
+              xv[4] = b.x; xv[5] = b.y; xv[6] = b.z; xv[7] = b.w;
+            }
 #pragma unroll
             for (int j = 0; j < 8; ++j) xr[t] = fmaf(rv[j], xv[j], xr[t]);
           }
