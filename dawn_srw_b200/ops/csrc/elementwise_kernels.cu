@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(128) ln_fwd_vec_kernel(const float* __restrict
 }
 
 // dx of the backward pass under the same conditions: dy and x are read once (7.2 us for 8192 x 384, 8.6
-// with a second read).
+// with a second read).  Narrow rows take fewer steps per lane: 65 536 x 8 took 23.2 us with NV = 4,
+// 10.6 with 1.
 template <int NV>
 __global__ void __launch_bounds__(128) ln_bwd_dx_vec_kernel(const __nv_bfloat16* __restrict__ dy,
                                                             const float* __restrict__ x,
@@ -172,10 +173,10 @@ __global__ void __launch_bounds__(128) ln_bwd_dx_vec_kernel(const __nv_bfloat16*
   }
 }
 
-// dw, db under the same conditions: a block covers 128 columns (four per thread) of 64 rows, or of more
-// where the grid could not hold them (4.3 us for 8192 x 384, 8.9 with 32 columns of 256 rows and scalar loads).
-constexpr int kRowsPerBlock = 64, kMaxGridY = 65535;
-int rows_per_block(int T) { return T <= kRowsPerBlock * kMaxGridY ? kRowsPerBlock : (T / kMaxGridY / 8 + 1) * 8; }
+// dw, db under the same conditions: a block covers 128 columns (four per thread) of 64 rows (4.3 us for
+// 8192 x 384, 8.9 with 32 columns of 256 rows and scalar loads), or of more where that would be more than 256
+// blocks that add to the same columns: 65 536 x 64 took 12.2 us in 1024 blocks, 8.0 in 256, x 384 32.7 and 29.9.
+int ln_rows_per_block(int T) { return T <= 64 * 256 ? 64 : (T / 256 / 8 + 1) * 8; }
 __global__ void __launch_bounds__(256) ln_bwd_dwdb_vec_kernel(const __nv_bfloat16* __restrict__ dy,
                                                               const float* __restrict__ x,
                                                               const float* __restrict__ mean,
@@ -649,10 +650,12 @@ extern "C" int dsb_layernorm_bwd(const void* dy_bf16, const float* x, const floa
   const __nv_bfloat16* dy = reinterpret_cast<const __nv_bfloat16*>(dy_bf16);
   if (D % 4 == 0 && D <= 2048 && aligned16(x, w, dy, dx)) {
     const int blocks = (T + 3) / 4;
-    if (D <= 512) ln_bwd_dx_vec_kernel<4><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
+    if (D <= 128) ln_bwd_dx_vec_kernel<1><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
+    else if (D <= 256) ln_bwd_dx_vec_kernel<2><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
+    else if (D <= 512) ln_bwd_dx_vec_kernel<4><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
     else if (D <= 1280) ln_bwd_dx_vec_kernel<10><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
     else ln_bwd_dx_vec_kernel<16><<<blocks, 128, 0, stream>>>(dy, x, w, mean, rstd, dx, T, D);
-    const int rows = rows_per_block(T);
+    const int rows = ln_rows_per_block(T);
     ln_bwd_dwdb_vec_kernel<<<dim3((D + 127) / 128, T / rows + (T % rows != 0)), 256, 0, stream>>>(
         dy, x, mean, rstd, dw, db, T, D, rows);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
@@ -814,6 +817,9 @@ extern "C" int dsb_dropout(const float* res, const float* x, float* y, long long
 // are added up in their order by column_sum_kernel, so that a bias gradient repeats bit by bit.
 namespace {
 
+constexpr int kPackRows = 64, kMaxGridY = 65535;
+int pack_rows(int T) { return T <= kPackRows * kMaxGridY ? kPackRows : (T / kMaxGridY / 8 + 1) * 8; }
+
 // out[j] = part[0][j] + part[1][j] + ... in a fixed order (n % 4 == 0, part 16-byte aligned): a block takes 32
 // columns, its 32 groups of eight threads every 32nd row.
 __global__ void __launch_bounds__(256) column_sum_kernel(const float* __restrict__ part, int rows, int n,
@@ -925,7 +931,7 @@ extern "C" int dsb_column_sum(const float* part, int rows, int n, float* out, cu
 }
 
 extern "C" int dsb_linear_pack_blocks(int T) {
-  const int rows = rows_per_block(T);
+  const int rows = pack_rows(T);
   return T / rows + (T % rows != 0);
 }
 
@@ -941,7 +947,7 @@ extern "C" int dsb_linear_pack(const DsbPackSrc* src, int n_src, int T, int n, v
     s[i].vec = (reinterpret_cast<uintptr_t>(s[i].ptr) & 15) == 0 && (s[i].ld & 3) == 0 && (s[i].col0 & 3) == 0;
   }
   const uint32_t thresh = static_cast<uint32_t>(static_cast<double>(p) * 4294967296.0);
-  const int rows = rows_per_block(T), row_blocks = dsb_linear_pack_blocks(T);
+  const int rows = pack_rows(T), row_blocks = dsb_linear_pack_blocks(T);
   const dim3 grid((n + 127) / 128, row_blocks);
   float* sums = colsum == nullptr ? nullptr : row_blocks == 1 ? colsum : part;
   __nv_bfloat16* d = static_cast<__nv_bfloat16*>(dst_bf16);

@@ -1349,3 +1349,17 @@ def test_decode_attention_around_the_positions_of_one_block(cb, B, H, dh, S):
         out = be.decode_attention(q, k, v, ck, cv, torch.tensor([pos], device=dev), H)
         ref = R.cached_attention(q.view(B, H, 1, dh), ck, cv, pos + 1).reshape(B, H * dh)
         assert torch.equal(ck[:, :, pos].reshape(B, -1), k) and _rel(out, ref) < 1e-5
+
+
+@pytest.mark.parametrize("T,D", [(16384, 384), (16385, 132), (70001, 8)])
+def test_layer_norm_gradients_where_a_block_takes_more_rows(cb, T, D):
+    """fp32 sums of T terms in another order: 1e-5 of the terms' norm."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device=dev).manual_seed(D)
+    x, dy = torch.randn(T, D, device=dev, generator=g), torch.randn(T, D, device=dev, generator=g).bfloat16()
+    w, b = torch.ones(D, device=dev, requires_grad=True), torch.zeros(D, device=dev, requires_grad=True)
+    cb.CudaBackend().layer_norm(x, w, b).backward(dy)
+    cb.check_status()
+    xn = torch.nn.functional.layer_norm(x.double(), (D,), eps=1e-6)
+    for got, terms in ((w.grad, dy.double() * xn), (b.grad, dy.double())):
+        assert float((got.double() - terms.sum(0)).norm()) < 1e-5 * float(terms.norm())
