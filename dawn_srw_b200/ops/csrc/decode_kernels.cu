@@ -1,4 +1,5 @@
-// SRW pool op for a handful of token rows (KV-cache decoding at batch 1..4).
+// SRW pool op for up to four stacked token rows (routes times sequences: V and Know of up to four
+// sequences, Q and K of up to two; half of that above d_model 1280).
 //
 // With one to four rows the op is a stream over the pool: per unit u it needs
 // e_u (r values), and r_u and w_u (d_model values each) where some row's gate is not
@@ -8,7 +9,7 @@
 // and a few hundred FMAs.  A tensor-core tile would spend a 128-row MMA on those rows, so
 // this path is plain SIMT and bound by HBM - if enough loads are in flight.  A block
 // therefore takes its units in two phases: all scores first, four embedding rows in flight
-// per group of lanes, the units with a gate going on a list in shared memory; then the
+// per group of lanes (eight with one token row and r <= 256), the units with a gate going on a list in shared memory; then the
 // listed units, dealt evenly to the warps, with the next unit's read row and this unit's
 // write row in flight.  (A warp that took a unit from score to write waited out the latency of
 // HBM twice for every active one.)  Every sum has a fixed order: lists are compacted in unit order,

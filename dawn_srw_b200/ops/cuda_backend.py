@@ -572,8 +572,8 @@ class _SRWCallFn(torch.autograd.Function):
     gradients of the Gram matrix and of the pool tensors go straight into the buffers that the
     pool's preparation node chains on.  (A node per route between statistics, selects and clamps
     was some 160 launches a layer more: a training step of 4 x 128 tokens on the 40M model took
-    57.8 ms for 41.6, a forward of 16 x 512 tokens 18.2 for 13.6.)  Backward per route starts with one row kernel that makes
-    the bf16 ``dy * scale / max(den, 1)`` operand and, from <dy, y>,
+    57.8 ms for 41.6, a forward of 16 x 512 tokens 18.2 for 13.6.)  Backward per route starts with
+    one row kernel that makes the bf16 ``dy * scale / max(den, 1)`` operand and, from <dy, y>,
         d_den = -<dy, y> / den  (den > 1),   d_scale = sum_t <dy, y> / scale.
     Returns y_0 .. y_{R-1} [T, D], hsum [r], den [R, T], tau and 1/sigma [R, T] (not
     differentiable)."""
@@ -602,7 +602,7 @@ class _SRWCallFn(torch.autograd.Function):
         count_launches(3 + 2 * R)
         ctx.save_for_backward(x_bf, off, hb, hg, tau, isd, mu, sd, den, sc_t, *ys)
         ctx.hd, ctx.esum, ctx.spec, ctx.args = hd, ex["esum"].detach(), spec, (T, R, r, U, inv_u, sc_f)
-        ctx.xrs, ctx.h_shape = xrs, h.shape
+        ctx.xrs = xrs
         ctx.set_materialize_grads(False)
         tau_o, isd_o = tau.view(R, T), isd.view(R, T)
         ctx.mark_non_differentiable(tau_o, isd_o)

@@ -500,7 +500,10 @@ def test_kernels_are_run_to_run_deterministic(cb):
     """Every tile-produced output must be bit-identical between two runs (a
     missing barrier or a racing tile shows up here); only the per-token sums
     that are accumulated with atomics may differ in the last bits.  Products with
-    few tiles and a long K, which are cut: the next test."""
+    few tiles and a long K, which are cut: test_split_products_repeat_bit_by_bit; row
+    and column sums of the backward pass have tests of their own; not promised to
+    repeat: denominators, LayerNorm's and the embeddings' gradients, and products
+    that accumulate (pool gradients, Gram matrices, write GEMMs of generation)."""
     from dawn_srw_b200.ops.gates import GateSpec
     dev = torch.device("cuda")
     g = torch.Generator(device=dev).manual_seed(9)
