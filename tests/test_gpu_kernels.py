@@ -953,7 +953,7 @@ def test_gemm_of_a_few_rows_with_swapped_operands(cb, M):
                                         (300, 131, 10400, False), (256, 128, 4096, True)])
 def test_plain_gemm_with_few_tiles_and_a_long_k(cb, M, N, K, a_mn):
     """K is cut although the caller does not accumulate: whatever the output held is gone, rows
-    beyond its width stay, and a row scale applies once per split part (fp32 sums: 1e-5)."""
+    beyond its width stay, and the row scale applies to the sum of the parts (fp32 sums: 1e-5)."""
     dev = torch.device("cuda")
     g = torch.Generator(device=dev).manual_seed(K + M)
     A = torch.randn(M, K, device=dev, generator=g).bfloat16()
