@@ -74,7 +74,7 @@ void gemm(const Tensor& A, bool a_mn, const Tensor& B, bool b_mn, Tensor& C, boo
   // a caller that accumulates gets reduce-adds in any order, any other a result that repeats
   const bool ordered = !accumulate && !c_bf16 && opt_f32(bias) == nullptr;
   auto ws = ordered ? gemm_workspace(M, N, K, block_n, A) : Tensor();
-  int rc = dsb_gemm_bf16(A.data_ptr(), a_mn, A.stride(0), B.data_ptr(), b_mn, B.stride(0), M, N, K,
+  int rc = dsb_gemm_bf16_ws(A.data_ptr(), a_mn, A.stride(0), B.data_ptr(), b_mn, B.stride(0), M, N, K,
                          C.data_ptr(), C.stride(0), c_bf16, accumulate, alpha, opt_f32(row_scale),
                          opt_f32(bias), block_n, ptr(ws), status.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "dsb_gemm_bf16 failed with code ", rc);
@@ -712,7 +712,7 @@ std::vector<Tensor> srw_stats(const Tensor& h, const Tensor& off, const Tensor& 
   int rc = dsb_score_pack(h.data_ptr<float>(), h.stride(0), h.stride(1), T, R, r, hb.data_ptr(),
                           den.data_ptr<float>(), N, hsum.data_ptr<float>(), r, cur_stream());
   if (rc == 0)
-    rc = dsb_gemm_bf16(hb.data_ptr(), 0, r, gcat.data_ptr(), 0, gcat.stride(0), N, 2 * r, r, hg.data_ptr(),
+    rc = dsb_gemm_bf16_ws(hb.data_ptr(), 0, r, gcat.data_ptr(), 0, gcat.stride(0), N, 2 * r, r, hg.data_ptr(),
                        2 * r, 0, 0, 1.f, nullptr, nullptr, block_width(2 * r), nullptr,
                        status.data_ptr<int>(), cur_stream());
   if (rc == 0)
@@ -833,7 +833,7 @@ c10::optional<Tensor> srw_route_bwd(const Tensor& x, const Tensor& h, const Tens
   auto mm = [&](const Tensor& A, bool a_mn, long long lda, const Tensor& B, long long ldb, int M, int N, int K,
                 Tensor& C, bool accumulate, bool ordered) {
     auto ws = ordered && C.scalar_type() == torch::kFloat32 ? gemm_workspace(M, N, K, block_width(N), C) : Tensor();
-    const int e = dsb_gemm_bf16(A.data_ptr(), a_mn, lda, B.data_ptr(), 1, ldb, M, N, K, C.data_ptr(),
+    const int e = dsb_gemm_bf16_ws(A.data_ptr(), a_mn, lda, B.data_ptr(), 1, ldb, M, N, K, C.data_ptr(),
                                 C.stride(0), C.scalar_type() == torch::kBFloat16, accumulate, 1.f, nullptr,
                                 nullptr, block_width(N), ptr(ws), status_p, st);
     TORCH_CHECK(e == 0, "srw_route_bwd: GEMM failed with code ", e);
@@ -901,7 +901,7 @@ std::vector<Tensor> srw_stats_bwd(const Tensor& dtau, const Tensor& dh32, c10::o
                                w.data_ptr(), d_off.data_ptr<float>(), g_esum.data_ptr<float>(), cur_stream());
   if (rc == 0 && g_gram.has_value() && g_gram->defined()) {
     TORCH_CHECK(ok(*g_gram, static_cast<int64_t>(r) * r));
-    rc = dsb_gemm_bf16(w.data_ptr(), 1, r, hb.data_ptr(), 1, r, r, r, N, g_gram->data_ptr(), r, 0, 1, inv_u,
+    rc = dsb_gemm_bf16_ws(w.data_ptr(), 1, r, hb.data_ptr(), 1, r, r, r, N, g_gram->data_ptr(), r, 0, 1, inv_u,
                        nullptr, nullptr, block_width(r), nullptr, status.data_ptr<int>(), cur_stream());
   }
   TORCH_CHECK(rc == 0, "srw_stats_bwd failed with code ", rc);

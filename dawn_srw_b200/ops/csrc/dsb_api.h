@@ -42,13 +42,17 @@ typedef struct DsbGather {
 //   B: b_mn == 0 -> stored [N][K];             b_mn == 1 -> stored [K][N]
 //   bf16 operands, fp32 accumulation; C is bf16 (c_is_bf16) or fp32.
 //   Leading dimensions must be multiples of 8 elements, bases 16-byte aligned.
-//   workspace: dsb_gemm_workspace floats, 16-byte aligned, or null.  With it a product of few output
-//   tiles and a long K (fp32, no bias) is cut in K and its parts are added up in order; without it
-//   it is cut only if it accumulates, and the parts arrive in any order.
+int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn, long long ldb,
+                  int M, int N, int K, void* C, long long ldc, int c_is_bf16, int accumulate,
+                  float alpha, const float* row_scale, const float* bias, int block_n,
+                  int* status, cudaStream_t stream);
+// The same with a workspace: dsb_gemm_workspace floats, 16-byte aligned, or null.  With it a product of few
+// output tiles and a long K (fp32, no bias) is cut in K and its parts are added up in order; without it
+// it is cut only if it accumulates, and the parts arrive in any order.
 long long dsb_gemm_workspace(int M, int N, int K, int block_n);
 // 1 if the output tiles of an M x N product leave half of the chip idle (so that K is worth cutting).
 int dsb_gemm_few_tiles(int M, int N, int block_n);
-int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn, long long ldb,
+int dsb_gemm_bf16_ws(const void* A, int a_mn, long long lda, const void* B, int b_mn, long long ldb,
                   int M, int N, int K, void* C, long long ldc, int c_is_bf16, int accumulate,
                   float alpha, const float* row_scale, const float* bias, int block_n,
                   float* workspace, int* status, cudaStream_t stream);

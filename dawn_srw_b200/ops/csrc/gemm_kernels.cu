@@ -1778,11 +1778,11 @@ extern "C" long long dsb_gemm_workspace(int M, int N, int K, int block_n) {
   return plan.splits > 1 ? static_cast<long long>(plan.splits) * plan.m_tiles * plan.tile_m * ((N + 3) / 4 * 4) : 0;
 }
 
-extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn,
-                             long long ldb, int M, int N, int K, void* C, long long ldc,
-                             int c_is_bf16, int accumulate, float alpha, const float* row_scale,
-                             const float* bias, int block_n, float* ws, int* status,
-                             cudaStream_t stream) {
+extern "C" int dsb_gemm_bf16_ws(const void* A, int a_mn, long long lda, const void* B, int b_mn,
+                                long long ldb, int M, int N, int K, void* C, long long ldc,
+                                int c_is_bf16, int accumulate, float alpha, const float* row_scale,
+                                const float* bias, int block_n, float* ws, int* status,
+                                cudaStream_t stream) {
   // (a long K that a workspace allows to cut is better off with token tiles: 24 rows, 384 x 8192: 42 / 13)
   if (M > 0 && N > 0 && K > 0 && !a_mn && !b_mn && !c_is_bf16 && !accumulate && row_scale == nullptr &&
       few_rows_plain(M, N, K, bias != nullptr) &&
@@ -1791,6 +1791,14 @@ extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void*
                          {static_cast<float*>(C), ldc, bias, nullptr, nullptr, alpha, 0}, status, stream);
   return gemm_bf16(A, a_mn, lda, B, b_mn, ldb, M, N, K, C, ldc, c_is_bf16, accumulate, alpha, row_scale,
                    bias, nullptr, nullptr, 1.f, block_n, ws, status, stream);
+}
+
+extern "C" int dsb_gemm_bf16(const void* A, int a_mn, long long lda, const void* B, int b_mn,
+                             long long ldb, int M, int N, int K, void* C, long long ldc,
+                             int c_is_bf16, int accumulate, float alpha, const float* row_scale,
+                             const float* bias, int block_n, int* status, cudaStream_t stream) {
+  return dsb_gemm_bf16_ws(A, a_mn, lda, B, b_mn, ldb, M, N, K, C, ldc, c_is_bf16, accumulate, alpha,
+                          row_scale, bias, block_n, nullptr, status, stream);
 }
 
 extern "C" int dsb_srw_write(const void* p, long long ldp, const void* write, long long ldw, int T, int U,
@@ -2072,7 +2080,7 @@ extern "C" int dsb_srw_forward(const void* h, long long ldh, const void* emb, lo
   if (rc) return rc;
   // raw_out[T,D] = p[T,U] . write[U,D]   (write is the MN-major B operand)
   return dsb_gemm_bf16(p_scratch, 0, ldp, write, 1, ldw, T, D, U, raw_out, ldo, 0, 0, 1.0f,
-                       nullptr, nullptr, 256, nullptr, status, stream);
+                       nullptr, nullptr, 256, status, stream);
 }
 
 // GEMM whose output rows are scattered to their owner ranks (first half of a
